@@ -1,6 +1,7 @@
 // Plain matrix product C[m,n] (+)= A[m,k] . W[n,k]^T on the CUDA cores with float32
-// multiply-add: the true 32-bit path of the engine (no tensor cores, no reduced
-// precision mode) and the reference the fast bf16 products are tested against.
+// multiply-add (no tensor cores, no reduced precision mode): the reference the fast bf16
+// products are tested against, and the product of bf16 shapes that those cannot take.  All-float32
+// operands, the engine's true 32-bit path, go to gemm_f32.cu.
 //
 // Every output element is accumulated by one thread over k in ascending order, so
 // its value does not depend on m, on the other rows of the batch or on the grid.
@@ -78,6 +79,9 @@ gemm_plain_kernel(const TA* A, const TW* __restrict__ W, TC* C, int m,
     }
 }
 
+RLLM_API int rllm_gemm_f32_batched(const float* A, const float* W, float* C, int m, int n, int k, int lda, int ldw, int ldc,
+                                   int accumulate, int batch, long long sa, long long sw, long long sc, cudaStream_t stream);
+
 // A batch of `batch` independent products, operand b at A + b * sa, W + b * sw, C + b * sc (elements):
 // the per-head products of attention through latents (heads as the batch, rows strided by the
 // token's whole row).
@@ -94,7 +98,9 @@ RLLM_API int rllm_gemm_plain_batched(const void* A, int a_dtype, const void* W, 
                        (const TW*)W, (TC*)C, m, n, k, lda, ldw, ldc, accumulate, sa, sw, sc)
     const int key = a_dtype * 4 + w_dtype * 2 + c_dtype;
     switch (key) {
-        case 0: LAUNCH(float, float, float); break;
+        case 0:
+            return rllm_gemm_f32_batched((const float*)A, (const float*)W, (float*)C, m, n, k, lda, ldw, ldc, accumulate, batch,
+                                         sa, sw, sc, stream);
         case 1: LAUNCH(float, float, bf16); break;
         case 2: LAUNCH(float, bf16, float); break;
         case 3: LAUNCH(float, bf16, bf16); break;
