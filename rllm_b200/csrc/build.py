@@ -31,7 +31,7 @@ NVCC_FLAGS = [
 
 # library name -> (sources, extra link flags)
 LIBRARIES = {
-    "core": (["elementwise.cu", "rowwise.cu", "headwise.cu", "joins.cu", "attention_generic.cu", "gemm_plain.cu", "gemm_f32.cu", "sampling.cu"], []),
+    "core": (["elementwise.cu", "rowwise.cu", "headwise.cu", "joins.cu", "attention_generic.cu", "attention_f32.cu", "gemm_plain.cu", "gemm_f32.cu", "sampling.cu"], []),
     "recur": (["recurrent.cu"], []),
     "delta": (["delta.cu"], []),
     "ssd": (["ssd.cu"], []),

@@ -1897,6 +1897,63 @@ DECODE_MAX_Q = 8               # requests with at most this many tokens in the s
 DECODE_ROWS = 8                # (token, head) rows of a decode tile: 8 takes the kernel with the keys as the M side
 
 
+F32_TILE_ROWS = 32             # rows (tokens x query heads) of a tile of attention_f32.cu
+
+
+class F32AttentionPlan:
+    """Tokens and tiles of one float32 step for one group size (query heads per key/value head): requests of at most
+    DECODE_MAX_Q tokens go token by token, longer portions in tiles.  Built once per step, shared by its layers."""
+
+    def __init__(self, ctx, g, device):
+        self.GH = min(g, F32_TILE_ROWS)
+        self.chunks = -(-g // self.GH)
+        self.TT = F32_TILE_ROWS // self.GH
+        toks, t_req, t_tok, at = [], [], [], 0
+        for r, k in enumerate(ctx.q_lens):
+            if k <= DECODE_MAX_Q:
+                toks += range(at, at + k)
+            else:
+                starts = range(at, at + k, self.TT)
+                t_req += [r] * len(starts)
+                t_tok += starts
+            at += k
+        self.n_rows, self.n_tiles = len(toks), len(t_req)
+        flat = torch.tensor(toks + t_req + t_tok + [0], dtype=torch.int32).to(device)
+        a, b = self.n_rows, self.n_rows + self.n_tiles
+        self.tokens, self.t_req, self.t_tok = flat[:a], flat[a:b], flat[b:b + self.n_tiles]
+
+
+def paged_attention_f32(q, k_cache, v_cache, out, ctx, block_table, H, K, hd, block_size, scale, window=0, keep_first=0,
+                        chunk=0, softcap=0.0, sink=None, slopes=None):
+    """float32 attention of the step's tokens over the paged cache for heads of 64 or 128 (attention_f32.cu); the masks,
+    caps, slopes and sinks of paged_attention_generic."""
+    _need_cuda(q, k_cache, v_cache, out, block_table, sink, slopes)
+    _need_contig(q=q, k_cache=k_cache, v_cache=v_cache, out=out)
+    assert q.dtype == k_cache.dtype == v_cache.dtype == out.dtype == torch.float32 and hd in FLASH_HEAD_DIMS
+    assert q.shape == out.shape == (ctx.n_tokens, H * hd) and k_cache.shape[1:] == v_cache.shape[1:] == (K, block_size, hd)
+    assert block_table.dtype == torch.int32 and block_table.dim() == 2 and block_table.stride(1) == 1
+    for w in (sink, slopes):
+        assert w is None or (w.dtype == torch.float32 and w.numel() == H and w.is_contiguous())
+    key = ("float32", H // K)
+    plan = ctx.plans.get(key)
+    if plan is None:
+        plan = ctx.plans[key] = F32AttentionPlan(ctx, H // K, q.device)
+    tail = (c_int(window), c_int(keep_first), c_int(chunk), c_float(softcap), c_int(min(k_cache.shape[0], 0x7fffffff)),
+            _ptr(error_word(q.device)), _ptr(sink), _ptr(slopes), _stream())
+    if plan.n_tiles:
+        _check(core().rllm_attn_f32_tiles(
+            _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(ctx.positions), _ptr(ctx.cu_q), _ptr(plan.t_req),
+            _ptr(plan.t_tok), c_int(plan.n_tiles), c_int(plan.TT), c_int(plan.GH), c_int(plan.chunks), _ptr(block_table),
+            c_int(block_table.stride(0)), c_int(H), c_int(K), c_int(hd), c_int(block_size), c_float(scale), *tail),
+            "attn_f32_tiles")
+    if plan.n_rows:
+        _check(core().rllm_attn_f32_rows(
+            _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(ctx.positions), _ptr(ctx.seq_ids), _ptr(plan.tokens),
+            c_int(plan.n_rows), _ptr(block_table), c_int(block_table.stride(0)), c_int(H), c_int(K), c_int(hd),
+            c_int(block_size), c_float(scale), *tail), "attn_f32_rows")
+    return out
+
+
 class AttentionPlan:
     """Tiles of one step for one attention geometry (query heads per key/value head, window):
     which requests take the decode shape (16-row tiles, split keys) and which the prefill shape
@@ -2149,11 +2206,16 @@ def shared_kv_attention(q, cache, out, ctx, block_table, H, hd, hdv, block_size,
 def paged_attention(q, k_cache, v_cache, out, ctx, block_table, H, K, hd, block_size, scale, window=0,
                     keep_first=0, v_head_dim=None, chunk=0, softcap=0.0, sink=None, slopes=None):
     """Attention of the step's tokens over the paged cache; chooses the kernel by element type,
-    head size and the shape of the step (`ctx`: the step's StepContext).  float32, head sizes
-    other than 64 and 128 and value heads of another size than the key heads take the plain kernel;
+    head size and the shape of the step (`ctx`: the step's StepContext).  Head sizes other than 64
+    and 128 and value heads of another size than the key heads take the plain kernel, float32 heads
+    of 64 and 128 those of attention_f32.cu (which read rows 16 bytes at a time);
     windows that keep the first keys take the mma.sync kernels, not the tcgen05 one."""
     hdv = hd if not v_head_dim else int(v_head_dim)
     keep_first = keep_first if window else 0
+    if (q.dtype == torch.float32 and k_cache.dtype == torch.float32 and hd in FLASH_HEAD_DIMS and hdv == hd
+            and all(t.data_ptr() % 16 == 0 for t in (q, k_cache, v_cache, out))):
+        return paged_attention_f32(q, k_cache, v_cache, out, ctx, block_table, H, K, hd, block_size, scale, window,
+                                   keep_first, chunk, softcap, sink, slopes)
     if q.dtype != torch.bfloat16 or hd not in FLASH_HEAD_DIMS or hdv != hd:
         return paged_attention_generic(q, k_cache, v_cache, out, ctx.positions, ctx.seq_ids, block_table,
                                        H, K, hd, block_size, scale, window, keep_first, hdv, chunk, softcap, sink, slopes)
