@@ -23,6 +23,60 @@ __device__ __forceinline__ void st_any(void* p, int dt, size_t i, float v) {
     else ((bf16*)p)[i] = __float2bfloat16_rn(v);
 }
 
+// four neighbouring entries (16 or 8 bytes, aligned)
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 ld4(const bf16* p) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void st4(bf16* p, float4 v) {
+    uint2 u;
+    *reinterpret_cast<__nv_bfloat162*>(&u.x) = __floats2bfloat162_rn(v.x, v.y);
+    *reinterpret_cast<__nv_bfloat162*>(&u.y) = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = u;
+}
+__device__ __forceinline__ float4 ld4_any(const void* p, int dt, size_t i) {
+    return dt == RLLM_F32 ? ld4((const float*)p + i) : ld4((const bf16*)p + i);
+}
+static inline bool al16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+
+// rows_act on rows that can be read four entries at a time (every stride a multiple of 4, bases on 16 bytes): bound by its
+// bytes.  A block takes 1,024 columns of one row, so no thread divides by the row's length (a 64-bit division per element
+// cost more than the memory); relu^2 of 2,048 x 12,288, float32 to bfloat16: 47 us one element a thread, now 19 us.
+#define ROWS4_THREADS 256
+__global__ void __launch_bounds__(ROWS4_THREADS)
+rows_act4_kernel(const void* in, int in_dt, long long in_stride, const float* __restrict__ bias, int act1, const void* mul,
+                 int mul_dt, long long mul_stride, int act2, void* out, int out_dt, long long out_stride, int cols, int mul_group,
+                 float factor, const float* row_scale) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const size_t t = blockIdx.x;
+    const int c = (blockIdx.y * ROWS4_THREADS + threadIdx.x) * 4;
+    if (c >= cols) return;
+    float4 v = ld4_any(in, in_dt, t * in_stride + c);
+    float x[4] = {v.x, v.y, v.z, v.w}, m[4];
+    if (mul) {
+        if (mul_group == 1) {
+            const float4 f = ld4_any(mul, mul_dt, t * mul_stride + c);
+            m[0] = f.x; m[1] = f.y; m[2] = f.z; m[3] = f.w;
+        } else m[0] = m[1] = m[2] = m[3] = ld_any(mul, mul_dt, t * mul_stride + c / mul_group);
+    }
+    const float s = row_scale ? row_scale[t] : 1.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (row_scale) x[i] *= s;
+        if (bias) x[i] += bias[c + i];
+        x[i] = act_apply(x[i], act1) * factor;
+        if (mul) x[i] *= act_apply(m[i], act2);
+    }
+    v = make_float4(x[0], x[1], x[2], x[3]);
+    if (out_dt == RLLM_F32) st4((float*)out + t * out_stride + c, v);
+    else st4((bf16*)out + t * out_stride + c, v);
+}
+
 __global__ void rows_act_kernel(const void* in, int in_dt, long long in_stride, const float* __restrict__ bias,
                                 int act1, const void* mul, int mul_dt, long long mul_stride, int act2, void* out,
                                 int out_dt, long long out_stride, int cols, size_t total, int mul_group, float factor,
@@ -69,13 +123,18 @@ RLLM_API int rllm_rows_act(const void* in, int in_dt, long long in_stride, const
     const size_t total = (size_t)n * cols;
     if (total == 0) return 0;
     if (mul_group <= 0) return (int)cudaErrorInvalidValue;
-    const auto al16 = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
     if (in_dt == RLLM_BF16 && out_dt == RLLM_BF16 && mul && mul_dt == RLLM_F32 && !bias && !row_scale && act1 == ACT_NONE &&
         mul_group % 8 == 0 && cols % 8 == 0 && in_stride % 8 == 0 && out_stride % 8 == 0 && al16(in) && al16(out)) {
         const size_t t8 = total / 8;
         return rllm_launch(rows_gate_bf16_kernel, dim3((unsigned)((t8 + 255) / 256)), dim3(256), 0, stream, (const bf16*)in,
                            in_stride, (const float*)mul, mul_stride, act2, (bf16*)out, out_stride, cols / 8, mul_group / 8, t8, factor);
     }
+    if (cols % 4 == 0 && in_stride % 4 == 0 && out_stride % 4 == 0 && al16(in) && al16(out) &&
+        (!mul || mul_group % 4 == 0 || (mul_group == 1 && mul_stride % 4 == 0 && al16(mul))) &&
+        cols <= 4 * ROWS4_THREADS * 65535)
+        return rllm_launch(rows_act4_kernel, dim3(n, (cols / 4 + ROWS4_THREADS - 1) / ROWS4_THREADS), dim3(ROWS4_THREADS), 0, stream,
+                           in, in_dt, in_stride, bias, act1, mul, mul_dt, mul_stride, act2, out, out_dt, out_stride, cols,
+                           mul_group, factor, row_scale);
     return rllm_launch(rows_act_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, in, in_dt,
                        in_stride, bias, act1, mul, mul_dt, mul_stride, act2, out, out_dt, out_stride, cols, total,
                        mul_group, factor, row_scale);
@@ -87,9 +146,22 @@ __global__ void axpby_kernel(float a, const float* x, float b, const float* y, f
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < total) out[i] = a * x[i] + b * y[i];
 }
+// four elements a thread: 2,048 x 4,096 36 -> 11 us
+__global__ void axpby4_kernel(float a, const float* x, float b, const float* y, float* out, size_t quads) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= quads) return;
+    const float4 u = ld4(x + 4 * i), v = ld4(y + 4 * i);
+    st4(out + 4 * i, make_float4(a * u.x + b * v.x, a * u.y + b * v.y, a * u.z + b * v.z, a * u.w + b * v.w));
+}
 RLLM_API int rllm_axpby(float a, const float* x, float b, const float* y, float* out, long long total,
                         cudaStream_t stream) {
     if (total <= 0) return 0;
+    if (total % 4 == 0 && al16(x) && al16(y) && al16(out)) {
+        const size_t quads = (size_t)total / 4;
+        return rllm_launch(axpby4_kernel, dim3((unsigned)((quads + 255) / 256)), dim3(256), 0, stream, a, x, b, y, out, quads);
+    }
     return rllm_launch(axpby_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, a, x, b, y, out,
                        (size_t)total);
 }
@@ -108,10 +180,35 @@ __global__ void cat2_cast_kernel(const float* x, const void* delta, int delta_dt
     st_any(out, out_dt, t * 2 * d + c, v);
     st_any(out, out_dt, t * 2 * d + d + c, y[i]);
 }
+// four columns a thread, no division: 2,048 x 4,096 43 -> 15 us
+__global__ void __launch_bounds__(ROWS4_THREADS)
+cat2_cast4_kernel(const float* x, const void* delta, int delta_dt, float s, const float* y, void* out, int out_dt, int d) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const size_t t = blockIdx.x;
+    const int c = (blockIdx.y * ROWS4_THREADS + threadIdx.x) * 4;
+    if (c >= d) return;
+    float4 v = ld4(x + t * d + c);
+    const float4 w = ld4(y + t * d + c);
+    if (delta) {
+        const float4 e = ld4_any(delta, delta_dt, t * d + c);
+        v = make_float4(v.x + s * e.x, v.y + s * e.y, v.z + s * e.z, v.w + s * e.w);
+    }
+    if (out_dt == RLLM_F32) {
+        st4((float*)out + t * 2 * d + c, v);
+        st4((float*)out + t * 2 * d + d + c, w);
+    } else {
+        st4((bf16*)out + t * 2 * d + c, v);
+        st4((bf16*)out + t * 2 * d + d + c, w);
+    }
+}
 RLLM_API int rllm_cat2_cast(const float* x, const void* delta, int delta_dt, float s, const float* y, void* out,
                             int out_dt, int n, int d, cudaStream_t stream) {
     const size_t total = (size_t)n * d;
     if (total == 0) return 0;
+    if (d % 4 == 0 && al16(x) && al16(y) && al16(out) && (!delta || al16(delta)) && d <= 4 * ROWS4_THREADS * 65535)
+        return rllm_launch(cat2_cast4_kernel, dim3(n, (d / 4 + ROWS4_THREADS - 1) / ROWS4_THREADS), dim3(ROWS4_THREADS), 0, stream, x,
+                           delta, delta_dt, s, y, out, out_dt, d);
     return rllm_launch(cat2_cast_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, x, delta,
                        delta_dt, s, y, out, out_dt, d, total);
 }
@@ -189,6 +286,69 @@ qkv_rownorm_store_kernel(const TI* qkv, const float* __restrict__ bias, const fl
     }
 }
 
+// The same without a rotation, on float32 rows that can be read four entries at a time: the q and k columns stay in
+// registers (NV float4 a thread) between the sums and the stores, both sums are taken in one exchange.  Bound by its bytes;
+// 2,048 rows of 4,096 + 1,024 + 1,024: 51 us through shared memory an entry at a time, now 32 us; 8 rows 9.9 -> 5.9 us.
+template <typename TO, int NV>
+__global__ void __launch_bounds__(1024)
+qkv_rownorm_store4_kernel(const float* qkv, const float* __restrict__ bias, const float* __restrict__ q_norm_w,
+                          const float* __restrict__ k_norm_w, const int* __restrict__ slots, TO* q_out, TO* k_cache, TO* v_cache,
+                          long long ld, int wq, int wk, int wv, int G, int dk, int dv, int bs, float eps, int write_kv,
+                          int n_slots, int* err, int v_off) {
+    __shared__ float red[2][32];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    const float* row = qkv + (size_t)t * ld;
+    auto biased = [&](int c) {
+        float4 v = ld4(row + c);
+        if (bias) { v.x += bias[c]; v.y += bias[c + 1]; v.z += bias[c + 2]; v.w += bias[c + 3]; }
+        return v;
+    };
+    float4 val[NV];
+    float sq = 0.f, sk = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int c = 4 * (tid + i * blockDim.x);
+        if (c >= wq + wk) continue;
+        val[i] = biased(c);
+        const float s = val[i].x * val[i].x + val[i].y * val[i].y + val[i].z * val[i].z + val[i].w * val[i].w;
+        if (c < wq) sq += s; else sk += s;
+    }
+    sq = warp_sum(sq);
+    sk = warp_sum(sk);
+    if (lane == 0) { red[0][tid >> 5] = sq; red[1][tid >> 5] = sk; }
+    __syncthreads();
+    const bool in = lane < (int)(blockDim.x >> 5);
+    sq = warp_sum(in ? red[0][lane] : 0.f);
+    sk = warp_sum(in ? red[1][lane] : 0.f);
+    const float rq = 1.0f / sqrtf(sq / (float)wq + eps), rk = 1.0f / sqrtf(sk / (float)wk + eps);
+    int slot = write_kv ? slots[t] : -1;
+    if (slot >= n_slots) {
+        if (tid == 0 && err) atomicExch(err, RLLM_ERR_SLOT);
+        slot = -1;
+    }
+    const size_t page = slot < 0 ? 0 : slot / bs, off = slot < 0 ? 0 : slot % bs;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        int c = 4 * (tid + i * blockDim.x);
+        if (c >= wq + wk) continue;
+        const bool is_q = c < wq;
+        if (!is_q) c -= wq;
+        const float* w = is_q ? q_norm_w : k_norm_w;
+        float4 v = val[i];
+        if (w) {
+            const float r = is_q ? rq : rk;
+            v = make_float4(v.x * r * w[c], v.y * r * w[c + 1], v.z * r * w[c + 2], v.w * r * w[c + 3]);
+        }
+        if (is_q) st4(q_out + (size_t)t * wq + c, v);
+        else if (slot >= 0) st4(k_cache + ((page * G + c / dk) * bs + off) * dk + c % dk, v);
+    }
+    if (slot < 0) return;
+    for (int c = 4 * tid; c < wv; c += 4 * blockDim.x)
+        st4(v_cache + ((page * G + c / dv) * bs + off) * dv + c % dv, biased(v_off + c));
+}
+
 RLLM_API int rllm_qkv_rownorm_store(const void* qkv, int in_dt, long long ld, const float* bias, const float* q_norm_w,
                                     const float* k_norm_w, const int* slots, void* q_out, void* k_cache,
                                     void* v_cache, int out_dt, int n, int H, int G, int dk, int dv, int bs,
@@ -202,6 +362,21 @@ RLLM_API int rllm_qkv_rownorm_store(const void* qkv, int in_dt, long long ld, co
     const int ns = (int)(n_slots > 0x7fffffffLL ? 0x7fffffffLL : n_slots);
     // a block per token: few tokens (a decode step) get more threads each, since the row's sums keep it in one block
     const int threads = n < 128 ? 1024 : 256;
+    const int qk = (H + G) * dk, nv = (qk / 4 + threads - 1) / threads;
+    if (in_dt == RLLM_F32 && !rot && nv <= 8 && ld % 4 == 0 && dk % 4 == 0 && dv % 4 == 0 && v_off % 4 == 0 && al16(qkv) &&
+        al16(q_out) && al16(k_cache) && al16(v_cache)) {
+#define LAUNCH4(TO, NV)                                                                                                        \
+    return rllm_launch(qkv_rownorm_store4_kernel<TO, NV>, dim3(n), dim3(threads), 0, stream, (const float*)qkv, bias, q_norm_w, \
+                       k_norm_w, slots, (TO*)q_out, (TO*)k_cache, (TO*)v_cache, ld, H * dk, G * dk, G * dv, G, dk, dv, bs, eps, \
+                       write_kv, ns, err, v_off)
+        if (out_dt == RLLM_F32) {
+            if (nv <= 2) { LAUNCH4(float, 2); }
+            LAUNCH4(float, 8);
+        }
+        if (nv <= 2) { LAUNCH4(bf16, 2); }
+        LAUNCH4(bf16, 8);
+#undef LAUNCH4
+    }
     const size_t smem = (size_t)(H + G) * dk * sizeof(float);
 #define LAUNCH(TI, TO)                                                                                         \
     if (smem <= 40 * 1024)                                                                                     \
