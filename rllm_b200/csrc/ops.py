@@ -2054,7 +2054,7 @@ def attention_tc_ok(q, hd, block_size, H, K) -> bool:
 
 
 def attention_tc(q, k_cache, v_cache, out, positions, cu_q, block_table, tile_req, tile_tok0, n_tiles, H, K, hd,
-                 block_size, scale, window, chunk=0, softcap=0.0, sink=None, slopes=None):
+                 block_size, scale, window, chunk=0, softcap=0.0, sink=None, slopes=None, keep_first=0):
     """Prefill attention on the tcgen05 tensor cores (S and O in tensor memory); see attention_tc.cu."""
     _need_cuda(q, k_cache, v_cache, out, positions, cu_q, block_table, tile_req, tile_tok0, sink, slopes)
     for w in (sink, slopes):
@@ -2067,7 +2067,8 @@ def attention_tc(q, k_cache, v_cache, out, positions, cu_q, block_table, tile_re
         _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), c_int(q.shape[0]), c_longlong(k_cache.shape[0]),
         _ptr(positions), _ptr(cu_q), _ptr(block_table), c_int(block_table.stride(0)), _ptr(tile_req),
         _ptr(tile_tok0), c_int(n_tiles), c_int(H), c_int(K), c_int(hd), c_int(block_size), c_float(scale),
-        c_int(window), c_int(chunk), c_float(softcap), _ptr(sink), _ptr(slopes), _ptr(error_word(q.device)), _stream())
+        c_int(window), c_int(keep_first), c_int(chunk), c_float(softcap), _ptr(sink), _ptr(slopes),
+        _ptr(error_word(q.device)), _stream())
     if st >= 30000:
         raise KernelError(f"attention_tc: tensor map encoding failed (CUresult {st - 30000})")
     _check(st, "attention_tc")
@@ -2208,8 +2209,7 @@ def paged_attention(q, k_cache, v_cache, out, ctx, block_table, H, K, hd, block_
     """Attention of the step's tokens over the paged cache; chooses the kernel by element type,
     head size and the shape of the step (`ctx`: the step's StepContext).  Head sizes other than 64
     and 128 and value heads of another size than the key heads take the plain kernel, float32 heads
-    of 64 and 128 those of attention_f32.cu (which read rows 16 bytes at a time);
-    windows that keep the first keys take the mma.sync kernels, not the tcgen05 one."""
+    of 64 and 128 those of attention_f32.cu (which read rows 16 bytes at a time)."""
     hdv = hd if not v_head_dim else int(v_head_dim)
     keep_first = keep_first if window else 0
     if (q.dtype == torch.float32 and k_cache.dtype == torch.float32 and hd in FLASH_HEAD_DIMS and hdv == hd
@@ -2223,9 +2223,9 @@ def paged_attention(q, k_cache, v_cache, out, ctx, block_table, H, K, hd, block_
     plan = ctx.plans.get(key)
     if plan is None:
         plan = ctx.plans[key] = AttentionPlan(ctx, H, K, window, q.device, chunk)
-    if plan.n_pre and plan.n_tc and USE_ATTENTION_TC and attention_tc_ok(q, hd, block_size, H, K) and not keep_first:
+    if plan.n_pre and plan.n_tc and USE_ATTENTION_TC and attention_tc_ok(q, hd, block_size, H, K):
         attention_tc(q, k_cache, v_cache, out, ctx.positions, ctx.cu_q, block_table, plan.t_req, plan.t_tok,
-                     plan.n_tc, H, K, hd, block_size, scale, window, chunk, softcap, sink, slopes)
+                     plan.n_tc, H, K, hd, block_size, scale, window, chunk, softcap, sink, slopes, keep_first)
     elif plan.n_pre:
         paged_flash_attention(q, k_cache, v_cache, out, ctx.positions, ctx.cu_q, block_table, plan.p_req,
                               plan.p_tok, plan.n_pre, H, K, hd, block_size, scale, window, 0, plan.TTp,
