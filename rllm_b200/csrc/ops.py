@@ -759,13 +759,15 @@ def conv_silu(xz, weight, bias, state, conv_off, ctx_seq_ids, cu_q, slots, out, 
 
 
 def selective_scan(x, xz, low, b_off, c_off, dtr, dt_bias, A, D, state, conv_off, cu_q, slots, out, n_requests,
-                   inner, N, taps, segments=None):
+                   inner, N, taps, segments=None, one_token=False):
     """The selective scan over each request's tokens with its state in state[slot, :inner*N]; see
-    recurrent.cu.  x, out: activation type [n, inner]; xz, low, dtr float32."""
+    recurrent.cu.  x, out: activation type [n, inner]; xz, low, dtr float32.  one_token: the caller says that
+    every request brings exactly one token."""
     _need_cuda(x, xz, low, dtr, dt_bias, A, D, state, out)
     _need_contig(x=x, out=out, dtr=dtr, A=A)
     _rows2d(xz, "xz"), _rows2d(low, "low")
     n = x.shape[0]
+    assert not one_token or (n == n_requests and segments is None)
     assert x.dtype == out.dtype and x.shape == out.shape == (n, inner) and dtr.shape == (n, inner)
     assert xz.dtype == low.dtype == dtr.dtype == torch.float32 and xz.shape[1] >= 2 * inner
     assert A.shape == (inner, N) and A.dtype == dt_bias.dtype == D.dtype == torch.float32
@@ -785,7 +787,7 @@ def selective_scan(x, xz, low, b_off, c_off, dtr, dt_bias, A, D, state, conv_off
         c_longlong(conv_off), _ptr(cu_q), _ptr(slots), _ptr(out), c_int(n_requests), c_int(inner), c_int(N),
         c_int(taps), _ptr(sg.t0 if sg else None), _ptr(sg.t1 if sg else None), _ptr(sg.req if sg else None),
         _ptr(sg.flags if sg else None), _ptr(sg.item0 if sg else None), _ptr(sg.items if sg else None),
-        c_int(sg.n_items if sg else 0), _ptr(carry), _ptr(decay), _stream()), "selective_scan")
+        c_int(sg.n_items if sg else 0), _ptr(carry), _ptr(decay), c_int(1 if one_token else 0), _stream()), "selective_scan")
     if sg is not None:
         global _launches
         _launches += 2                         # the local pass and the combine kernel
@@ -857,13 +859,15 @@ def time_segments(ctx, device, length=SEGMENT_TOKENS, shortest=SEGMENT_FROM):
     return plan
 
 
-def wkv(r, k, v, wraw, g, w0, u, norm_w, eps, state, prev_off, h, cu_q, slots, out, n_requests, H, D, segments=None):
+def wkv(r, k, v, wraw, g, w0, u, norm_w, eps, state, prev_off, h, cu_q, slots, out, n_requests, H, D, segments=None,
+        one_token=False):
     """The RWKV recurrence with data-dependent decay, unit norm per head, norm weight and silu gate; see
     recurrent.cu.  r, k, v, wraw, g float32 [n, H*D] (equal row strides); out activation type.
     segments: the step's TimeSegments (long portions are then worked through segment by segment, side
-    by side) or None."""
+    by side) or None.  one_token: the caller says that every request brings exactly one token."""
     _need_cuda(r, k, v, wraw, g, w0, u, norm_w, state, h, out)
     n = out.shape[0]
+    assert not one_token or (n == n_requests and segments is None)
     for name, t in (("r", r), ("k", k), ("v", v), ("wraw", wraw), ("g", g)):
         _rows2d(t, name)
         assert t.dtype == torch.float32 and t.shape == (n, H * D) and t.stride(0) == r.stride(0)
@@ -888,7 +892,7 @@ def wkv(r, k, v, wraw, g, w0, u, norm_w, eps, state, prev_off, h, cu_q, slots, o
                                   _ptr(sg.t0 if sg else None), _ptr(sg.t1 if sg else None), _ptr(sg.req if sg else None),
                                   _ptr(sg.flags if sg else None), _ptr(sg.item0 if sg else None),
                                   _ptr(sg.items if sg else None), c_int(sg.n_items if sg else 0), _ptr(carry),
-                                  _ptr(decay), _stream()), "wkv")
+                                  _ptr(decay), c_int(1 if one_token else 0), _stream()), "wkv")
     if sg is not None:
         global _launches
         _launches += 2                         # the local pass and the combine kernel

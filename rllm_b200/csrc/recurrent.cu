@@ -28,7 +28,85 @@
 //   out[t, c] = silu(b[c] + sum_j w[c, j] * in(i - (taps-1) + j)),  in(i') = xz row of that token
 //   for i' >= 0, else the request's kept inputs (state) -- zeros at the start of a sequence.
 // The state itself is advanced by the scan kernel, which runs after every read here.
+//
+// conv_silu4_kernel (four taps, rows that can be read 16 bytes at a time): bound by its bytes, every input read once and
+// every output written once.  A thread takes four neighbouring channels of `tok` tokens in a row and keeps the three
+// rows before the current one in registers; two bytes and four bytes at a time, each input read four times over,
+// 2,048 x 8,192 took 125 us, now 36 us.  conv_silu_kernel: any shape.
 #define CONV_TOK 1             // tokens per block (more did not pay: 119 us against 116 for 2,048 x 8,192, and decode steps lost)
+__device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store4(bf16* p, float4 v) {
+    uint2 u;
+    *reinterpret_cast<__nv_bfloat162*>(&u.x) = __floats2bfloat162_rn(v.x, v.y);
+    *reinterpret_cast<__nv_bfloat162*>(&u.y) = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = u;
+}
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const bf16* p) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+#define ROW4_THREADS 128
+template <typename TO>
+__global__ void __launch_bounds__(ROW4_THREADS)
+conv_silu4_kernel(const float* xz, long long ld, const float* __restrict__ w, const float* __restrict__ b, const float* state,
+                  long long slot_stride, long long conv_off, const int* __restrict__ seq_ids, const int* __restrict__ cu_q,
+                  const int* __restrict__ slots, TO* out, int n, int inner, int tok) {
+    const int c = (blockIdx.y * ROW4_THREADS + threadIdx.x) * 4;
+    float wt[4][4], bias[4];                               // [channel][tap]
+    const bool on = c < inner;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float4 v = on ? load4(w + (size_t)(c + i) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        wt[i][0] = v.x; wt[i][1] = v.y; wt[i][2] = v.z; wt[i][3] = v.w;
+        bias[i] = on && b ? b[c + i] : 0.f;
+    }
+    pdl_wait();
+    pdl_launch_dependents();
+    if (!on) return;
+    const int ta = blockIdx.x * tok, tb = min(n, ta + tok);
+    float4 h3 = make_float4(0.f, 0.f, 0.f, 0.f), h2 = h3, h1 = h3;      // the inputs three, two and one token back
+    int r = -1;
+    for (int t = ta; t < tb; ++t) {
+        const float4 x = load4(xz + (size_t)t * ld + c);
+        const int rt = seq_ids[t];
+        if (rt != r) {                                     // a request begins, here or before this block's tokens
+            r = rt;
+            const int i = t - cu_q[r];
+            const float* st = state + (size_t)slots[r] * slot_stride + conv_off + (size_t)c * 3;
+            // the input `back` tokens before t: a row of this step, or place 3 - back + i of the kept inputs (oldest first)
+            auto before = [&](int back) {
+                if (back <= i) return load4(xz + (size_t)(t - back) * ld + c);
+                const float* k = st + (3 - back + i);
+                return make_float4(k[0], k[3], k[6], k[9]);
+            };
+            h3 = before(3);
+            h2 = before(2);
+            h1 = before(1);
+        }
+        auto value = [&](int i, float a, float b2, float c2, float d) {
+            float acc = bias[i];
+            acc += wt[i][0] * a;
+            acc += wt[i][1] * b2;
+            acc += wt[i][2] * c2;
+            acc += wt[i][3] * d;
+            return silu_f(acc);
+        };
+        store4(out + (size_t)t * inner + c, make_float4(value(0, h3.x, h2.x, h1.x, x.x), value(1, h3.y, h2.y, h1.y, x.y),
+                                                        value(2, h3.z, h2.z, h1.z, x.z), value(3, h3.w, h2.w, h1.w, x.w)));
+        h3 = h2; h2 = h1; h1 = x;
+    }
+}
+
+// tokens per thread of the kernels that keep rows in registers: enough threads for the SMs, at most 16 tokens
+static int row4_tokens(int n, int columns) {
+    const long long quads = (long long)n * ((columns + 3) / 4);
+    const long long t = quads / (148LL * 1024);
+    return t < 1 ? 1 : t > 16 ? 16 : (int)t;
+}
+
 template <typename TO>
 __global__ void conv_silu_kernel(const float* xz, long long ld, const float* __restrict__ w,
                                  const float* __restrict__ b, const float* state, long long slot_stride,
@@ -60,6 +138,15 @@ RLLM_API int rllm_conv_silu(const float* xz, long long ld, const float* w, const
                             cudaStream_t stream) {
     if (n <= 0) return 0;
     if (taps < 1 || inner <= 0) return (int)cudaErrorInvalidValue;
+    if (taps == 4 && inner % 4 == 0 && ld % 4 == 0 && ((uintptr_t)xz | (uintptr_t)w | (uintptr_t)out) % 16 == 0) {
+        const int tok = row4_tokens(n, inner);
+        const dim3 grid4((n + tok - 1) / tok, (inner / 4 + ROW4_THREADS - 1) / ROW4_THREADS);
+        if (out_dt == RLLM_F32)
+            return rllm_launch(conv_silu4_kernel<float>, grid4, dim3(ROW4_THREADS), 0, stream, xz, ld, w, b, state, slot_stride,
+                               conv_off, seq_ids, cu_q, slots, (float*)out, n, inner, tok);
+        return rllm_launch(conv_silu4_kernel<bf16>, grid4, dim3(ROW4_THREADS), 0, stream, xz, ld, w, b, state, slot_stride,
+                           conv_off, seq_ids, cu_q, slots, (bf16*)out, n, inner, tok);
+    }
     const dim3 grid((n + CONV_TOK - 1) / CONV_TOK, (inner + 255) / 256 > 64 ? 64 : (inner + 255) / 256);
     if (out_dt == RLLM_F32)
         return rllm_launch(conv_silu_kernel<float>, grid, dim3(256), 0, stream, xz, ld, w, b, state, slot_stride,
@@ -73,9 +160,9 @@ RLLM_API int rllm_conv_silu(const float* xz, long long ld, const float* w, const
 //   dt = softplus(dtr[t, c] + dt_b[c]);  S[c, n] = exp(dt * A[c, n]) * S[c, n] + dt * x[t, c] * B[t, n]
 //   y  = sum_n S[c, n] * C[t, n] + D[c] * x[t, c];      out[t, c] = y * silu(z[t, c])
 // x: the convolution's output (activation type), B and C: columns of `low` (float32), z: columns
-// [inner, 2 inner) of xz.  SCAN_LANES lanes share a channel (state index n = lane + SCAN_LANES * k);
+// [inner, 2 inner) of xz.  SCAN_LANES lanes share a channel, with neighbouring states each (B and C are read four at a time);
 // their partial sums are added in a fixed butterfly.  A block owns SCAN_CH channels of one request and
-// walks its tokens SCAN_TOK at a time: x, the step sizes (softplus done on the way in), silu(z), B and
+// walks its tokens a chunk at a time: x, the step sizes (softplus done on the way in), silu(z), B and
 // C of a chunk lie in shared memory, and the next chunk's values are already on their way from global
 // memory (held in registers) while this one is worked through, so the recurrence never waits for a
 // load.  At the end the convolution's kept inputs move on by this step's tokens.
@@ -98,23 +185,24 @@ struct TimeSegments {
 
 #define SCAN_LANES 4
 #define SCAN_CH 32            // channels per block (128 threads)
-#define SCAN_TOK 16           // tokens per chunk
+#define SCAN_TOK 16           // tokens per chunk (1 where every request brings one token)
 #define SCAN_THREADS (SCAN_LANES * SCAN_CH)
 
-template <typename TA, int NPT, int PASS>
+template <typename TA, int NPT, int PASS, int TOK>
 __global__ void __launch_bounds__(SCAN_THREADS)
 selective_scan_kernel(const TA* x, const float* xz, long long ld_xz, const float* low, long long ld_low, int b_off,
                       int c_off, const float* dtr, const float* __restrict__ dt_b, const float* __restrict__ A,
                       const float* __restrict__ Dp, float* state, long long slot_stride, long long conv_off,
                       const int* __restrict__ cu_q, const int* __restrict__ slots, TA* out, int inner, int N,
                       int taps, const TimeSegments seg) {
-    constexpr int PRE_X = 3 * SCAN_TOK * SCAN_CH / SCAN_THREADS;      // x, dt, z of a chunk: values per thread
-    constexpr int PRE_BC = NPT;                                        // B and C of a chunk (N <= SCAN_LANES * NPT)
-    extern __shared__ float sm_scan[];
-    float* s_x = sm_scan;                                // [SCAN_TOK][SCAN_CH]
-    float* s_dt = s_x + SCAN_TOK * SCAN_CH;
-    float* s_z = s_dt + SCAN_TOK * SCAN_CH;              // silu(z)
-    float* s_bc = s_z + SCAN_TOK * SCAN_CH;              // [SCAN_TOK][2][N]
+    constexpr int PRE_X = (3 * TOK * SCAN_CH + SCAN_THREADS - 1) / SCAN_THREADS;   // x, dt, z of a chunk: values per thread
+    constexpr int NP = SCAN_LANES * NPT;                               // N rounded up; what lies beyond N is zero
+    constexpr int PRE_BC = (2 * TOK * NP + SCAN_THREADS - 1) / SCAN_THREADS;       // B and C of a chunk
+    extern __shared__ __align__(16) float sm_scan[];
+    float* s_x = sm_scan;                                // [TOK][SCAN_CH]
+    float* s_dt = s_x + TOK * SCAN_CH;
+    float* s_z = s_dt + TOK * SCAN_CH;              // silu(z)
+    float* s_bc = s_z + TOK * SCAN_CH;              // [TOK][2][NP]
     pdl_wait();
     pdl_launch_dependents();
     const int item = blockIdx.y;
@@ -136,7 +224,7 @@ selective_scan_kernel(const TA* x, const float* xz, long long ld_xz, const float
     float sum_dt = 0.f;
 #pragma unroll
     for (int k = 0; k < NPT; ++k) {
-        const int n = lane + SCAN_LANES * k;
+        const int n = lane * NPT + k;
         const bool on = n < N;
         S[k] = (on && PASS != 1) ? from[(size_t)c * N + n] : 0.f;
         a[k] = on ? A[(size_t)c * N + n] : 0.f;
@@ -145,14 +233,14 @@ selective_scan_kernel(const TA* x, const float* xz, long long ld_xz, const float
     float px[PRE_X], pbc[PRE_BC];
     // element e of the x/dt/z part: which (0 x, 1 dt, 2 z), token, channel of the block
     auto fetch = [&](int tb) {
-        const int nt = min(SCAN_TOK, t1 - tb);
+        const int nt = min(TOK, t1 - tb);
 #pragma unroll
         for (int i = 0; i < PRE_X; ++i) {
             const int e = tid + i * SCAN_THREADS;
-            const int which = e / (SCAN_TOK * SCAN_CH), rem = e % (SCAN_TOK * SCAN_CH);
+            const int which = e / (TOK * SCAN_CH), rem = e % (TOK * SCAN_CH);
             const int tt = rem / SCAN_CH, ch = c_base + rem % SCAN_CH;
             float v = 0.f;
-            if (tt < nt && ch < inner) {
+            if (which < 3 && tt < nt && ch < inner) {
                 const size_t t = tb + tt;
                 v = which == 0 ? to_f<TA>(x[t * inner + ch]) : which == 1 ? dtr[t * inner + ch] : xz[t * ld_xz + inner + ch];
             }
@@ -161,25 +249,25 @@ selective_scan_kernel(const TA* x, const float* xz, long long ld_xz, const float
 #pragma unroll
         for (int i = 0; i < PRE_BC; ++i) {
             const int e = tid + i * SCAN_THREADS;
-            const int tt = e / (2 * N), j = e % (2 * N);
-            pbc[i] = (tt < nt) ? low[(size_t)(tb + tt) * ld_low + (j < N ? b_off + j : c_off + j - N)] : 0.f;
+            const int tt = e / (2 * NP), j = e % (2 * NP), n = j % NP;
+            pbc[i] = (tt < nt && n < N) ? low[(size_t)(tb + tt) * ld_low + (j < NP ? b_off : c_off) + n] : 0.f;
         }
     };
     auto stash = [&]() {
 #pragma unroll
         for (int i = 0; i < PRE_X; ++i) {
             const int e = tid + i * SCAN_THREADS;
-            const int which = e / (SCAN_TOK * SCAN_CH), rem = e % (SCAN_TOK * SCAN_CH);
+            const int which = e / (TOK * SCAN_CH), rem = e % (TOK * SCAN_CH);
             const int ch = c_base + rem % SCAN_CH;
             float v = px[i];
             if (which == 1) v = softplus_f(v + (ch < inner ? dt_b[ch] : 0.f));
             else if (which == 2) v = silu_f(v);
-            sm_scan[e] = v;
+            if (which < 3) sm_scan[e] = v;
         }
 #pragma unroll
         for (int i = 0; i < PRE_BC; ++i) {
             const int e = tid + i * SCAN_THREADS;
-            if (e < SCAN_TOK * 2 * N) s_bc[e] = pbc[i];
+            if (e < TOK * 2 * NP) s_bc[e] = pbc[i];
         }
     };
     if (t0 < t1) {
@@ -187,37 +275,39 @@ selective_scan_kernel(const TA* x, const float* xz, long long ld_xz, const float
         stash();
     }
     __syncthreads();
-    for (int tb = t0; tb < t1; tb += SCAN_TOK) {
-        const int nt = min(SCAN_TOK, t1 - tb);
-        const bool more = tb + SCAN_TOK < t1;
-        if (more) fetch(tb + SCAN_TOK);
+    for (int tb = t0; tb < t1; tb += TOK) {
+        const int nt = min(TOK, t1 - tb);
+        const bool more = tb + TOK < t1;
+        if (more) fetch(tb + TOK);
         // One token: only S carries over from the token before, so with the loop unrolled the
         // exponentials, loads and shuffles of neighbouring tokens overlap.
         auto token = [&](int tt) {
             const float xv = s_x[tt * SCAN_CH + cl];
             const float dt = s_dt[tt * SCAN_CH + cl];
             const float dx = dt * xv;
-            const float* Bt = s_bc + tt * 2 * N;
-            const float* Ct = Bt + N;
+            const float4* Bt = reinterpret_cast<const float4*>(s_bc + tt * 2 * NP + lane * NPT);
+            const float4* Ct = reinterpret_cast<const float4*>(s_bc + tt * 2 * NP + NP + lane * NPT);
             float part = 0.f;
             if (PASS == 1) sum_dt += dt;
 #pragma unroll
-            for (int k = 0; k < NPT; ++k) {
-                const int n = lane + SCAN_LANES * k;
-                if (n < N) {
-                    S[k] = expf(dt * a[k]) * S[k] + dx * Bt[n];
-                    if (PASS != 1) part += S[k] * Ct[n];
+            for (int k = 0; k < NPT; k += 4) {
+                const float4 B4 = Bt[k / 4], C4 = PASS != 1 ? Ct[k / 4] : B4;
+                const float bb[4] = {B4.x, B4.y, B4.z, B4.w}, cc[4] = {C4.x, C4.y, C4.z, C4.w};
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    S[k + x] = fmaf(expf(dt * a[k + x]), S[k + x], __fmul_rn(dx, bb[x]));      // written out: every instance rounds alike
+                    if (PASS != 1) part = fmaf(S[k + x], cc[x], part);
                 }
             }
             if (PASS == 1) return;
             part += __shfl_xor_sync(0xffffffffu, part, 1);
             part += __shfl_xor_sync(0xffffffffu, part, 2);
             if (lane == 0 && live)
-                out[(size_t)(tb + tt) * inner + c] = from_f<TA>((part + dd * xv) * s_z[tt * SCAN_CH + cl]);
+                out[(size_t)(tb + tt) * inner + c] = from_f<TA>(fmaf(dd, xv, part) * s_z[tt * SCAN_CH + cl]);
         };
-        if (nt == SCAN_TOK) {
+        if (nt == TOK) {
 #pragma unroll 4
-            for (int tt = 0; tt < SCAN_TOK; ++tt) token(tt);
+            for (int tt = 0; tt < TOK; ++tt) token(tt);
         } else {
             for (int tt = 0; tt < nt; ++tt) token(tt);
         }
@@ -230,7 +320,7 @@ selective_scan_kernel(const TA* x, const float* xz, long long ld_xz, const float
         float* to = seg.carry + (size_t)item * inner * N;
 #pragma unroll
         for (int k = 0; k < NPT; ++k) {
-            const int n = lane + SCAN_LANES * k;
+            const int n = lane * NPT + k;
             if (n < N) to[(size_t)c * N + n] = S[k];
         }
         if (lane == 0) seg.decay[(size_t)item * inner + c] = sum_dt;
@@ -239,7 +329,7 @@ selective_scan_kernel(const TA* x, const float* xz, long long ld_xz, const float
     if (!last) return;
 #pragma unroll
     for (int k = 0; k < NPT; ++k) {
-        const int n = lane + SCAN_LANES * k;
+        const int n = lane * NPT + k;
         if (n < N) st[(size_t)c * N + n] = S[k];
     }
     if (lane == 0 && taps > 1) {
@@ -272,7 +362,7 @@ scan_combine_kernel(const float* state, long long slot_stride, const int* __rest
     float* keep = seg.carry + (size_t)(item0 + n_it - 1) * inner * N;
 #pragma unroll
     for (int k = 0; k < NPT; ++k) {
-        const int n = lane + SCAN_LANES * k;
+        const int n = lane * NPT + k;
         S[k] = n < N ? st[(size_t)c * N + n] : 0.f;
         a[k] = n < N ? A[(size_t)c * N + n] : 0.f;
         if (n < N) keep[(size_t)c * N + n] = S[k];
@@ -282,7 +372,7 @@ scan_combine_kernel(const float* state, long long slot_stride, const int* __rest
         const float sum_dt = seg.decay[(size_t)it * inner + c];
 #pragma unroll
         for (int k = 0; k < NPT; ++k) {
-            const int n = lane + SCAN_LANES * k;
+            const int n = lane * NPT + k;
             if (n < N) {
                 S[k] = expf(sum_dt * a[k]) * S[k] + C[(size_t)c * N + n];
                 C[(size_t)c * N + n] = S[k];
@@ -292,42 +382,48 @@ scan_combine_kernel(const float* state, long long slot_stride, const int* __rest
 }
 
 template <typename TA, int NPT>
-static int launch_scan(int n_requests, size_t smem, cudaStream_t stream, const void* x, const float* xz, long long ld_xz,
+static int launch_scan(int n_requests, cudaStream_t stream, const void* x, const float* xz, long long ld_xz,
                        const float* low, long long ld_low, int b_off, int c_off, const float* dtr, const float* dt_b,
                        const float* A, const float* Dp, float* state, long long slot_stride, long long conv_off,
-                       const int* cu_q, const int* slots, void* out, int inner, int N, int taps, const TimeSegments& seg) {
+                       const int* cu_q, const int* slots, void* out, int inner, int N, int taps, int one_token,
+                       const TimeSegments& seg) {
     const int cols = (inner + SCAN_CH - 1) / SCAN_CH;
 #define SCAN_ARGS (const TA*)x, xz, ld_xz, low, ld_low, b_off, c_off, dtr, dt_b, A, Dp, state, slot_stride, conv_off, cu_q, \
                   slots, (TA*)out, inner, N, taps, seg
+    const auto bytes = [](int tok) { return (size_t)(3 * tok * SCAN_CH + tok * 2 * SCAN_LANES * NPT) * sizeof(float); };
+    const size_t smem = bytes(SCAN_TOK);
+    if (one_token)
+        return rllm_launch(selective_scan_kernel<TA, NPT, 0, 1>, dim3(cols, n_requests), dim3(SCAN_THREADS), bytes(1), stream, SCAN_ARGS);
     if (seg.n_items <= 0)
-        return rllm_launch(selective_scan_kernel<TA, NPT, 0>, dim3(cols, n_requests), dim3(SCAN_THREADS), smem, stream, SCAN_ARGS);
-    int st = rllm_launch(selective_scan_kernel<TA, NPT, 1>, dim3(cols, seg.n_items), dim3(SCAN_THREADS), smem, stream, SCAN_ARGS);
+        return rllm_launch(selective_scan_kernel<TA, NPT, 0, SCAN_TOK>, dim3(cols, n_requests), dim3(SCAN_THREADS), smem, stream, SCAN_ARGS);
+    int st = rllm_launch(selective_scan_kernel<TA, NPT, 1, SCAN_TOK>, dim3(cols, seg.n_items), dim3(SCAN_THREADS), smem, stream, SCAN_ARGS);
     if (st) return st;
     st = rllm_launch(scan_combine_kernel<NPT>, dim3(cols, n_requests), dim3(SCAN_THREADS), 0, stream, (const float*)state,
                      slot_stride, slots, A, inner, N, seg);
     if (st) return st;
-    return rllm_launch(selective_scan_kernel<TA, NPT, 2>, dim3(cols, seg.n_items), dim3(SCAN_THREADS), smem, stream, SCAN_ARGS);
+    return rllm_launch(selective_scan_kernel<TA, NPT, 2, SCAN_TOK>, dim3(cols, seg.n_items), dim3(SCAN_THREADS), smem, stream, SCAN_ARGS);
 #undef SCAN_ARGS
 }
 
 // seg_* / carry / decay: the cut along time (TimeSegments; n_items 0: none).  carry needs n_items * inner * N
-// floats, decay n_items * inner.
+// floats, decay n_items * inner.  one_token: every request brings exactly one token (a decode step).  A chunk is then one
+// token, so that nothing is done for the fifteen that are not there: the same sums, 8 requests of 8,192 channels of 16
+// states 20.8 -> 8.4 us.
 RLLM_API int rllm_selective_scan(const void* x, int act_dt, const float* xz, long long ld_xz, const float* low,
                                  long long ld_low, int b_off, int c_off, const float* dtr, const float* dt_b,
                                  const float* A, const float* Dp, float* state, long long slot_stride,
                                  long long conv_off, const int* cu_q, const int* slots, void* out, int n_requests,
                                  int inner, int N, int taps, const int* seg_t0, const int* seg_t1, const int* seg_req,
                                  const int* seg_flags, const int* req_item0, const int* req_items, int n_items,
-                                 float* carry, float* decay, cudaStream_t stream) {
+                                 float* carry, float* decay, int one_token, cudaStream_t stream) {
     if (n_requests <= 0) return 0;
     if (N <= 0 || N > SCAN_LANES * 64 || inner <= 0 || taps < 1) return (int)cudaErrorInvalidValue;
     TimeSegments seg = {seg_t0, seg_t1, seg_req, seg_flags, req_item0, req_items, carry, decay, n_items};
     if (n_items > 0 && (!seg_t0 || !seg_t1 || !seg_req || !seg_flags || !req_item0 || !req_items || !carry || !decay))
         return (int)cudaErrorInvalidValue;
-    const size_t smem = (size_t)(3 * SCAN_TOK * SCAN_CH + SCAN_TOK * 2 * N) * sizeof(float);
 #define LAUNCH(TA, NPT)                                                                                          \
-    return launch_scan<TA, NPT>(n_requests, smem, stream, x, xz, ld_xz, low, ld_low, b_off, c_off, dtr, dt_b, A, Dp, \
-                                state, slot_stride, conv_off, cu_q, slots, out, inner, N, taps, seg)
+    return launch_scan<TA, NPT>(n_requests, stream, x, xz, ld_xz, low, ld_low, b_off, c_off, dtr, dt_b, A, Dp, \
+                                state, slot_stride, conv_off, cu_q, slots, out, inner, N, taps, one_token, seg)
 #define BY_N(TA)                                                                                                 \
     do {                                                                                                         \
         if (N <= SCAN_LANES * 4) { LAUNCH(TA, 4); }                                                              \
@@ -346,6 +442,46 @@ RLLM_API int rllm_selective_scan(const void* x, int act_dt, const float* xz, lon
 // out[s][t, c] = h[t, c] + (prev(t)[c] - h[t, c]) * mu[s][c] for s < n_streams; prev(t) is the row
 // before t of the same request, or the request's kept row (state) for the first token of its
 // portion -- zeros at the start of a sequence.  The kept row is advanced by the WKV kernel.
+//
+// token_shift4_kernel (rows that can be read four columns at a time): bound by its bytes.  A thread takes four columns of
+// `tok` tokens in a row with the streams' factors in registers, so a row is read once and the factors once per thread;
+// a column at a time, 2,048 x 4,096 to five streams took 65 us, now 20 us.
+#define SHIFT_STREAMS 5        // of the time mixing; other numbers take the plain kernel
+template <typename TA>
+__global__ void __launch_bounds__(ROW4_THREADS)
+token_shift4_kernel(const TA* h, const float* __restrict__ mu, const float* state, long long slot_stride, long long prev_off,
+                    const int* __restrict__ seq_ids, const int* __restrict__ cu_q, const int* __restrict__ slots, TA* out, int n,
+                    int d, int tok) {
+    const int c = (blockIdx.y * ROW4_THREADS + threadIdx.x) * 4;
+    const bool on = c < d;
+    float4 m[SHIFT_STREAMS];
+#pragma unroll
+    for (int s = 0; s < SHIFT_STREAMS; ++s) m[s] = on ? load4(mu + (size_t)s * d + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    pdl_wait();
+    pdl_launch_dependents();
+    if (!on) return;
+    const int ta = blockIdx.x * tok, tb = min(n, ta + tok);
+    float4 prev = make_float4(0.f, 0.f, 0.f, 0.f);
+    int r = -1;
+    for (int t = ta; t < tb; ++t) {
+        const float4 cur = load4(h + (size_t)t * d + c);
+        const int rt = seq_ids[t];
+        if (rt != r) {                                     // a request begins, here or before this block's tokens
+            r = rt;
+            if (t == cu_q[r]) {
+                const float* pv = state + (size_t)slots[r] * slot_stride + prev_off + c;
+                prev = make_float4(pv[0], pv[1], pv[2], pv[3]);
+            } else prev = load4(h + (size_t)(t - 1) * d + c);
+        }
+#pragma unroll
+        for (int s = 0; s < SHIFT_STREAMS; ++s)
+            store4(out + ((size_t)s * n + t) * d + c,
+                   make_float4(cur.x + (prev.x - cur.x) * m[s].x, cur.y + (prev.y - cur.y) * m[s].y,
+                               cur.z + (prev.z - cur.z) * m[s].z, cur.w + (prev.w - cur.w) * m[s].w));
+        prev = cur;
+    }
+}
+
 template <typename TA>
 __global__ void token_shift_kernel(const TA* h, const float* __restrict__ mu, const float* state,
                                    long long slot_stride, long long prev_off, const int* __restrict__ seq_ids,
@@ -369,6 +505,15 @@ RLLM_API int rllm_token_shift(const void* h, int act_dt, const float* mu, const 
                               long long prev_off, const int* seq_ids, const int* cu_q, const int* slots, void* out,
                               int n, int d, int n_streams, cudaStream_t stream) {
     if (n <= 0) return 0;
+    if (n_streams == SHIFT_STREAMS && d % 4 == 0 && ((uintptr_t)h | (uintptr_t)mu | (uintptr_t)out) % 16 == 0) {
+        const int tok = row4_tokens(n, d);
+        const dim3 grid4((n + tok - 1) / tok, (d / 4 + ROW4_THREADS - 1) / ROW4_THREADS);
+        if (act_dt == RLLM_F32)
+            return rllm_launch(token_shift4_kernel<float>, grid4, dim3(ROW4_THREADS), 0, stream, (const float*)h, mu, state,
+                               slot_stride, prev_off, seq_ids, cu_q, slots, (float*)out, n, d, tok);
+        return rllm_launch(token_shift4_kernel<bf16>, grid4, dim3(ROW4_THREADS), 0, stream, (const bf16*)h, mu, state,
+                           slot_stride, prev_off, seq_ids, cu_q, slots, (bf16*)out, n, d, tok);
+    }
     // few tokens (a decode step): the row is spread over several blocks; many: a block per row
     // (2,048 x 4,096: 62 us against 81 with sixteen blocks a row)
     const dim3 grid(n, n >= 256 ? 1 : (d + 255) / 256 > 32 ? 32 : (d + 255) / 256);
@@ -387,10 +532,11 @@ RLLM_API int rllm_token_shift(const void* h, int act_dt, const float* mu, const 
 // norm weight and by silu(gate), and stored in the activation type.  The bonus term is the same
 // number for every value channel, o[j] = sum_i r[i] S[i][j] + (sum_i r[i] u[i] k[i]) * v[j], and is
 // worked out once per token.
-// A thread owns an eighth of the key channels (DMAX / 8) of two neighbouring value channels of the
-// state, in registers: r, k and w are read once for both columns (the kernel is bound by those
-// reads), and the WKV_PARTS lanes that share a pair of columns add their partial sums in a fixed
-// butterfly.  Tokens are taken WKV_TOK at a time: r, k, the decay (exponentials done on the way in),
+// A thread owns an eighth of the key channels (DMAX / 8) of four neighbouring value channels of the
+// state (two for heads of 256), in registers: r, k and w are read once for all of them (the kernel is
+// bound by those reads: with two columns, 7 reads of 16 bytes for 48 FMA, pass 1 / pass 2 of 2,048
+// tokens x 64 heads took 194 / 272 us, with four WKVP us), and the WKV_PARTS lanes that share
+// columns add their partial sums in a fixed order.  Tokens are taken a chunk at a time: r, k, the decay (exponentials done on the way in),
 // v and the gate of a chunk lie in shared memory (rows padded with zeros to DMAX, read four at a
 // time), the next chunk's values are already on their way from global memory (held in registers)
 // while this one is worked through, and the chunk's outputs are normalised by the warps in turn.
@@ -404,24 +550,29 @@ RLLM_API int rllm_token_shift(const void* h, int act_dt, const float* mu, const 
 // the request's state).  Twice the arithmetic, as many blocks as segments x heads.  The sums inside a
 // segment run in the same order as without the cut; across the cut they are associated differently,
 // which moves results by rounding only.
-#define WKV_TOK 16
 #define WKV_PARTS 8
-#define WKV_COLS 2
+// value columns a thread holds, and tokens per chunk (what a thread fetches ahead of a chunk lies in registers)
+__host__ __device__ constexpr int wkv_cols(int dmax) { return dmax <= 128 ? 4 : 2; }
+__host__ __device__ constexpr int wkv_tok(int dmax) { return dmax <= 128 ? 8 : 2; }
+// key channel of a thread's register ii: runs of four, so that the eight parts' 16-byte reads of a row lie side by side
+__device__ __forceinline__ int wkv_channel(int part, int ii) { return (ii / 4) * (4 * WKV_PARTS) + part * 4 + ii % 4; }
+__host__ __device__ constexpr int wkv_threads(int dmax) { return WKV_PARTS * dmax / wkv_cols(dmax); }
 
 // PASS 0: whole requests.  1: end state from a zero start and the product of the decays, no output.
 // 2: from the carried start state, with output.
-template <typename TA, int DMAX, int PASS>
-__global__ void __launch_bounds__(WKV_PARTS * DMAX / WKV_COLS, DMAX <= 64 ? 4 : 1)
+template <typename TA, int DMAX, int PASS, int TOK>
+__global__ void __launch_bounds__(wkv_threads(DMAX), DMAX <= 64 ? 4 : 1)
 wkv_kernel(const float* rp, const float* kp, const float* vp, const float* wraw, const float* gp, long long ld,
            const float* __restrict__ w0, const float* __restrict__ u, const float* __restrict__ norm_w, float eps,
            float* state, long long slot_stride, long long prev_off, const TA* h, int width,
            const int* __restrict__ cu_q, const int* __restrict__ slots, TA* out, int H, int D,
            const TimeSegments seg) {
     constexpr int IPT = DMAX / WKV_PARTS;               // key channels per thread
-    constexpr int NT = WKV_PARTS * DMAX / WKV_COLS;     // threads
-    constexpr int TD = WKV_TOK * DMAX;
-    constexpr int PRE = 5 * TD / NT;                    // values a thread brings in per chunk
-    extern __shared__ __align__(16) float sm_wkv[];      // r, k, w, v, gate: [5][WKV_TOK][DMAX]; o: [WKV_TOK][DMAX]; u: [DMAX]; bonus: [WKV_TOK]
+    constexpr int COLS = wkv_cols(DMAX);                // neighbouring value channels per thread
+    constexpr int NT = wkv_threads(DMAX);
+    constexpr int TD = TOK * DMAX;
+    constexpr int PRE = (5 * TD + NT - 1) / NT;         // values a thread brings in per chunk
+    extern __shared__ __align__(16) float sm_wkv[];      // r, k, w, v, gate: [5][TOK][DMAX]; o: [TOK][DMAX]; u: [DMAX]; bonus: [TOK]
     float* s_r = sm_wkv;
     float* s_k = s_r + TD;
     float* s_w = s_k + TD;
@@ -430,7 +581,7 @@ wkv_kernel(const float* rp, const float* kp, const float* vp, const float* wraw,
     float* s_o = s_g + TD;
     float* s_u = s_o + TD;
     float* s_c = s_u + DMAX;
-    const int tid = threadIdx.x, j0 = WKV_COLS * (tid / WKV_PARTS), part = tid % WKV_PARTS;
+    const int tid = threadIdx.x, j0 = COLS * (tid / WKV_PARTS), part = tid % WKV_PARTS;
     const int head = blockIdx.x, item = blockIdx.y;
     const size_t col = (size_t)head * D;
     for (int i = tid; i < DMAX; i += NT) s_u[i] = i < D ? u[col + i] : 0.f;
@@ -442,9 +593,8 @@ wkv_kernel(const float* rp, const float* kp, const float* vp, const float* wraw,
     if (PASS == 1 && last) return;                       // its end state comes out of pass 2
     float* st = state + (size_t)slots[r] * slot_stride;
     float* Sg = st + (size_t)head * DMAX * DMAX;
-    const int i0 = part * IPT;
-    // key channels i0 .. i0 + IPT of the value channels j0 and j0 + 1; what lies beyond D stays zero
-    float S0[IPT], S1[IPT], cw[PASS == 1 ? IPT : 1];
+    // key channels wkv_channel(part, 0 .. IPT) of the value channels j0 .. j0 + COLS; what lies beyond D stays zero
+    float S[IPT][COLS], cw[PASS == 1 ? IPT : 1];
     {
         // A request's start state: in its slot; with several segments the combine step has put a copy
         // where the last segment's local state would be, because the last segment overwrites the slot
@@ -453,36 +603,36 @@ wkv_kernel(const float* rp, const float* kp, const float* vp, const float* wraw,
         const float* from = (first && last) ? Sg : seg.carry + ((size_t)src * H + head) * DMAX * DMAX;
 #pragma unroll
         for (int ii = 0; ii < IPT; ++ii) {
-            S0[ii] = PASS == 1 ? 0.f : from[(size_t)(2 * ii) * NT + tid];
-            S1[ii] = PASS == 1 ? 0.f : from[(size_t)(2 * ii + 1) * NT + tid];
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) S[ii][c] = PASS == 1 ? 0.f : from[(size_t)(COLS * ii + c) * NT + tid];
             if (PASS == 1) cw[ii] = 1.f;
         }
     }
     float pre[PRE];
     auto fetch = [&](int tb) {
-        const int nt = min(WKV_TOK, t1 - tb);
+        const int nt = min(TOK, t1 - tb);
 #pragma unroll
         for (int x = 0; x < PRE; ++x) {
             const int e = tid + x * NT;
             const int arr = e / TD, rem = e % TD, tt = rem / DMAX, cc = rem % DMAX;
             const float* src = arr == 0 ? rp : arr == 1 ? kp : arr == 2 ? wraw : arr == 3 ? vp : gp;
-            pre[x] = (tt < nt && cc < D) ? src[(size_t)(tb + tt) * ld + col + cc] : 0.f;
+            pre[x] = (e < 5 * TD && tt < nt && cc < D) ? src[(size_t)(tb + tt) * ld + col + cc] : 0.f;
         }
     };
     const int warp = tid >> 5, lane = tid & 31;
     constexpr int n_warps = NT / 32;
     // the chunk's values into shared memory, then the bonus sums of its tokens, a warp per token
-    auto stash = [&]() {
+    auto stash = [&](int nt) {
 #pragma unroll
         for (int x = 0; x < PRE; ++x) {
             const int e = tid + x * NT;
             const int arr = e / TD, cc = e % DMAX;
             float v = pre[x];
-            if (arr == 2) v = cc < D ? expf(-expf(v + w0[col + cc])) : 0.f;
-            sm_wkv[e] = v;
+            if (arr == 2) v = e % TD / DMAX >= nt ? 1.f : cc < D ? expf(-expf(v + w0[col + cc])) : 0.f;
+            if (e < 5 * TD) sm_wkv[e] = v;
         }
         __syncthreads();
-        for (int tt = warp; tt < WKV_TOK; tt += n_warps) {
+        for (int tt = warp; tt < TOK; tt += n_warps) {
             float c = 0.f;
             for (int i = lane; i < D; i += 32) c += s_r[tt * DMAX + i] * s_u[i] * s_k[tt * DMAX + i];
             c = warp_sum(c);
@@ -491,50 +641,72 @@ wkv_kernel(const float* rp, const float* kp, const float* vp, const float* wraw,
     };
     if (t0 < t1) fetch(t0);
     __syncthreads();                                     // s_u is there
-    if (t0 < t1) stash();
+    if (t0 < t1) stash(min(TOK, t1 - t0));
     __syncthreads();
-    for (int tb = t0; tb < t1; tb += WKV_TOK) {
-        const int nt = min(WKV_TOK, t1 - tb);
-        const bool more = tb + WKV_TOK < t1;
-        if (more) fetch(tb + WKV_TOK);
-        // One token: only S carries over from the token before, so with the loop unrolled the loads and
-        // products of neighbouring tokens overlap.
+    for (int tb = t0; tb < t1; tb += TOK) {
+        const int nt = min(TOK, t1 - tb);
+        const bool more = tb + TOK < t1;
+        if (more) fetch(tb + TOK);
+        // One token: only S carries over from the token before.  The loop is unrolled and a token's output stays in a
+        // register until the chunk's end (a store to shared memory would hold back the next token's loads), so
+        // neighbouring tokens overlap.  Places behind the last token have zero keys and a decay of one.
+        float keep[TOK];
+        int mycol = 0;                                     // the lane's column of the thread's COLS
         auto token = [&](int tt) {
-            const float2 vj = *reinterpret_cast<const float2*>(s_v + tt * DMAX + j0);
-            const float4* r4 = reinterpret_cast<const float4*>(s_r + tt * DMAX + i0);
-            const float4* k4 = reinterpret_cast<const float4*>(s_k + tt * DMAX + i0);
-            const float4* w4 = reinterpret_cast<const float4*>(s_w + tt * DMAX + i0);
-            float a0 = 0.f, a1 = 0.f, b0 = 0.f, b1 = 0.f;
+            float vj[COLS];
+#pragma unroll
+            for (int c = 0; c < COLS; c += 2) {
+                const float2 v2 = *reinterpret_cast<const float2*>(s_v + tt * DMAX + j0 + c);
+                vj[c] = v2.x; vj[c + 1] = v2.y;
+            }
+            const float4* r4 = reinterpret_cast<const float4*>(s_r + tt * DMAX + part * 4);
+            const float4* k4 = reinterpret_cast<const float4*>(s_k + tt * DMAX + part * 4);
+            const float4* w4 = reinterpret_cast<const float4*>(s_w + tt * DMAX + part * 4);
+            float acc[2][COLS];                            // even and odd key channels
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) acc[0][c] = acc[1][c] = 0.f;
 #pragma unroll
             for (int q = 0; q < IPT / 4; ++q) {
-                const float4 rr = r4[q], kk = k4[q], ww = w4[q];
-#define WKV_STEP(R, K, W, I, A, B)                                   \
-                if (PASS != 1) { A += R * S0[I]; B += R * S1[I]; }   \
-                else cw[I] *= W;                                     \
-                S0[I] = W * S0[I] + K * vj.x; S1[I] = W * S1[I] + K * vj.y;
-                WKV_STEP(rr.x, kk.x, ww.x, 4 * q, a0, b0)
-                WKV_STEP(rr.y, kk.y, ww.y, 4 * q + 1, a1, b1)
-                WKV_STEP(rr.z, kk.z, ww.z, 4 * q + 2, a0, b0)
-                WKV_STEP(rr.w, kk.w, ww.w, 4 * q + 3, a1, b1)
-#undef WKV_STEP
+                const float4 k_ = k4[q * WKV_PARTS], w_ = w4[q * WKV_PARTS], r_ = PASS != 1 ? r4[q * WKV_PARTS] : k_;
+                const float rr[4] = {r_.x, r_.y, r_.z, r_.w}, kk[4] = {k_.x, k_.y, k_.z, k_.w}, ww[4] = {w_.x, w_.y, w_.z, w_.w};
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    if (PASS == 1) cw[4 * q + x] *= ww[x];
+#pragma unroll
+                    for (int c = 0; c < COLS; ++c) {
+                        float& s = S[4 * q + x][c];
+                        if (PASS != 1) acc[x & 1][c] = fmaf(rr[x], s, acc[x & 1][c]);
+                        s = fmaf(ww[x], s, __fmul_rn(kk[x], vj[c]));       // written out: every instance rounds alike
+                    }
+                }
             }
             if (PASS == 1) return;
-            float oa = a0 + a1, ob = b0 + b1;
+            // the eight parts' sums: each exchange halves the columns that a lane goes on with
+            float o[COLS];
 #pragma unroll
-            for (int m = 1; m < WKV_PARTS; m <<= 1) {
-                oa += __shfl_xor_sync(0xffffffffu, oa, m);
-                ob += __shfl_xor_sync(0xffffffffu, ob, m);
+            for (int c = 0; c < COLS; ++c) o[c] = acc[0][c] + acc[1][c];
+            int m = 1;
+            mycol = 0;
+#pragma unroll
+            for (int left = COLS / 2; left > 0; left >>= 1, m <<= 1) {
+                const bool upper = part & m;
+#pragma unroll
+                for (int c = 0; c < left; ++c) {
+                    const float give = upper ? o[c] : o[c + left], mine = upper ? o[c + left] : o[c];
+                    o[c] = mine + __shfl_xor_sync(0xffffffffu, give, m);
+                }
+                if (upper) mycol += left;
             }
-            if (part == 0) {
-                const float c = s_c[tt];
-                *reinterpret_cast<float2*>(s_o + tt * DMAX + j0) = make_float2(oa + c * vj.x, ob + c * vj.y);
-            }
+#pragma unroll
+            for (; m < WKV_PARTS; m <<= 1) o[0] += __shfl_xor_sync(0xffffffffu, o[0], m);
+            keep[tt] = o[0];
         };
-        if (nt == WKV_TOK) {
-#pragma unroll 2
-            for (int tt = 0; tt < WKV_TOK; ++tt) token(tt);
-        } else {
-            for (int tt = 0; tt < nt; ++tt) token(tt);
+#pragma unroll
+        for (int tt = 0; tt < TOK; ++tt) token(tt);
+        if (PASS != 1 && part < COLS) {
+#pragma unroll
+            for (int tt = 0; tt < TOK; ++tt) s_o[tt * DMAX + j0 + mycol] =
+                fmaf(s_c[tt], s_v[tt * DMAX + j0 + mycol], keep[tt]);
         }
         __syncthreads();
         for (int tt = warp; PASS != 1 && tt < nt; tt += n_warps) {
@@ -546,119 +718,116 @@ wkv_kernel(const float* rp, const float* kp, const float* vp, const float* wraw,
                     from_f<TA>(s_o[tt * DMAX + i] * rs * norm_w[col + i] * silu_f(s_g[tt * DMAX + i]));
         }
         __syncthreads();                                 // everyone is done with this chunk
-        if (more) stash();
+        if (more) stash(min(TOK, t1 - tb - TOK));
         __syncthreads();
     }
     if (PASS == 1) {
         float* to = seg.carry + ((size_t)item * H + head) * DMAX * DMAX;
 #pragma unroll
         for (int ii = 0; ii < IPT; ++ii) {
-            to[(size_t)(2 * ii) * NT + tid] = S0[ii];
-            to[(size_t)(2 * ii + 1) * NT + tid] = S1[ii];
-            if (tid < WKV_PARTS) seg.decay[((size_t)item * H + head) * DMAX + i0 + ii] = cw[ii];
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) to[(size_t)(COLS * ii + c) * NT + tid] = S[ii][c];
+            if (tid < WKV_PARTS) seg.decay[((size_t)item * H + head) * DMAX + wkv_channel(part, ii)] = cw[ii];
         }
         return;
     }
     if (!last) return;
 #pragma unroll
-    for (int ii = 0; ii < IPT; ++ii) {
-        Sg[(size_t)(2 * ii) * NT + tid] = S0[ii];
-        Sg[(size_t)(2 * ii + 1) * NT + tid] = S1[ii];
-    }
-    if (head == 0 && t1 > t0) {
+    for (int ii = 0; ii < IPT; ++ii)
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) Sg[(size_t)(COLS * ii + c) * NT + tid] = S[ii][c];
+    if (t1 > t0) {                                       // the kept row moves on, every head's block its share of the columns
         float* pv = st + prev_off;
-        for (int c = tid; c < width; c += NT) pv[c] = to_f<TA>(h[(size_t)(t1 - 1) * width + c]);
+        for (int c = head * NT + tid; c < width; c += H * NT) pv[c] = to_f<TA>(h[(size_t)(t1 - 1) * width + c]);
     }
 }
 
+#define WKV_COMBINE_THREADS 256
 // Between the passes: a request's segments in order, S_end = decay * S_start + local end state, in place.
 template <int DMAX>
-__global__ void __launch_bounds__(WKV_PARTS * DMAX / WKV_COLS)
+__global__ void __launch_bounds__(WKV_COMBINE_THREADS)
 wkv_combine_kernel(const float* state, long long slot_stride, const int* __restrict__ slots, int H, const TimeSegments seg) {
-    constexpr int IPT = DMAX / WKV_PARTS;
-    constexpr int NT = WKV_PARTS * DMAX / WKV_COLS;
+    constexpr int COLS = wkv_cols(DMAX), NT = wkv_threads(DMAX);
     pdl_wait();
     pdl_launch_dependents();
-    const int tid = threadIdx.x, head = blockIdx.x, r = blockIdx.y;
+    // a thread takes one state value through all segments; reads run ahead of the chain four segments at a time
+    // (16 segments of 64 heads of 64: 40 us with a block per head, now 6 us)
+    const int head = blockIdx.x, r = blockIdx.y;
+    const int e = blockIdx.z * WKV_COMBINE_THREADS + threadIdx.x;      // register * NT + thread of the WKV kernel
     const int n = seg.req_items[r], item0 = seg.req_item0[r];
-    if (n < 2) return;
-    const float* Sg = state + (size_t)slots[r] * slot_stride + (size_t)head * DMAX * DMAX;
-    const int i0 = (tid % WKV_PARTS) * IPT;
-    float S0[IPT], S1[IPT];
+    if (n < 2 || e >= DMAX * DMAX) return;
+    const int i = wkv_channel(e % NT % WKV_PARTS, e / NT / COLS);      // its key channel
+    float S = state[(size_t)slots[r] * slot_stride + (size_t)head * DMAX * DMAX + e];
+    const size_t step = (size_t)H * DMAX * DMAX, wstep = (size_t)H * DMAX;
+    float* C = seg.carry + ((size_t)item0 * H + head) * DMAX * DMAX + e;
+    const float* dec = seg.decay + ((size_t)item0 * H + head) * DMAX + i;
+    C[(n - 1) * step] = S;                                             // the start state, for pass 2
+    for (int it = 0; it < n - 1; it += 4) {
+        float c[4], w[4];
 #pragma unroll
-    for (int ii = 0; ii < IPT; ++ii) {
-        S0[ii] = Sg[(size_t)(2 * ii) * NT + tid];
-        S1[ii] = Sg[(size_t)(2 * ii + 1) * NT + tid];
-    }
-    {
-        float* keep = seg.carry + ((size_t)(item0 + n - 1) * H + head) * DMAX * DMAX;    // the start state, for pass 2
+        for (int x = 0; x < 4; ++x)
+            if (it + x < n - 1) { c[x] = C[(it + x) * step]; w[x] = dec[(it + x) * wstep]; }
 #pragma unroll
-        for (int ii = 0; ii < IPT; ++ii) {
-            keep[(size_t)(2 * ii) * NT + tid] = S0[ii];
-            keep[(size_t)(2 * ii + 1) * NT + tid] = S1[ii];
-        }
-    }
-    for (int it = item0; it < item0 + n - 1; ++it) {
-        float* C = seg.carry + ((size_t)it * H + head) * DMAX * DMAX;
-        const float* dec = seg.decay + ((size_t)it * H + head) * DMAX + i0;
-#pragma unroll
-        for (int ii = 0; ii < IPT; ++ii) {
-            const float w = dec[ii];
-            S0[ii] = w * S0[ii] + C[(size_t)(2 * ii) * NT + tid];
-            S1[ii] = w * S1[ii] + C[(size_t)(2 * ii + 1) * NT + tid];
-            C[(size_t)(2 * ii) * NT + tid] = S0[ii];
-            C[(size_t)(2 * ii + 1) * NT + tid] = S1[ii];
-        }
+        for (int x = 0; x < 4; ++x)
+            if (it + x < n - 1) {
+                S = w[x] * S + c[x];
+                C[(it + x) * step] = S;
+            }
     }
 }
 
-template <typename TA, int DMAX, int PASS>
-static int launch_wkv_pass(dim3 grid, size_t smem, cudaStream_t stream, const float* rp, const float* kp,
+template <typename TA, int DMAX, int PASS, int TOK>
+static int launch_wkv_pass(dim3 grid, cudaStream_t stream, const float* rp, const float* kp,
                            const float* vp, const float* wraw, const float* gp, long long ld, const float* w0,
                            const float* u, const float* norm_w, float eps, float* state, long long slot_stride,
                            long long prev_off, const void* h, int width, const int* cu_q, const int* slots, void* out,
                            int H, int D, const TimeSegments& seg) {
+    const size_t smem = ((size_t)(6 * TOK + 1) * DMAX + TOK) * sizeof(float);
     if (smem > 48 * 1024) {
         static bool raised = false;                      // once per instantiation: more dynamic shared memory than the default
         if (!raised) {
-            cudaError_t e = cudaFuncSetAttribute(wkv_kernel<TA, DMAX, PASS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            cudaError_t e = cudaFuncSetAttribute(wkv_kernel<TA, DMAX, PASS, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)smem);
             if (e != cudaSuccess) return (int)e;
             raised = true;
         }
     }
-    return rllm_launch(wkv_kernel<TA, DMAX, PASS>, grid, dim3(WKV_PARTS * DMAX / WKV_COLS), smem, stream, rp, kp, vp, wraw,
+    return rllm_launch(wkv_kernel<TA, DMAX, PASS, TOK>, grid, dim3(wkv_threads(DMAX)), smem, stream, rp, kp, vp, wraw,
                        gp, ld, w0, u, norm_w, eps, state, slot_stride, prev_off, (const TA*)h, width, cu_q, slots, (TA*)out,
                        H, D, seg);
 }
 
 template <typename TA, int DMAX>
-static int launch_wkv(int n_requests, size_t smem, cudaStream_t stream, const float* rp, const float* kp, const float* vp,
+static int launch_wkv(int n_requests, cudaStream_t stream, const float* rp, const float* kp, const float* vp,
                       const float* wraw, const float* gp, long long ld, const float* w0, const float* u,
                       const float* norm_w, float eps, float* state, long long slot_stride, long long prev_off,
                       const void* h, int width, const int* cu_q, const int* slots, void* out, int H, int D,
-                      const TimeSegments& seg) {
+                      int one_token, const TimeSegments& seg) {
+    constexpr int TOK = wkv_tok(DMAX);
 #define WKV_ARGS rp, kp, vp, wraw, gp, ld, w0, u, norm_w, eps, state, slot_stride, prev_off, h, width, cu_q, slots, out, H, D, seg
+    if (one_token) return launch_wkv_pass<TA, DMAX, 0, 1>(dim3(H, n_requests), stream, WKV_ARGS);
     if (seg.n_items <= 0)
-        return launch_wkv_pass<TA, DMAX, 0>(dim3(H, n_requests), smem, stream, WKV_ARGS);
-    int st = launch_wkv_pass<TA, DMAX, 1>(dim3(H, seg.n_items), smem, stream, WKV_ARGS);
+        return launch_wkv_pass<TA, DMAX, 0, TOK>(dim3(H, n_requests), stream, WKV_ARGS);
+    int st = launch_wkv_pass<TA, DMAX, 1, TOK>(dim3(H, seg.n_items), stream, WKV_ARGS);
     if (st) return st;
-    st = rllm_launch(wkv_combine_kernel<DMAX>, dim3(H, n_requests), dim3(WKV_PARTS * DMAX / WKV_COLS), 0, stream,
+    st = rllm_launch(wkv_combine_kernel<DMAX>, dim3(H, n_requests, (DMAX * DMAX + WKV_COMBINE_THREADS - 1) / WKV_COMBINE_THREADS),
+                     dim3(WKV_COMBINE_THREADS), 0, stream,
                      (const float*)state, slot_stride, slots, H, seg);
     if (st) return st;
-    return launch_wkv_pass<TA, DMAX, 2>(dim3(H, seg.n_items), smem, stream, WKV_ARGS);
+    return launch_wkv_pass<TA, DMAX, 2, TOK>(dim3(H, seg.n_items), stream, WKV_ARGS);
 #undef WKV_ARGS
 }
 
 // seg_* / carry / decay: the cut along time (TimeSegments; n_items 0: none).  carry needs n_items * H * DMAX * DMAX
-// floats, decay n_items * H * DMAX (DMAX as in rllm_wkv_state_floats).
+// floats, decay n_items * H * DMAX (DMAX as in rllm_wkv_state_floats).  one_token: every request brings exactly one
+// token (a decode step): chunks of one token, the same sums; 8 requests of 64 heads of 64 22.8 -> 7.2 us.
 RLLM_API int rllm_wkv(const float* rp, const float* kp, const float* vp, const float* wraw, const float* gp,
                       long long ld, const float* w0, const float* u, const float* norm_w, float eps, float* state,
                       long long slot_stride, long long prev_off, const void* h, int act_dt, int width,
                       const int* cu_q, const int* slots, void* out, int n_requests, int H, int D,
                       const int* seg_t0, const int* seg_t1, const int* seg_req, const int* seg_flags,
                       const int* req_item0, const int* req_items, int n_items, float* carry, float* decay,
-                      cudaStream_t stream) {
+                      int one_token, cudaStream_t stream) {
     if (n_requests <= 0) return 0;
     if (D <= 0 || D > 256 || H <= 0) return (int)cudaErrorInvalidValue;
     const int dmax = D <= 32 ? 32 : D <= 64 ? 64 : D <= 128 ? 128 : 256;
@@ -666,10 +835,9 @@ RLLM_API int rllm_wkv(const float* rp, const float* kp, const float* vp, const f
     TimeSegments seg = {seg_t0, seg_t1, seg_req, seg_flags, req_item0, req_items, carry, decay, n_items};
     if (n_items > 0 && (!seg_t0 || !seg_t1 || !seg_req || !seg_flags || !req_item0 || !req_items || !carry || !decay))
         return (int)cudaErrorInvalidValue;
-    const size_t smem = ((size_t)(6 * WKV_TOK + 1) * dmax + WKV_TOK) * sizeof(float);
 #define LAUNCH(TA, DMAX)                                                                                        \
-    return launch_wkv<TA, DMAX>(n_requests, smem, stream, rp, kp, vp, wraw, gp, ld, w0, u, norm_w, eps, state,  \
-                                slot_stride, prev_off, h, width, cu_q, slots, out, H, D, seg)
+    return launch_wkv<TA, DMAX>(n_requests, stream, rp, kp, vp, wraw, gp, ld, w0, u, norm_w, eps, state,  \
+                                slot_stride, prev_off, h, width, cu_q, slots, out, H, D, one_token, seg)
 #define BY_D(TA)                                                                                               \
     do {                                                                                                       \
         if (dmax == 32) { LAUNCH(TA, 32); }                                                                    \

@@ -71,7 +71,7 @@ class Mamba1(Mixer):
         y = torch.empty((n, I), dtype=dt, device=dev)
         ops.selective_scan(x, xz, low, R, R + N, dtr, self.dt_b, self.A, self.Dp, cache.state, self.conv_off,
                            ctx.cu_q, cache.slots, y, ctx.n_requests, I, N, self.taps,
-                           segments=ops.time_segments(ctx, dev))
+                           segments=ops.time_segments(ctx, dev), one_token=ctx.max_q_len == 1)
         return ops.linear(y, self.w_o, out_dtype=torch.float32)
 
 
