@@ -535,7 +535,7 @@ RLLM_API int rllm_token_shift(const void* h, int act_dt, const float* mu, const 
 // A thread owns an eighth of the key channels (DMAX / 8) of four neighbouring value channels of the
 // state (two for heads of 256), in registers: r, k and w are read once for all of them (the kernel is
 // bound by those reads: with two columns, 7 reads of 16 bytes for 48 FMA, pass 1 / pass 2 of 2,048
-// tokens x 64 heads took 194 / 272 us, with four WKVP us), and the WKV_PARTS lanes that share
+// tokens x 64 heads took 194 / 272 us, with four and conflict-free reads 107 / 240 us), and the WKV_PARTS lanes that share
 // columns add their partial sums in a fixed order.  Tokens are taken a chunk at a time: r, k, the decay (exponentials done on the way in),
 // v and the gate of a chunk lie in shared memory (rows padded with zeros to DMAX, read four at a
 // time), the next chunk's values are already on their way from global memory (held in registers)
