@@ -17,7 +17,7 @@
 //            never of the batch); unnormalized partials (o, m, l) per split that
 //            paged_flash_combine merges in split order.  Two kernels write those partials:
 //            - paged_decode_attention_kernel, tiles of at most 8 (token, head) rows, the product
-//              turned round (keys as the M side of the MMA); one warp per CTA; the default;
+//              turned round (keys as the M side of the MMA); one warp per CTA, or four where the launch is small; the default;
 //            - the 1-warp, 16-row instance of the template for callers with tiles of 9 to 16 rows.
 // K/V tiles come in through cp.async (16-byte chunks, zero-filled beyond the context) into a
 // double buffer with an XOR swizzle on the chunk index, so ldmatrix is free of bank conflicts.
@@ -377,14 +377,22 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
     return d;
 }
 
-template <int HD, int BN, int NS>
-__global__ void __launch_bounds__(32) paged_decode_attention_kernel(const FlashParams p) {
+//
+// With NW > 1 a CTA's warps share a split's keys in runs of whole tiles (a function of the split's own bounds) and merge in
+// shared memory, in the order of the warps: one warp for the 128 keys of a split is a chain of eight tiles behind the chain
+// of index reads, four warps have all tiles of a split in flight at once, before the dependency wait where the keys are old.
+template <int HD, int BN, int NS, int NW>
+__global__ void __launch_bounds__(NW * 32) paged_decode_attention_kernel(const FlashParams p) {
     constexpr int CH = HD / 8;
     constexpr int TILE_BYTES = BN * HD * 2;
     constexpr int KB = BN / 16;                   // blocks of 16 keys per tile
     constexpr int DT = HD / 16;                   // blocks of 16 head dims
-    extern __shared__ __align__(128) unsigned char smem[];   // [NS stages][K tile, V tile]
-    const int lane = threadIdx.x, g = lane >> 2, t = lane & 3;
+    extern __shared__ __align__(128) unsigned char smem_all[];   // per warp [NS stages][K tile, V tile]
+    __shared__ float s_ml[NW][8][2];
+    constexpr int WARP_BYTES = NS * 2 * TILE_BYTES;
+    constexpr int OLD = HD + 4;                   // row stride of the merge: rows 2t of the four t in different banks
+    static_assert(8 * OLD * 4 <= WARP_BYTES, "a warp's partial output takes the place of its tiles");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     // No griddepcontrol.wait yet: the tiles, positions and block tables were uploaded before the
     // step's first kernel, and the keys of earlier steps are in the cache; only the queries and
     // this step's own keys come from the kernels before (see below).
@@ -434,7 +442,7 @@ __global__ void __launch_bounds__(32) paged_decode_attention_kernel(const FlashP
     }
     if (kb >= ke) {                                // an empty split: mark it so
         pdl_wait();                                // the partials of the layer before may still be read
-        if (p.split_keys > 0 && g == 0) {
+        if (warp == 0 && g == 0) {
 #pragma unroll
             for (int x = 0; x < 2; ++x)
                 if (rowc[x] < p.part_rows) {
@@ -444,12 +452,20 @@ __global__ void __launch_bounds__(32) paged_decode_attention_kernel(const FlashP
         }
         return;
     }
+    if (NW > 1) {
+        const int run = (ke - kb + NW * BN - 1) / (NW * BN) * BN;      // this warp's keys of the split
+        kb += warp * run;
+        ke = min(ke, kb + run);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) hic[x] = min(hic[x], ke);
+    }
+    unsigned char* smem = smem_all + warp * WARP_BYTES;
 
     const int* table = p.block_table + (size_t)req * p.table_stride;
     constexpr int ROWS_PER_PASS = 32 / CH;
     static_assert(32 % CH == 0, "a warp must cover whole rows of chunks");
     const int my_chunk = lane % CH, my_row0 = lane / CH;
-    const int last_blk = (ke - 1) / p.bs;
+    const int last_blk = max(ke - 1, 0) / p.bs;
     // Fast path (page size a power of two and at least a tile): a tile lies in one page, so one
     // table look-up and one base address per tile; this lane's rows are my_row0 + i * ROWS_PER_PASS,
     // their swizzled positions are fixed and kept in registers.
@@ -510,15 +526,16 @@ __global__ void __launch_bounds__(32) paged_decode_attention_kernel(const FlashP
     for (int j = 0; j < DT; ++j) { o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f; }
     float mx[2] = {-INFINITY, -INFINITY}, lsum[2] = {0.f, 0.f};
 
-    const int n_tiles = (ke - kb + BN - 1) / BN;
-    // The first NS - 1 tiles are requested before the wait when they hold keys of earlier steps
+    const int n_tiles = max(0, (ke - kb + BN - 1) / BN);
+    constexpr int AHEAD = NW == 1 ? NS - 1 : NS;   // tiles in flight beside the one that is worked on, or with it
+    // The first AHEAD tiles are requested before the wait when they hold keys of earlier steps
     // only (all splits of a request but its last one or two): the kernel starts while the one
     // before it still runs, and its first memory round trip is over when that one ends.
     const int written_from = p.positions[p.cu_q[req]];          // first position this step writes for the request
-    const bool ahead = kb + min(n_tiles, NS - 1) * BN <= written_from;
+    const bool ahead = kb + min(n_tiles, AHEAD) * BN <= written_from;
     if (ahead) {
 #pragma unroll
-        for (int i = 0; i < NS - 1; ++i) {         // NS - 1 tiles ahead; empty groups keep the count uniform
+        for (int i = 0; i < AHEAD; ++i) {          // empty groups keep the count uniform
             if (i < n_tiles) load_tile(i, kb + i * BN);
             cp_async_commit();
         }
@@ -526,7 +543,7 @@ __global__ void __launch_bounds__(32) paged_decode_attention_kernel(const FlashP
     pdl_wait();
     if (!ahead) {
 #pragma unroll
-        for (int i = 0; i < NS - 1; ++i) {
+        for (int i = 0; i < AHEAD; ++i) {
             if (i < n_tiles) load_tile(i, kb + i * BN);
             cp_async_commit();
         }
@@ -551,8 +568,10 @@ __global__ void __launch_bounds__(32) paged_decode_attention_kernel(const FlashP
     const int v_row = (mat >> 1) * 8 + ri, v_ch = mat & 1;
     for (int it = 0; it < n_tiles; ++it) {
         const int kt = kb + it * BN;
-        if (it + NS - 1 < n_tiles) load_tile((it + NS - 1) % NS, kt + (NS - 1) * BN);
-        cp_async_commit();
+        if (NW == 1) {
+            if (it + AHEAD < n_tiles) load_tile((it + AHEAD) % NS, kt + AHEAD * BN);
+            cp_async_commit();
+        }
         cp_async_wait<NS - 1>();
         __syncwarp();
         const unsigned char* sk = smem + (size_t)(it % NS) * 2 * TILE_BYTES;
@@ -629,6 +648,10 @@ __global__ void __launch_bounds__(32) paged_decode_attention_kernel(const FlashP
             }
         }
         __syncwarp();                              // the stage may be overwritten from here on
+        if (NW > 1) {
+            if (it + NS < n_tiles) load_tile(it % NS, kt + NS * BN);
+            cp_async_commit();
+        }
     }
     pdl_launch_dependents();
 #pragma unroll
@@ -637,7 +660,7 @@ __global__ void __launch_bounds__(32) paged_decode_attention_kernel(const FlashP
         lsum[x] += __shfl_xor_sync(0xffffffffu, lsum[x], 8);
         lsum[x] += __shfl_xor_sync(0xffffffffu, lsum[x], 16);
     }
-    if (p.split_keys > 0) {
+    if (NW == 1) {
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
             if (rowc[x] >= p.part_rows) continue;
@@ -649,18 +672,42 @@ __global__ void __launch_bounds__(32) paged_decode_attention_kernel(const FlashP
                 p.part_ml[(part_base + rowc[x]) * 2 + 1] = validc[x] ? lsum[x] : 0.f;
             }
         }
-    } else {
+        return;
+    }
+    // this warp's part of the split, over its tiles; then all threads add the warps' parts in order
+    cp_async_wait<0>();
+    __syncwarp();
+    float* so = reinterpret_cast<float*>(smem);
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
-            if (!validc[x]) continue;
-            lsum[x] += flash_sink_term(p, head0 + hlc[x], mx[x]);
-            const float inv = lsum[x] > 0.f ? 1.0f / lsum[x] : 0.f;
-            bf16* po = p.out + ((size_t)(tok0 + tlc[x]) * p.H + head0 + hlc[x]) * HD;
+    for (int x = 0; x < 2; ++x) {
 #pragma unroll
-            for (int dp = 0; dp < DT; ++dp) {
-                po[16 * dp + g] = from_f<bf16>(o[dp][x] * inv);
-                po[16 * dp + 8 + g] = from_f<bf16>(o[dp][2 + x] * inv);
+        for (int dp = 0; dp < DT; ++dp) {
+            so[rowc[x] * OLD + 16 * dp + g] = o[dp][x];
+            so[rowc[x] * OLD + 16 * dp + 8 + g] = o[dp][2 + x];
+        }
+        if (g == 0) {
+            s_ml[warp][rowc[x]][0] = mx[x];
+            s_ml[warp][rowc[x]][1] = validc[x] ? lsum[x] : 0.f;
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < p.part_rows * HD; i += NW * 32) {
+        const int row = i / HD, d = i % HD;
+        float M = -INFINITY, num = 0.f, den = 0.f;
+#pragma unroll
+        for (int w = 0; w < NW; ++w)
+            if (s_ml[w][row][1] > 0.f) M = fmaxf(M, s_ml[w][row][0]);
+#pragma unroll
+        for (int w = 0; w < NW; ++w)
+            if (s_ml[w][row][1] > 0.f) {
+                const float f = exp2f(s_ml[w][row][0] - M);
+                num = fmaf(reinterpret_cast<const float*>(smem_all + w * WARP_BYTES)[row * OLD + d], f, num);
+                den = fmaf(s_ml[w][row][1], f, den);
             }
+        p.part_o[(part_base + row) * HD + d] = num;
+        if (d == 0) {
+            p.part_ml[(part_base + row) * 2] = M;
+            p.part_ml[(part_base + row) * 2 + 1] = den;
         }
     }
 }
@@ -737,18 +784,29 @@ static int launch_flash(const FlashParams& p, int mode, int n_tiles, int n_split
         if (e != cudaSuccess) return (int)e;
         return rllm_launch(kern, grid, dim3(NW * 32), smem, stream, p);
     }
-    // decode shape: one warp per CTA, the keys-as-M kernel for tiles of at most 8 rows, else the 16-row
-    // instance of the template with a ring of two 32-key tiles.  (A 4-warp variant that split a CTA's
-    // keys and requested them all at once was faster at batch 1 until the 8-row kernel asked for its
-    // first tiles before the dependency wait: 11.3 against 10.6 us; it is gone.)
+    // decode shape: the keys-as-M kernel for tiles of at most 8 rows, else the 16-row instance of the template with a
+    // ring of two 32-key tiles, one warp per CTA.
     int st;
     if (p.part_rows <= 8) {
         // tiles of at most 8 query rows: the keys as the M side of the MMA.  Tiles of 16 keys in a ring
         // of three (24 KB): nine CTAs share an SM, which counts for more here than a deeper ring
         // (measured at batch 8 and 64, context 2,048: 32-key tiles x 2 stages 24.8 / 109 us,
         // 16 x 3: 21.0 / 104, 16 x 4: 25.6 / 112, 32 x 4: 30.8 / 166).
-        constexpr int BN = 16, NS = 3;
-        st = rllm_launch(paged_decode_attention_kernel<HD, BN, NS>, grid, dim3(32), NS * 2 * BN * HD * 2, stream, p);
+        constexpr int BN = 16;
+        if ((long long)grid.x * grid.y * grid.z <= 3 * 148) {
+            // Few CTAs: four warps each, 64 KB, three CTAs an SM.  The line is where they no longer all run at once; then
+            // nine one-warp CTAs an SM keep more in flight.  Whole decode steps, one warp against four (CTAs): 0.6B sizes,
+            // 1 request of 128 tokens 890 -> 731 us (16), 3 of 1,500 971 -> 842 (288), 16 of 400 1,130 / 1,132 (512), 40 of
+            // 600 1,851 / 1,940 (1,920); 8B sizes, 1 of 700 3,288 -> 3,187 (48), 8 of 2,048 3,519 / 3,800 (1,088).
+            constexpr int NS = 2, NW = 4, smem = NW * NS * 2 * BN * HD * 2;
+            auto kern = paged_decode_attention_kernel<HD, BN, NS, NW>;
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            if (e != cudaSuccess) return (int)e;
+            st = rllm_launch(kern, grid, dim3(NW * 32), smem, stream, p);
+        } else {
+            constexpr int NS = 3;
+            st = rllm_launch(paged_decode_attention_kernel<HD, BN, NS, 1>, grid, dim3(32), NS * 2 * BN * HD * 2, stream, p);
+        }
     } else {
         constexpr int BN = 32;
         st = rllm_launch(paged_flash_attention_kernel<HD, 1, BN>, grid, dim3(32), 2 * 2 * BN * HD * 2, stream, p);
