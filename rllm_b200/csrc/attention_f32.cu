@@ -75,7 +75,6 @@ attn_f32_rows_kernel(const float* q, const float* k_cache, const float* v_cache,
     __shared__ float ml[2][A32_WARPS][G];
     __shared__ __align__(16) float os[A32_WARPS][G][HD];
     pdl_wait();
-    pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = tokens[blockIdx.x];
     const int kvh = blockIdx.y / head_chunks, g = H / K, g0 = (blockIdx.y % head_chunks) * G;
@@ -219,7 +218,6 @@ attn_f32_tile_kernel(const float* q, const float* k_cache, const float* v_cache,
     TileShared<HD>& sm = *reinterpret_cast<TileShared<HD>*>(raw);
     constexpr int F4 = HD / 4, C4 = HD / 64;
     pdl_wait();
-    pdl_launch_dependents();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int req = tile_req[blockIdx.x], tok0 = tile_tok0[blockIdx.x];
     const int n_tok = min(TT, cu_q[req + 1] - tok0);
@@ -395,7 +393,7 @@ RLLM_API int rllm_attn_f32_rows(const float* q, const float* k_cache, const floa
     const int g = H / K, G = g >= 3 ? 4 : g, chunks = (g + G - 1) / G;
 #define ROWS(HD, GG)                                                                                                            \
     if (hd == HD && G == GG)                                                                                                    \
-        return rllm_launch(attn_f32_rows_kernel<HD, GG>, dim3(n_tokens, K * chunks), dim3(A32_WARPS * 32), 0, stream, q, k_cache, \
+        return rllm_launch_after(attn_f32_rows_kernel<HD, GG>, dim3(n_tokens, K * chunks), dim3(A32_WARPS * 32), 0, stream, q, k_cache, \
                            v_cache, out, positions, seq_ids, tokens, block_table, table_stride, H, K, chunks, bs, mask, n_pages, \
                            err, sink, slopes);
     ROWS(64, 1) ROWS(64, 2) ROWS(64, 4) ROWS(128, 1) ROWS(128, 2) ROWS(128, 4)
@@ -418,7 +416,7 @@ RLLM_API int rllm_attn_f32_tiles(const float* q, const float* k_cache, const flo
         const int e = (int)cudaFuncSetAttribute(attn_f32_tile_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize,          \
                                                 (int)sizeof(TileShared<HD>));                                                  \
         if (e) return e;                                                                                                       \
-        return rllm_launch(attn_f32_tile_kernel<HD>, dim3(n_tiles, K * head_chunks), dim3(128), sizeof(TileShared<HD>), stream, \
+        return rllm_launch_after(attn_f32_tile_kernel<HD>, dim3(n_tiles, K * head_chunks), dim3(128), sizeof(TileShared<HD>), stream, \
                            q, k_cache, v_cache, out, positions, cu_q, tile_req, tile_tok0, block_table, table_stride, H, K, TT, \
                            GH, head_chunks, bs, mask, n_pages, err, sink, slopes);                                              \
     }

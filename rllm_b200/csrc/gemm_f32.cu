@@ -20,6 +20,9 @@
 // 16 multiply-adds, a block per 64 columns also for a single row): float32 requests of 300 and 161 tokens at the 0.6B
 // sizes with 8 decode steps 259 -> 63 ms; the head of 151,936 x 1,024 for one row 94 us (6.6 TB/s), 4,096 columns of
 // 1,024 for 1,024 rows 30 TFLOP/s.
+//
+// Both are launched behind the kernel before, not early beside its end: they fill the SMs, and blocks that wait there keep
+// the rest of the kernel before from its place (the same requests 39.3 ms launched early, 36.9 ms so).
 #include "common.cuh"
 
 #define F32_CLASSES 32
@@ -50,7 +53,6 @@ gemv_f32_kernel(const float* A, const float* W, float* C, int m, int n, int k, i
                 long long sa, long long sw, long long sc) {
     __shared__ float part[GEMV_WARPS][M * NR][F32_CLASSES + 1];
     pdl_wait();
-    pdl_launch_dependents();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int m0 = blockIdx.y * M;
     A += (size_t)blockIdx.z * sa + (size_t)m0 * lda;
@@ -129,7 +131,6 @@ gemm_f32_kernel(const float* A, const float* W, float* C, int m, int n, int k, i
     constexpr int BM = TY * TM, BN = TX * TN, THREADS = TY * TX, ROWS = BM + BN;
     __shared__ __align__(16) float tile[GEMM_STAGES][ROWS * GEMM_LD];
     pdl_wait();
-    pdl_launch_dependents();
     const int tid = threadIdx.x;
     // a warp covers 4 rows x 8 columns of threads: its stores fill 32-byte sectors
     const int lane = tid & 31, warp = tid >> 5;
@@ -242,9 +243,9 @@ RLLM_API int rllm_gemm_f32_batched(const float* A, const float* W, float* C, int
     {                                                                                                                    \
         const int need = ((n + NR - 1) / NR + GEMV_WARPS - 1) / GEMV_WARPS, most = n_sm * (M >= 4 ? 2 : 3);               \
         dim3 grid(need < most ? need : most, (m + M - 1) / M, batch);                                                     \
-        return vec ? rllm_launch(gemv_f32_kernel<M, NR, U, true>, grid, dim3(GEMV_WARPS * 32), 0, stream, A, W, C, m, n,  \
+        return vec ? rllm_launch_after(gemv_f32_kernel<M, NR, U, true>, grid, dim3(GEMV_WARPS * 32), 0, stream, A, W, C, m, n,  \
                                  k, lda, ldw, ldc, accumulate, sa, sw, sc)                                                \
-                   : rllm_launch(gemv_f32_kernel<M, NR, U, false>, grid, dim3(GEMV_WARPS * 32), 0, stream, A, W, C, m, n, \
+                   : rllm_launch_after(gemv_f32_kernel<M, NR, U, false>, grid, dim3(GEMV_WARPS * 32), 0, stream, A, W, C, m, n, \
                                  k, lda, ldw, ldc, accumulate, sa, sw, sc);                                               \
     }
     if (m <= GEMV_ROWS) {
@@ -257,9 +258,9 @@ RLLM_API int rllm_gemm_f32_batched(const float* A, const float* W, float* C, int
 #define GEMM(TY, TX, TM, TN)                                                                                             \
     {                                                                                                                    \
         dim3 grid((n + TX * TN - 1) / (TX * TN), (m + TY * TM - 1) / (TY * TM), batch);                                   \
-        return vec ? rllm_launch(gemm_f32_kernel<TY, TX, TM, TN, true>, grid, dim3(TY * TX), 0, stream, A, W, C, m, n, k, \
+        return vec ? rllm_launch_after(gemm_f32_kernel<TY, TX, TM, TN, true>, grid, dim3(TY * TX), 0, stream, A, W, C, m, n, k, \
                                  lda, ldw, ldc, accumulate, sa, sw, sc)                                                   \
-                   : rllm_launch(gemm_f32_kernel<TY, TX, TM, TN, false>, grid, dim3(TY * TX), 0, stream, A, W, C, m, n,   \
+                   : rllm_launch_after(gemm_f32_kernel<TY, TX, TM, TN, false>, grid, dim3(TY * TX), 0, stream, A, W, C, m, n,   \
                                  k, lda, ldw, ldc, accumulate, sa, sw, sc);                                               \
     }
     const long long large = (long long)((n + 63) / 64) * ((m + 127) / 128) * batch;
