@@ -378,9 +378,10 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
 }
 
 //
-// With NW > 1 a CTA's warps share a split's keys in runs of whole tiles (a function of the split's own bounds) and merge in
-// shared memory, in the order of the warps: one warp for the 128 keys of a split is a chain of eight tiles behind the chain
-// of index reads, four warps have all tiles of a split in flight at once, before the dependency wait where the keys are old.
+// One warp for the 128 keys of a split is a chain of eight tiles behind the chain of index reads.  With NW > 1 warps all tiles
+// of a split are in flight at once (before the dependency wait where the keys are old), each warp works out the scores of
+// its tiles, and then every warp goes through all tiles' softmax in order, each with the dims of its own: the same
+// operations in the same order as with one warp, so the bits do not depend on which of the two runs.
 template <int HD, int BN, int NS, int NW>
 __global__ void __launch_bounds__(NW * 32) paged_decode_attention_kernel(const FlashParams p) {
     constexpr int CH = HD / 8;
@@ -388,10 +389,11 @@ __global__ void __launch_bounds__(NW * 32) paged_decode_attention_kernel(const F
     constexpr int KB = BN / 16;                   // blocks of 16 keys per tile
     constexpr int DT = HD / 16;                   // blocks of 16 head dims
     extern __shared__ __align__(128) unsigned char smem_all[];   // per warp [NS stages][K tile, V tile]
-    __shared__ float s_ml[NW][8][2];
+    constexpr int GROUP = NW * NS;                // tiles whose keys and values are in shared memory together (NW > 1)
+    constexpr int DW = DT / NW;                   // blocks of dims whose output this warp adds up
+    static_assert(DT % NW == 0, "the warps share the head dims");
+    __shared__ float4 s_sc[NW == 1 ? 1 : GROUP][32];             // scores of a group, in the lanes' order
     constexpr int WARP_BYTES = NS * 2 * TILE_BYTES;
-    constexpr int OLD = HD + 4;                   // row stride of the merge: rows 2t of the four t in different banks
-    static_assert(8 * OLD * 4 <= WARP_BYTES, "a warp's partial output takes the place of its tiles");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     // No griddepcontrol.wait yet: the tiles, positions and block tables were uploaded before the
     // step's first kernel, and the keys of earlier steps are in the cache; only the queries and
@@ -452,20 +454,13 @@ __global__ void __launch_bounds__(NW * 32) paged_decode_attention_kernel(const F
         }
         return;
     }
-    if (NW > 1) {
-        const int run = (ke - kb + NW * BN - 1) / (NW * BN) * BN;      // this warp's keys of the split
-        kb += warp * run;
-        ke = min(ke, kb + run);
-#pragma unroll
-        for (int x = 0; x < 2; ++x) hic[x] = min(hic[x], ke);
-    }
     unsigned char* smem = smem_all + warp * WARP_BYTES;
 
     const int* table = p.block_table + (size_t)req * p.table_stride;
     constexpr int ROWS_PER_PASS = 32 / CH;
     static_assert(32 % CH == 0, "a warp must cover whole rows of chunks");
     const int my_chunk = lane % CH, my_row0 = lane / CH;
-    const int last_blk = max(ke - 1, 0) / p.bs;
+    const int last_blk = (ke - 1) / p.bs;
     // Fast path (page size a power of two and at least a tile): a tile lies in one page, so one
     // table look-up and one base address per tile; this lane's rows are my_row0 + i * ROWS_PER_PASS,
     // their swizzled positions are fixed and kept in registers.
@@ -521,22 +516,22 @@ __global__ void __launch_bounds__(NW * 32) paged_decode_attention_kernel(const F
         }
     };
 
-    float o[DT][4];                                // O^T: (d = 16 dp + g, + 8) x (rows 2t, 2t + 1)
+    float o[DW][4];                                // O^T: (d = 16 (warp * DW + dp) + g, + 8) x (rows 2t, 2t + 1)
 #pragma unroll
-    for (int j = 0; j < DT; ++j) { o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f; }
+    for (int j = 0; j < DW; ++j) { o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f; }
     float mx[2] = {-INFINITY, -INFINITY}, lsum[2] = {0.f, 0.f};
 
-    const int n_tiles = max(0, (ke - kb + BN - 1) / BN);
-    constexpr int AHEAD = NW == 1 ? NS - 1 : NS;   // tiles in flight beside the one that is worked on, or with it
+    const int n_tiles = (ke - kb + BN - 1) / BN;
+    constexpr int AHEAD = NW == 1 ? NS - 1 : NS;   // tiles of this warp in flight beside the one that is worked on, or with it
     // The first AHEAD tiles are requested before the wait when they hold keys of earlier steps
     // only (all splits of a request but its last one or two): the kernel starts while the one
     // before it still runs, and its first memory round trip is over when that one ends.
     const int written_from = p.positions[p.cu_q[req]];          // first position this step writes for the request
-    const bool ahead = kb + min(n_tiles, AHEAD) * BN <= written_from;
+    const bool ahead = kb + min(n_tiles, AHEAD * NW) * BN <= written_from;
     if (ahead) {
 #pragma unroll
         for (int i = 0; i < AHEAD; ++i) {          // empty groups keep the count uniform
-            if (i < n_tiles) load_tile(i, kb + i * BN);
+            if (i * NW + warp < n_tiles) load_tile(i, kb + (i * NW + warp) * BN);
             cp_async_commit();
         }
     }
@@ -544,7 +539,7 @@ __global__ void __launch_bounds__(NW * 32) paged_decode_attention_kernel(const F
     if (!ahead) {
 #pragma unroll
         for (int i = 0; i < AHEAD; ++i) {
-            if (i < n_tiles) load_tile(i, kb + i * BN);
+            if (i * NW + warp < n_tiles) load_tile(i, kb + (i * NW + warp) * BN);
             cp_async_commit();
         }
     }
@@ -566,19 +561,8 @@ __global__ void __launch_bounds__(NW * 32) paged_decode_attention_kernel(const F
     const int mat = lane >> 3, ri = lane & 7;
     const int k_row = (mat & 1) * 8 + ri, k_ch = mat >> 1;
     const int v_row = (mat >> 1) * 8 + ri, v_ch = mat & 1;
-    for (int it = 0; it < n_tiles; ++it) {
-        const int kt = kb + it * BN;
-        if (NW == 1) {
-            if (it + AHEAD < n_tiles) load_tile((it + AHEAD) % NS, kt + AHEAD * BN);
-            cp_async_commit();
-        }
-        cp_async_wait<NS - 1>();
-        __syncwarp();
-        const unsigned char* sk = smem + (size_t)(it % NS) * 2 * TILE_BYTES;
-        const unsigned char* sv = sk + TILE_BYTES;
-
+    auto scores = [&](const unsigned char* sk, float (&s)[KB][4]) {
         // ---- S^T = K Q^T
-        float s[KB][4];
 #pragma unroll
         for (int j = 0; j < KB; ++j) { s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f; }
 #pragma unroll
@@ -591,6 +575,8 @@ __global__ void __launch_bounds__(NW * 32) paged_decode_attention_kernel(const F
                 mma_bf16(s[j], a0, a1, a2, a3, qf[ks][0], qf[ks][1]);
             }
         }
+    };
+    auto attend = [&](float (&s)[KB][4], int kt, const unsigned char* sv) {
         // ---- scale, mask, online softmax over the keys (lanes of equal t hold one column pair)
         const bool need_mask = (kt + BN > min(hic[0], hic[1])) || (kt < max(firstc[0], firstc[1]));
         float tmax[2] = {-INFINITY, -INFINITY};
@@ -632,7 +618,7 @@ __global__ void __launch_bounds__(NW * 32) paged_decode_attention_kernel(const F
         lsum[1] = lsum[1] * al[1] + rs[1];
         if (__any_sync(0xffffffffu, al[0] != 1.f || al[1] != 1.f)) {       // the maxima seldom move after the first tiles
 #pragma unroll
-            for (int j = 0; j < DT; ++j) { o[j][0] *= al[0]; o[j][1] *= al[1]; o[j][2] *= al[0]; o[j][3] *= al[1]; }
+            for (int j = 0; j < DW; ++j) { o[j][0] *= al[0]; o[j][1] *= al[1]; o[j][2] *= al[0]; o[j][3] *= al[1]; }
         }
         // ---- O^T += V^T P^T
 #pragma unroll
@@ -640,17 +626,56 @@ __global__ void __launch_bounds__(NW * 32) paged_decode_attention_kernel(const F
             const uint32_t b0 = movmatrix_trans(pack_bf16(s[j][0], s[j][1]));     // keys 0-7 of the block
             const uint32_t b1 = movmatrix_trans(pack_bf16(s[j][2], s[j][3]));     // keys 8-15
 #pragma unroll
-            for (int dp = 0; dp < DT; ++dp) {
+            for (int dp = 0; dp < DW; ++dp) {
                 const int row = j * 16 + v_row;
                 uint32_t a0, a1, a2, a3;
-                ldsm_x4_t(smem_u32(sv + row * (HD * 2) + (((dp * 2 + v_ch) ^ (row & 7)) << 4)), a0, a1, a2, a3);
+                ldsm_x4_t(smem_u32(sv + row * (HD * 2) + ((((warp * DW + dp) * 2 + v_ch) ^ (row & 7)) << 4)), a0, a1, a2, a3);
                 mma_bf16(o[dp], a0, a1, a2, a3, b0, b1);
             }
         }
-        __syncwarp();                              // the stage may be overwritten from here on
-        if (NW > 1) {
-            if (it + NS < n_tiles) load_tile(it % NS, kt + NS * BN);
+    };
+    if (NW == 1) {
+        for (int it = 0; it < n_tiles; ++it) {
+            const int kt = kb + it * BN;
+            if (it + AHEAD < n_tiles) load_tile((it + AHEAD) % NS, kt + AHEAD * BN);
             cp_async_commit();
+            cp_async_wait<NS - 1>();
+            __syncwarp();
+            const unsigned char* sk = smem + (size_t)(it % NS) * 2 * TILE_BYTES;
+            float s[KB][4];
+            scores(sk, s);
+            attend(s, kt, sk + TILE_BYTES);
+            __syncwarp();                          // the stage may be overwritten from here on
+        }
+    } else {
+        static_assert(NW == 1 || KB == 1, "a tile's scores are one float4 a lane");
+        for (int base = 0; base < n_tiles; base += GROUP) {
+            if (base > 0) {
+                __syncthreads();                   // nobody reads the group before any more
+#pragma unroll
+                for (int i = 0; i < NS; ++i) {
+                    const int at = base + i * NW + warp;
+                    if (at < n_tiles) load_tile(i, kb + at * BN);
+                }
+                cp_async_commit();
+            }
+            cp_async_wait<0>();
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < NS; ++i)
+                if (base + i * NW + warp < n_tiles) {
+                    float s[KB][4];
+                    scores(smem + (size_t)i * 2 * TILE_BYTES, s);
+                    s_sc[i * NW + warp][lane] = make_float4(s[0][0], s[0][1], s[0][2], s[0][3]);
+                }
+            __syncthreads();                       // the group's scores and values are there for every warp
+            const int count = min(GROUP, n_tiles - base);
+            for (int i = 0; i < count; ++i) {
+                const float4 f = s_sc[i][lane];
+                float s[KB][4];
+                s[0][0] = f.x; s[0][1] = f.y; s[0][2] = f.z; s[0][3] = f.w;
+                attend(s, kb + (base + i) * BN, smem_all + (size_t)(i % NW) * WARP_BYTES + (size_t)(i / NW) * 2 * TILE_BYTES + TILE_BYTES);
+            }
         }
     }
     pdl_launch_dependents();
@@ -660,54 +685,15 @@ __global__ void __launch_bounds__(NW * 32) paged_decode_attention_kernel(const F
         lsum[x] += __shfl_xor_sync(0xffffffffu, lsum[x], 8);
         lsum[x] += __shfl_xor_sync(0xffffffffu, lsum[x], 16);
     }
-    if (NW == 1) {
-#pragma unroll
-        for (int x = 0; x < 2; ++x) {
-            if (rowc[x] >= p.part_rows) continue;
-            float* po = p.part_o + (part_base + rowc[x]) * HD;
-#pragma unroll
-            for (int dp = 0; dp < DT; ++dp) { po[16 * dp + g] = o[dp][x]; po[16 * dp + 8 + g] = o[dp][2 + x]; }
-            if (g == 0) {
-                p.part_ml[(part_base + rowc[x]) * 2] = mx[x];
-                p.part_ml[(part_base + rowc[x]) * 2 + 1] = validc[x] ? lsum[x] : 0.f;
-            }
-        }
-        return;
-    }
-    // this warp's part of the split, over its tiles; then all threads add the warps' parts in order
-    cp_async_wait<0>();
-    __syncwarp();
-    float* so = reinterpret_cast<float*>(smem);
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
+        if (rowc[x] >= p.part_rows) continue;
+        float* po = p.part_o + (part_base + rowc[x]) * HD + 16 * warp * DW;
 #pragma unroll
-        for (int dp = 0; dp < DT; ++dp) {
-            so[rowc[x] * OLD + 16 * dp + g] = o[dp][x];
-            so[rowc[x] * OLD + 16 * dp + 8 + g] = o[dp][2 + x];
-        }
-        if (g == 0) {
-            s_ml[warp][rowc[x]][0] = mx[x];
-            s_ml[warp][rowc[x]][1] = validc[x] ? lsum[x] : 0.f;
-        }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < p.part_rows * HD; i += NW * 32) {
-        const int row = i / HD, d = i % HD;
-        float M = -INFINITY, num = 0.f, den = 0.f;
-#pragma unroll
-        for (int w = 0; w < NW; ++w)
-            if (s_ml[w][row][1] > 0.f) M = fmaxf(M, s_ml[w][row][0]);
-#pragma unroll
-        for (int w = 0; w < NW; ++w)
-            if (s_ml[w][row][1] > 0.f) {
-                const float f = exp2f(s_ml[w][row][0] - M);
-                num = fmaf(reinterpret_cast<const float*>(smem_all + w * WARP_BYTES)[row * OLD + d], f, num);
-                den = fmaf(s_ml[w][row][1], f, den);
-            }
-        p.part_o[(part_base + row) * HD + d] = num;
-        if (d == 0) {
-            p.part_ml[(part_base + row) * 2] = M;
-            p.part_ml[(part_base + row) * 2 + 1] = den;
+        for (int dp = 0; dp < DW; ++dp) { po[16 * dp + g] = o[dp][x]; po[16 * dp + 8 + g] = o[dp][2 + x]; }
+        if (warp == 0 && g == 0) {
+            p.part_ml[(part_base + rowc[x]) * 2] = mx[x];
+            p.part_ml[(part_base + rowc[x]) * 2 + 1] = validc[x] ? lsum[x] : 0.f;
         }
     }
 }
@@ -795,9 +781,10 @@ static int launch_flash(const FlashParams& p, int mode, int n_tiles, int n_split
         constexpr int BN = 16;
         if ((long long)grid.x * grid.y * grid.z <= 3 * 148) {
             // Few CTAs: four warps each, 64 KB, three CTAs an SM.  The line is where they no longer all run at once; then
-            // nine one-warp CTAs an SM keep more in flight.  Whole decode steps, one warp against four (CTAs): 0.6B sizes,
-            // 1 request of 128 tokens 890 -> 731 us (16), 3 of 1,500 971 -> 842 (288), 16 of 400 1,130 / 1,132 (512), 40 of
-            // 600 1,851 / 1,940 (1,920); 8B sizes, 1 of 700 3,288 -> 3,187 (48), 8 of 2,048 3,519 / 3,800 (1,088).
+            // nine one-warp CTAs an SM keep more in flight.  Whole decode steps, one warp against four (CTAs): 0.6B sizes, 1
+            // request of 128 tokens 890 -> 789 us (16); 8B sizes, 1 of 700 3,317 -> 3,246 (48).  Beyond the line, with a first
+            // form of the four warps that merged their own partial sums: 16 of 400 1,130 / 1,132 (512), 40 of 600 1,851 / 1,940
+            // (1,920), 8B sizes, 8 of 2,048 3,519 / 3,800 (1,088).
             constexpr int NS = 2, NW = 4, smem = NW * NS * 2 * BN * HD * 2;
             auto kern = paged_decode_attention_kernel<HD, BN, NS, NW>;
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

@@ -48,5 +48,15 @@ def test_decode(hd, H, K, bs, form, copies):
     o.check_device_errors()
     top = max(float(v.abs().max()) for v in vs)
     assert float((out.cpu().double() - want).abs().max()) < 2.0 ** -7 * top
+    # a request alone (four warps a CTA) and in the batch: the same bits
+    at = 0
+    for r in range(9):
+        one = Step([lens[r]], [q_lens[r]])
+        one.start_pos = [lens[r] - q_lens[r]]
+        alone = torch.empty(q_lens[r], H * hd, dtype=torch.bfloat16, device=DEV)
+        o.paged_attention(q[at:at + q_lens[r]].reshape(q_lens[r], -1).to(DEV), kc.to(DEV), vc.to(DEV), alone, one, table[r:r + 1].to(DEV), H,
+                          K, hd, bs, hd ** -0.5, window, keep, None, chunk, cap, dev(sink), dev(slopes))
+        assert torch.equal(alone, out[at:at + q_lens[r]])
+        at += q_lens[r]
     for c in range(1, copies):
         assert torch.equal(out[:n], out[c * n:(c + 1) * n])
