@@ -2,26 +2,32 @@
 // attention_generic.cu computes (masks, caps, slopes and sinks as its head describes them), with float32 arithmetic
 // throughout, for the shapes in which a block per (token, head) that reads its keys from memory by itself is slow.
 //
-// attn_f32_rows_kernel, requests of few tokens: bound by the latency of the key and value reads.  A block per (token,
-// key/value head and up to 4 of its query heads); 16 warps take chunks of 32 keys in turn (chunk c belongs to warp
-// c mod 16), eight lanes read one key's row in whole lines, one softmax per warp, merged in the order of the warps.
+// Both kernels give a token the same bits, so its result depends on its own keys alone: not on the requests around it, not on
+// how its prompt was cut into portions, not on which of the two ran.  The order that they share: keys in chunks of 32 that
+// start at multiples of 32 of the position (those of the kept first keys, then those of the window), and per chunk
+//   a score  eight sums, lane q of eight over the entries 4 (q + 8 x) .. + 3 in ascending order, added as a tree of pairs;
+//   M        the largest score so far, this chunk's included;
+//   the sum  of the weights exp(s - M): four keys 8 apart one after the other, then a tree of pairs over the eight;
+//   o        the weighted values: one chain over the keys for heads of 128, one each over even and odd keys for heads of 64;
+//   l = l * exp(M before - M) + sum,  acc = acc * exp(M before - M) + o   (one fused multiply-add each).
+// A key that a row does not see adds nothing to it, not even where its value is infinite: tiles with masked pairs test the weight.
 //
-// attn_f32_tile_kernel, prompt portions: 32 rows (tokens x query heads of one key/value head) against tiles of 32 keys,
-// which cp.async brings in one tile ahead; a score is a chain over the head's entries, rows of 132 floats keep the
-// reads of eight keys in different banks.  Keys are read once per 32 rows where they were read once per row.
+// attn_f32_rows_kernel: bound by the latency of the key and value reads.  A block per (token, key/value head and up to 4 of its
+// query heads); its warps take one chunk each, eight lanes read one key's row in whole lines, and a round of chunks is
+// merged in order by all threads.  M is known before the weights are worked out (a maximum has no order), so only the
+// merge is a chain.
 //
-// In both kernels chunks and tiles start at multiples of 32 of the key's position, so a token's result depends only on
-// its own keys and on whether its request has few tokens in the step, never on the requests around it.  A key that a row
-// does not see adds nothing to it, not even where its value is infinite: tiles with masked pairs test the weight.
+// attn_f32_tile_kernel: 32 rows (tokens x query heads of one key/value head) against tiles of 32 keys, which cp.async brings
+// in one tile ahead; rows of 132 floats keep the reads of eight keys in different banks.  Keys are read once per 32 rows,
+// but a tile's keys are one chain on one SM, 4.8 us each.
 //
-// Measured (head size 128, 16 query heads on 8): requests of 300 keys, two decoding 108 -> 12 us a layer,
-// portions of 300 and 161 tokens 540 -> 64 us.
+// Measured (head size 128, 16 query heads on 8) against the plain kernel, us a launch: two decoding requests of 300 keys
+// 38 -> 7.0, of 4,096 471 -> 46, 32 of 300 102 -> 17; one portion of 461 tokens 964 -> 89, two of 300 793 -> 61.
 #include "common.cuh"
 #include <math.h>
 
 #define A32_KEYS 32
-#define A32_WARPS 16
-#define A32_HEADS 4
+#define A32_MAX_WARPS 16
 #define A32_ROWS 32
 
 struct F32Mask {
@@ -43,12 +49,15 @@ __device__ __forceinline__ int page_of(const int* table, int p, int bs, int n_pa
     }
     return page;
 }
+// (written out, so that both kernels round alike)
 __device__ __forceinline__ float shape_score(const F32Mask& k, float dot, const float* slopes, int head, int distance) {
-    float s = dot * k.scale;
-    if (k.softcap > 0.f) s = k.softcap * tanhf(s / k.softcap);
-    if (slopes) s -= slopes[head] * (float)distance;
+    float s = __fmul_rn(dot, k.scale);
+    if (k.softcap > 0.f) s = __fmul_rn(k.softcap, tanhf(s / k.softcap));
+    if (slopes) s = fmaf(-slopes[head], (float)distance, s);
     return s;
 }
+// the factor of what was summed up to a largest score of `before` when it has become `now`
+__device__ __forceinline__ float rescale(float before, float now) { return before == -INFINITY ? 0.f : expf(before - now); }
 __device__ __forceinline__ float dot4(float4 a, float4 b, float c) {
     return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, c))));
 }
@@ -60,54 +69,81 @@ __device__ __forceinline__ float4 load_or_zero(const float* cache, long long off
     return v;
 }
 
-// ---------------------------------------------------------------- few tokens
+// ---------------------------------------------------------------- token by token
+
+// dynamic shared memory, in floats: q [G][HD], scores and weights [warps][G][32], o [warps][G][HD], the warps' largest score,
+// factor and sum [3][warps][G]
+static size_t rows_smem(int hd, int G, int warps) { return (size_t)(G * hd + warps * G * (A32_KEYS + hd + 3)) * sizeof(float); }
 
 template <int HD, int G>
-__global__ void __launch_bounds__(A32_WARPS * 32)
+__global__ void __launch_bounds__(A32_MAX_WARPS * 32)
 attn_f32_rows_kernel(const float* q, const float* k_cache, const float* v_cache, float* out, const int* __restrict__ positions,
                      const int* __restrict__ seq_ids, const int* __restrict__ tokens, const int* __restrict__ block_table,
                      int table_stride, int H, int K, int head_chunks, int bs, F32Mask mask, int n_pages, int* err,
                      const float* __restrict__ sink, const float* __restrict__ slopes) {
     constexpr int X = HD / 32;                     // float4 of a key row per lane, eight lanes a key
     constexpr int LPK = HD / 4, KPP = 32 / LPK;    // lanes per value row, value rows at a time
-    constexpr int PB = G >= 2 ? 2 : 4, VB = G >= 4 ? 4 : 8;
-    __shared__ float sc[A32_WARPS][G][A32_KEYS];
-    __shared__ float ml[2][A32_WARPS][G];
-    __shared__ __align__(16) float os[A32_WARPS][G][HD];
+    constexpr int PB = 16 / X;                     // passes (of four keys) whose loads are in flight together
+    constexpr int VB = 16;                         // value rows in flight
+    constexpr int PER = (G * HD + 127) / 128;      // outputs a thread merges, at most (blocks have 128 threads or more)
+    extern __shared__ __align__(16) float shared[];
+    const int threads = blockDim.x, warps = threads >> 5, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float* sq = shared;
+    float* sc = sq + G * HD + warp * (G * A32_KEYS);
+    float* os = sq + G * HD + warps * (G * A32_KEYS);
+    float* s_top = os + warps * (G * HD);
+    float* s_factor = s_top + warps * G;
+    float* s_sum = s_factor + warps * G;
     pdl_wait();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = tokens[blockIdx.x];
     const int kvh = blockIdx.y / head_chunks, g = H / K, g0 = (blockIdx.y % head_chunks) * G;
     const int pos = positions[t], first = first_key(mask, pos);
     const int* table = block_table + (size_t)seq_ids[t] * table_stride;
     const int kept = min(mask.keep_first, first);
+    for (int x = tid; x < G * LPK; x += threads) {
+        const int h = kvh * g + min(g0 + x / LPK, g - 1);
+        reinterpret_cast<float4*>(sq)[x] = reinterpret_cast<const float4*>(q + ((size_t)t * H + h) * HD)[x % LPK];
+    }
+    float m_run[G], acc[PER], l[PER];
+#pragma unroll
+    for (int j = 0; j < G; ++j) m_run[j] = sink ? sink[kvh * g + min(g0 + j, g - 1)] : -INFINITY;
+#pragma unroll
+    for (int r = 0; r < PER; ++r) {
+        acc[r] = 0.f;
+        l[r] = sink ? 1.f : 0.f;
+    }
+    __syncthreads();
 
-    float4 qv[G][X];
+    const int n_kept = (kept + A32_KEYS - 1) / A32_KEYS, c_first = first / A32_KEYS;
+    const int n_chunks = n_kept + pos / A32_KEYS + 1 - c_first;
+    // where the row of this lane's key of chunk c starts, -1: the key is not seen
+    auto row_of = [&](int c, int& p) -> long long {
+        const bool in_kept = c < n_kept;
+        const int lo = in_kept ? 0 : first, hi = in_kept ? kept : pos + 1;
+        p = (in_kept ? c : c_first + c - n_kept) * A32_KEYS + lane;
+        if (c >= n_chunks || p < lo || p >= hi) return -1;
+        return (((long long)page_of(table, p, bs, n_pages, err) * K + kvh) * bs + p % bs) * HD;
+    };
+    int p, p_next;
+    long long off_next = row_of(warp, p_next);
+    for (int base = 0; base < n_chunks; base += warps) {
+        const int n_live = min(warps, n_chunks - base);
+        const bool live = warp < n_live;
+        const long long off = off_next;
+        p = p_next;
+        const bool seen = off >= 0;
+        const uint32_t any = __ballot_sync(0xffffffffu, seen);       // runs of keys of which none is seen are passed over
+        float s[G];
+        float4 v[VB];
+        auto load_values = [&](int i0) {
 #pragma unroll
-    for (int j = 0; j < G; ++j) {
-        const int h = kvh * g + min(g0 + j, g - 1);
-        const float4* row = reinterpret_cast<const float4*>(q + ((size_t)t * H + h) * HD);
-#pragma unroll
-        for (int x = 0; x < X; ++x) qv[j][x] = row[(lane & 7) + 8 * x];
-    }
-    float m_run[G], l_run[G];
-    float4 acc[G];
-#pragma unroll
-    for (int j = 0; j < G; ++j) {
-        m_run[j] = -INFINITY;
-        l_run[j] = 0.f;
-        acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    for (int run = 0; run < 2; ++run) {            // the kept first keys outside the window, then the window
-        const int lo = run == 0 ? 0 : first, hi = run == 0 ? kept : pos + 1;
-        for (int c = lo / A32_KEYS + (warp - lo / A32_KEYS % A32_WARPS + A32_WARPS) % A32_WARPS; c * A32_KEYS < hi; c += A32_WARPS) {
-            const int p = c * A32_KEYS + lane;
-            const bool seen = p >= lo && p < hi;
-            long long off = -1;                    // where the key's row starts, -1: not seen
-            if (seen) off = (((long long)page_of(table, p, bs, n_pages, err) * K + kvh) * bs + p % bs) * HD;
-            // the loads of PB passes are in flight together (a pass: four keys)
+            for (int b = 0; b < VB; ++b)
+                v[b] = load_or_zero(v_cache, __shfl_sync(0xffffffffu, off, i0 + b * KPP + lane / LPK), 4 * (lane % LPK));
+        };
+        if (live) {
 #pragma unroll
             for (int i0 = 0; i0 < 8; i0 += PB) {
+                if (!(any >> (4 * i0) & (uint32_t)((1ull << (4 * PB)) - 1))) continue;
                 float4 kv[PB][X];
 #pragma unroll
                 for (int b = 0; b < PB; ++b) {
@@ -116,78 +152,102 @@ attn_f32_rows_kernel(const float* q, const float* k_cache, const float* v_cache,
                     for (int x = 0; x < X; ++x) kv[b][x] = load_or_zero(k_cache, o, 4 * ((lane & 7) + 8 * x));
                 }
 #pragma unroll
-                for (int b = 0; b < PB; ++b)
+                for (int j = 0; j < G; ++j) {
+                    float d[PB];
 #pragma unroll
-                    for (int j = 0; j < G; ++j) {
-                        float d = 0.f;
+                    for (int b = 0; b < PB; ++b) d[b] = 0.f;
 #pragma unroll
-                        for (int x = 0; x < X; ++x) d = dot4(qv[j][x], kv[b][x], d);
-                        d += __shfl_xor_sync(0xffffffffu, d, 1);
-                        d += __shfl_xor_sync(0xffffffffu, d, 2);
-                        d += __shfl_xor_sync(0xffffffffu, d, 4);
-                        if ((lane & 7) == j) sc[warp][j][4 * (i0 + b) + (lane >> 3)] = d;
+                    for (int x = 0; x < X; ++x) {
+                        const float4 qv = reinterpret_cast<const float4*>(sq)[j * LPK + (lane & 7) + 8 * x];
+#pragma unroll
+                        for (int b = 0; b < PB; ++b) d[b] = dot4(qv, kv[b][x], d[b]);
                     }
+#pragma unroll
+                    for (int b = 0; b < PB; ++b) {
+                        d[b] += __shfl_xor_sync(0xffffffffu, d[b], 1);
+                        d[b] += __shfl_xor_sync(0xffffffffu, d[b], 2);
+                        d[b] += __shfl_xor_sync(0xffffffffu, d[b], 4);
+                        if ((lane & 7) == j) sc[j * A32_KEYS + 4 * (i0 + b) + (lane >> 3)] = d[b];
+                    }
+                }
             }
             __syncwarp();
 #pragma unroll
             for (int j = 0; j < G; ++j) {
-                const float s = seen ? shape_score(mask, sc[warp][j][lane], slopes, kvh * g + min(g0 + j, g - 1), pos - p) : -INFINITY;
-                const float m_new = fmaxf(m_run[j], warp_max(s));
-                const float e = seen ? expf(s - m_new) : 0.f;
-                const float alpha = m_run[j] == -INFINITY ? 0.f : expf(m_run[j] - m_new);
-                l_run[j] = l_run[j] * alpha + warp_sum(e);
-                m_run[j] = m_new;
-                acc[j].x *= alpha; acc[j].y *= alpha; acc[j].z *= alpha; acc[j].w *= alpha;
-                __syncwarp();
-                sc[warp][j][lane] = e;
+                s[j] = seen ? shape_score(mask, sc[j * A32_KEYS + lane], slopes, kvh * g + min(g0 + j, g - 1), pos - p) : -INFINITY;
+                const float top = warp_max(s[j]);
+                if (lane == 0) s_top[warp * G + j] = top;
             }
-            __syncwarp();
+            load_values(0);                        // on their way while the block meets
+        }
+        off_next = row_of(base + warps + warp, p_next);
+        __syncthreads();                           // the round's maxima are there
+#pragma unroll
+        for (int j = 0; j < G; ++j) {
+            const float v = lane < n_live ? s_top[lane * G + j] : -INFINITY;
+            const float before = fmaxf(m_run[j], warp_max(lane < warp ? v : -INFINITY));
+            m_run[j] = fmaxf(m_run[j], warp_max(v));
+            if (live) {
+                const float now = fmaxf(before, s_top[warp * G + j]);
+                sc[j * A32_KEYS + lane] = seen ? expf(s[j] - now) : 0.f;
+                if (lane == 0) s_factor[warp * G + j] = rescale(before, now);
+            }
+        }
+        __syncwarp();
+        if (live) {
+            float4 o[G];
+#pragma unroll
+            for (int j = 0; j < G; ++j) {
+                const float* e = sc + j * A32_KEYS + (lane & 7);
+                float sum = e[0] + e[8] + e[16] + e[24];
+                sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+                if (lane == 0) s_sum[warp * G + j] = sum;
+                o[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
 #pragma unroll
             for (int i0 = 0; i0 < A32_KEYS; i0 += VB * KPP) {
-                float4 v[VB];
-#pragma unroll
-                for (int b = 0; b < VB; ++b)
-                    v[b] = load_or_zero(v_cache, __shfl_sync(0xffffffffu, off, i0 + b * KPP + lane / LPK), 4 * (lane % LPK));
+                if (i0 > 0) {
+                    if (!(any >> i0)) continue;
+                    load_values(i0);
+                }
 #pragma unroll
                 for (int b = 0; b < VB; ++b)
 #pragma unroll
                     for (int j = 0; j < G; ++j) {
-                        const float e = sc[warp][j][i0 + b * KPP + lane / LPK];
-                        acc[j].x = fmaf(e, v[b].x, acc[j].x); acc[j].y = fmaf(e, v[b].y, acc[j].y);
-                        acc[j].z = fmaf(e, v[b].z, acc[j].z); acc[j].w = fmaf(e, v[b].w, acc[j].w);
+                        const float e = sc[j * A32_KEYS + i0 + b * KPP + lane / LPK];
+                        o[j].x = fmaf(e, v[b].x, o[j].x); o[j].y = fmaf(e, v[b].y, o[j].y);
+                        o[j].z = fmaf(e, v[b].z, o[j].z); o[j].w = fmaf(e, v[b].w, o[j].w);
                     }
             }
-            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < G; ++j) {
+                if (KPP == 2) {
+                    o[j].x += __shfl_xor_sync(0xffffffffu, o[j].x, 16); o[j].y += __shfl_xor_sync(0xffffffffu, o[j].y, 16);
+                    o[j].z += __shfl_xor_sync(0xffffffffu, o[j].z, 16); o[j].w += __shfl_xor_sync(0xffffffffu, o[j].w, 16);
+                }
+                if (lane < LPK) *reinterpret_cast<float4*>(os + (warp * G + j) * HD + 4 * lane) = o[j];
+            }
+        }
+        __syncthreads();                           // the round's parts are there; they are written again behind the next barrier but one
+#pragma unroll
+        for (int r = 0; r < PER; ++r) {
+            const int x = tid + r * threads, j = x / HD;
+            if (x >= G * HD) break;
+            for (int w = 0; w < n_live; ++w) {
+                const float f = s_factor[w * G + j];
+                acc[r] = fmaf(acc[r], f, os[w * (G * HD) + x]);
+                l[r] = fmaf(l[r], f, s_sum[w * G + j]);
+            }
         }
     }
+    pdl_launch_dependents();
 #pragma unroll
-    for (int j = 0; j < G; ++j) {
-#pragma unroll
-        for (int o = LPK; o < 32; o <<= 1) {
-            acc[j].x += __shfl_xor_sync(0xffffffffu, acc[j].x, o); acc[j].y += __shfl_xor_sync(0xffffffffu, acc[j].y, o);
-            acc[j].z += __shfl_xor_sync(0xffffffffu, acc[j].z, o); acc[j].w += __shfl_xor_sync(0xffffffffu, acc[j].w, o);
-        }
-        if (lane < LPK) *reinterpret_cast<float4*>(&os[warp][j][4 * lane]) = acc[j];
-        if (lane == 0) {
-            ml[0][warp][j] = m_run[j];
-            ml[1][warp][j] = l_run[j];
-        }
-    }
-    __syncthreads();
-    for (int x = threadIdx.x; x < G * HD; x += A32_WARPS * 32) {
-        const int j = x / HD, d = x % HD, h = kvh * g + g0 + j;
-        if (g0 + j >= g) continue;
-        float m = sink ? sink[h] : -INFINITY;
-        for (int w = 0; w < A32_WARPS; ++w) m = fmaxf(m, ml[0][w][j]);
-        float l = sink ? expf(sink[h] - m) : 0.f, o = 0.f;
-        for (int w = 0; w < A32_WARPS; ++w) {
-            const float lw = ml[1][w][j];
-            if (lw == 0.f) continue;               // no keys: a warp that saw one has a sum that is not zero
-            const float f = expf(ml[0][w][j] - m);
-            l = fmaf(lw, f, l);
-            o = fmaf(os[w][j][d], f, o);
-        }
-        out[((size_t)t * H + h) * HD + d] = o * (1.0f / l);
+    for (int r = 0; r < PER; ++r) {
+        const int x = tid + r * threads, j = x / HD;
+        if (x >= G * HD) break;
+        if (g0 + j < g) out[((size_t)t * H + kvh * g + g0 + j) * HD + x % HD] = acc[r] * (1.0f / l[r]);
     }
 }
 
@@ -209,14 +269,14 @@ struct TileShared {
 };
 
 template <int HD>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, HD == 64 ? 4 : 2)      // as many as shared memory allows
 attn_f32_tile_kernel(const float* q, const float* k_cache, const float* v_cache, float* out, const int* __restrict__ positions,
                      const int* __restrict__ cu_q, const int* __restrict__ tile_req, const int* __restrict__ tile_tok0,
                      const int* __restrict__ block_table, int table_stride, int H, int K, int TT, int GH, int head_chunks, int bs,
                      F32Mask mask, int n_pages, int* err, const float* __restrict__ sink, const float* __restrict__ slopes) {
     extern __shared__ __align__(16) unsigned char raw[];
     TileShared<HD>& sm = *reinterpret_cast<TileShared<HD>*>(raw);
-    constexpr int F4 = HD / 4, C4 = HD / 64;
+    constexpr int F4 = HD / 4, C4 = HD / 64, KPP = 128 / HD;
     pdl_wait();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int req = tile_req[blockIdx.x], tok0 = tile_tok0[blockIdx.x];
@@ -281,22 +341,46 @@ attn_f32_tile_kernel(const float* q, const float* k_cache, const float* v_cache,
         if (t + 1 < n_tiles) fetch(t + 1);
         const int c0 = tile_start(t);
         const bool kept_run = t < kept_tiles;
+        // the eight sums of a score, as a tree of pairs
         float s[2][4];
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
-#pragma unroll 8
-        for (int f = 0; f < HD; f += 4) {
-            float4 a[2], b[4];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) a[i] = *reinterpret_cast<const float4*>(&sm.q[rs + 16 * i][f]);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(&sm.k[t & 1][ks + 8 * j][f]);
+        auto part = [&](int q, float (&d)[2][4]) {
 #pragma unroll
             for (int i = 0; i < 2; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) s[i][j] = dot4(a[i], b[j], s[i][j]);
+                for (int j = 0; j < 4; ++j) d[i][j] = 0.f;
+#pragma unroll
+            for (int f = 4 * q; f < HD; f += 32) {
+                float4 a[2], b[4];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) a[i] = *reinterpret_cast<const float4*>(&sm.q[rs + 16 * i][f]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(&sm.k[t & 1][ks + 8 * j][f]);
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) d[i][j] = dot4(a[i], b[j], d[i][j]);
+            }
+        };
+        auto add = [](float (&to)[2][4], const float (&d)[2][4]) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) to[i][j] += d[i][j];
+        };
+#pragma unroll
+        for (int q = 0; q < 8; q += 4) {
+            float d0[2][4], d1[2][4], d2[2][4];
+            part(q, d0); part(q + 1, d1);
+            add(d0, d1);
+            part(q + 2, d1); part(q + 3, d2);
+            add(d1, d2);
+            add(d0, d1);
+            if (q == 0) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) s[i][j] = d0[i][j];
+            } else add(s, d0);
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
@@ -312,31 +396,33 @@ attn_f32_tile_kernel(const float* q, const float* k_cache, const float* v_cache,
             top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
             top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 4));
             const float m_new = fmaxf(m_run[i], top);
-            const float alpha = m_run[i] == -INFINITY ? 0.f : expf(m_run[i] - m_new);
+            const float alpha = rescale(m_run[i], m_new);
             float sum = 0.f;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int p = c0 + ks + 8 * j;
-                const float e = p >= lo && p < hi ? expf(s[i][j] - m_new) : 0.f;
+                const bool seen = p >= lo && p < hi;
+                const float e = seen ? expf(s[i][j] - m_new) : 0.f;
                 sm.p[rs + 16 * i][ks + 8 * j] = e;
                 sum += e;
             }
             sum += __shfl_xor_sync(0xffffffffu, sum, 1);
             sum += __shfl_xor_sync(0xffffffffu, sum, 2);
             sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-            l_run[i] = l_run[i] * alpha + sum;
+            l_run[i] = fmaf(l_run[i], alpha, sum);
             m_run[i] = m_new;
             if (ks == 0) sm.alpha[rs + 16 * i] = alpha;
         }
         __syncthreads();                                  // weights and factors are there
         // every pair of the tile is seen where the last key is at or before the first row and the first key is in all rows' windows
         const bool whole = !kept_run && c0 + A32_KEYS - 1 <= pos0 && c0 >= first_key(mask, pos1);
+        float4 o[KPP][4][C4];                             // heads of 64: even and odd keys apart
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float f = sm.alpha[ro + 8 * i];
+        for (int e = 0; e < KPP; ++e)
 #pragma unroll
-            for (int j = 0; j < C4; ++j) { acc[i][j].x *= f; acc[i][j].y *= f; acc[i][j].z *= f; acc[i][j].w *= f; }
-        }
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < C4; ++j) o[e][i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 2
         for (int key = 0; key < A32_KEYS; key += 4) {
             float4 w[4];
@@ -350,12 +436,24 @@ attn_f32_tile_kernel(const float* q, const float* k_cache, const float* v_cache,
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const float e = x == 0 ? w[i].x : x == 1 ? w[i].y : x == 2 ? w[i].z : w[i].w;
+                        float4& to = o[x % KPP][i][j];
                         if (whole || e != 0.f) {
-                            acc[i][j].x = fmaf(e, v.x, acc[i][j].x); acc[i][j].y = fmaf(e, v.y, acc[i][j].y);
-                            acc[i][j].z = fmaf(e, v.z, acc[i][j].z); acc[i][j].w = fmaf(e, v.w, acc[i][j].w);
+                            to.x = fmaf(e, v.x, to.x); to.y = fmaf(e, v.y, to.y);
+                            to.z = fmaf(e, v.z, to.z); to.w = fmaf(e, v.w, to.w);
                         }
                     }
                 }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float f = sm.alpha[ro + 8 * i];
+#pragma unroll
+            for (int j = 0; j < C4; ++j) {
+                float4 v = o[0][i][j];
+                if (KPP == 2) { v.x += o[KPP - 1][i][j].x; v.y += o[KPP - 1][i][j].y; v.z += o[KPP - 1][i][j].z; v.w += o[KPP - 1][i][j].w; }
+                acc[i][j].x = fmaf(acc[i][j].x, f, v.x); acc[i][j].y = fmaf(acc[i][j].y, f, v.y);
+                acc[i][j].z = fmaf(acc[i][j].z, f, v.z); acc[i][j].w = fmaf(acc[i][j].w, f, v.w);
+            }
         }
     }
 #pragma unroll
@@ -390,12 +488,24 @@ RLLM_API int rllm_attn_f32_rows(const float* q, const float* k_cache, const floa
     if (n_tokens <= 0) return 0;
     if (!f32_shape_ok(H, K, hd, bs, keep_first, chunk)) return (int)cudaErrorInvalidValue;
     const F32Mask mask = {scale, softcap, window, keep_first, chunk};
-    const int g = H / K, G = g >= 3 ? 4 : g, chunks = (g + G - 1) / G;
+    // keys that a token can see, from the table's width; a warp per chunk of them up to 16 (the order does not depend on it)
+    long long span = (long long)table_stride * bs;
+    if (chunk > 0 && (long long)chunk + keep_first < span) span = (long long)chunk + keep_first;
+    if (window > 0 && (long long)window + keep_first < span) span = (long long)window + keep_first;
+    const int warps = span <= 4 * A32_KEYS ? 4 : span <= 8 * A32_KEYS ? 8 : A32_MAX_WARPS;
+    // Query heads per block: as few as still run all at once (16 warps of 128 registers fill an SM), so that a block's chain is
+    // short; up to four share the reads of their keys otherwise.  (One token of 32 heads on 8: with four heads a block 9.3 us
+    // for one key and 88 for 4,096, with one 4.1 and 46.)
+    const int g = H / K;
+    const long long slots = (long long)rllm_sm_count() * (A32_MAX_WARPS / warps);
+    int G = 1;
+    while (G < 4 && G < g && (long long)n_tokens * K * ((g + G - 1) / G) > slots) G *= 2;
+    const int chunks = (g + G - 1) / G;
 #define ROWS(HD, GG)                                                                                                            \
     if (hd == HD && G == GG)                                                                                                    \
-        return rllm_launch_after(attn_f32_rows_kernel<HD, GG>, dim3(n_tokens, K * chunks), dim3(A32_WARPS * 32), 0, stream, q, k_cache, \
-                           v_cache, out, positions, seq_ids, tokens, block_table, table_stride, H, K, chunks, bs, mask, n_pages, \
-                           err, sink, slopes);
+        return rllm_launch_after(attn_f32_rows_kernel<HD, GG>, dim3(n_tokens, K * chunks), dim3(warps * 32),                     \
+                                 rows_smem(HD, GG, warps), stream, q, k_cache, v_cache, out, positions, seq_ids, tokens,         \
+                                 block_table, table_stride, H, K, chunks, bs, mask, n_pages, err, sink, slopes);
     ROWS(64, 1) ROWS(64, 2) ROWS(64, 4) ROWS(128, 1) ROWS(128, 2) ROWS(128, 4)
 #undef ROWS
     return (int)cudaErrorInvalidValue;

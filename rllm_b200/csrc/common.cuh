@@ -106,6 +106,17 @@ static inline int rllm_pdl_enabled() {
     }
     return on;
 }
+// SMs of the device (the first one that asked; all devices of a run are alike)
+static inline int rllm_sm_count() {
+    static int n_sm = 0;
+    if (!n_sm) {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        n_sm = n > 0 ? n : 148;
+    }
+    return n_sm;
+}
 template <typename... KArgs, typename... Args>
 static inline int rllm_launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                               Args... args) {
