@@ -10,7 +10,8 @@
 //   the sum  of the weights exp(s - M): four keys 8 apart one after the other, then a tree of pairs over the eight;
 //   o        the weighted values: one chain over the keys for heads of 128, one each over even and odd keys for heads of 64;
 //   l = l * exp(M before - M) + sum,  acc = acc * exp(M before - M) + o   (one fused multiply-add each).
-// A key that a row does not see adds nothing to it, not even where its value is infinite: tiles with masked pairs test the weight.
+// A key that a row does not see adds nothing to it, not even where its value is infinite.  Scores of -inf weigh nothing beside
+// finite ones wherever those are.
 //
 // attn_f32_rows_kernel: bound by the latency of the key and value reads.  A block per (token, key/value head and up to 4 of its
 // query heads); its warps take one chunk each, eight lanes read one key's row in whole lines, and a round of chunks is
@@ -58,6 +59,8 @@ __device__ __forceinline__ float shape_score(const F32Mask& k, float dot, const 
 }
 // the factor of what was summed up to a largest score of `before` when it has become `now`
 __device__ __forceinline__ float rescale(float before, float now) { return before == -INFINITY ? 0.f : expf(before - now); }
+// the weight of score s (-inf only: nothing seen yet, every weight zero)
+__device__ __forceinline__ float weight(float s, float top) { return expf(s - (top == -INFINITY ? 0.f : top)); }
 __device__ __forceinline__ float dot4(float4 a, float4 b, float c) {
     return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, c))));
 }
@@ -189,7 +192,7 @@ attn_f32_rows_kernel(const float* q, const float* k_cache, const float* v_cache,
             m_run[j] = fmaxf(m_run[j], warp_max(v));
             if (live) {
                 const float now = fmaxf(before, s_top[warp * G + j]);
-                sc[j * A32_KEYS + lane] = seen ? expf(s[j] - now) : 0.f;
+                sc[j * A32_KEYS + lane] = seen ? weight(s[j], now) : 0.f;
                 if (lane == 0) s_factor[warp * G + j] = rescale(before, now);
             }
         }
@@ -263,7 +266,7 @@ struct TileShared {
     float q[A32_ROWS][HD + 4];
     float k[2][A32_KEYS][HD + 4];
     float v[2][A32_KEYS][HD + 4];
-    float p[A32_ROWS][A32_KEYS + 4];
+    float p[A32_ROWS][A32_KEYS + 4];               // weights; -1 where the row does not see the key
     float alpha[A32_ROWS];
     float l[A32_ROWS];
 };
@@ -402,8 +405,8 @@ attn_f32_tile_kernel(const float* q, const float* k_cache, const float* v_cache,
             for (int j = 0; j < 4; ++j) {
                 const int p = c0 + ks + 8 * j;
                 const bool seen = p >= lo && p < hi;
-                const float e = seen ? expf(s[i][j] - m_new) : 0.f;
-                sm.p[rs + 16 * i][ks + 8 * j] = e;
+                const float e = seen ? weight(s[i][j], m_new) : 0.f;
+                sm.p[rs + 16 * i][ks + 8 * j] = seen ? e : -1.f;
                 sum += e;
             }
             sum += __shfl_xor_sync(0xffffffffu, sum, 1);
@@ -437,7 +440,7 @@ attn_f32_tile_kernel(const float* q, const float* k_cache, const float* v_cache,
                     for (int i = 0; i < 4; ++i) {
                         const float e = x == 0 ? w[i].x : x == 1 ? w[i].y : x == 2 ? w[i].z : w[i].w;
                         float4& to = o[x % KPP][i][j];
-                        if (whole || e != 0.f) {
+                        if (whole || !(e < 0.f)) {
                             to.x = fmaf(e, v.x, to.x); to.y = fmaf(e, v.y, to.y);
                             to.z = fmaf(e, v.z, to.z); to.w = fmaf(e, v.w, to.w);
                         }

@@ -1,8 +1,9 @@
-"""float32 attention gives a token the same bits however its prompt is cut into portions."""
+"""float32 attention gives a token the same bits however its prompt is cut into portions, and treats infinite scores and values as
+the plain kernel does."""
 import pytest
 import torch
 
-from test_f32_path_gpu import DEV, Step, ops, rnd
+from test_f32_path_gpu import DEV, Step, attend64, ops, rnd
 
 pytestmark = pytest.mark.gpu
 
@@ -14,7 +15,7 @@ def paged(x, bs):
     return torch.cat([x, torch.zeros(n * bs - L, K, hd)]).view(n, bs, K, hd).transpose(1, 2).contiguous().to(DEV)
 
 
-def run(q, k, v, start, H, K, hd, bs, **mask):
+def run(q, k, v, start, H, K, hd, bs, fn="paged_attention", **mask):
     """Attention of the tokens start.. of one request whose queries are q."""
     n, L = q.shape[0], start + q.shape[0]
     step = Step([L], [n])
@@ -23,7 +24,10 @@ def run(q, k, v, start, H, K, hd, bs, **mask):
     args = (q.reshape(n, -1).to(DEV), paged(k, bs), paged(v, bs), out)
     m = (hd ** -0.5, mask.get("window", 0), mask.get("keep", 0), None, mask.get("chunk", 0), mask.get("cap", 0.0),
          mask.get("sink"), mask.get("slopes"))
-    ops().paged_attention(*args, step, table, H, K, hd, bs, *m)
+    if fn == "paged_attention":
+        ops().paged_attention(*args, step, table, H, K, hd, bs, *m)
+    else:
+        ops().paged_attention_generic(*args, step.positions, step.seq_ids, table, H, K, hd, bs, *m)
     ops().check_device_errors()
     return out
 
@@ -44,3 +48,35 @@ def test_cuts(hd, H, K, form):
         assert torch.equal(part, whole[at:at + size]), (form, at, size)
         at += size
     assert at == n
+
+
+@pytest.mark.parametrize("n", [1, 9, 40])
+def test_scores_of_minus_infinity(n):
+    """Some keys score -inf for every query (a query entry of one sign against a key entry of -inf): beside finite scores they
+    weigh nothing, wherever they lie; 32 of them in a row are one chunk of the kernels."""
+    H, K, hd, bs, L = 2, 1, 64, 16, 100
+    q, k, v = rnd(n, H, hd, seed=1), rnd(L, K, hd, seed=2), rnd(L, K, hd, seed=3)
+    q[..., 0] = q[..., 0].abs() + 0.5
+    k[0:64, :, 0] = float("-inf")
+    got = run(q, k, v, L - n, H, K, hd, bs)
+    plain = run(q, k, v, L - n, H, K, hd, bs, fn="generic")
+    rows = plain.isfinite().all(1)
+    assert bool(rows.any())
+    want = attend64(q, [k[64:]], [v[64:]], [(0, p - 64) for p in range(L - n, L)], hd ** -0.5, 0, 0, 0, 0.0, None, None) if n < 36 else None
+    assert bool(got[rows].isfinite().all())
+    assert float((got[rows] - plain[rows]).abs().max()) < 1e-5
+    if want is not None:
+        assert float((got.cpu().double() - want).abs().max()) < 1e-5
+
+
+@pytest.mark.parametrize("n", [1, 9, 40])
+def test_an_infinite_value_whose_weight_underflows(n):
+    """A key that is seen with a weight of exactly zero and an infinite value: not a number, as in the plain kernel."""
+    H, K, hd, bs, L = 2, 2, 128, 16, 64
+    q, k, v = rnd(n, H, hd, seed=1), rnd(L, K, hd, seed=2), rnd(L, K, hd, seed=3)
+    q[..., 0] = 40.0
+    k[:, :, 0] = 0.0
+    k[5, :, 0] = -1000.0
+    v[5] = float("inf")
+    got, plain = run(q, k, v, L - n, H, K, hd, bs), run(q, k, v, L - n, H, K, hd, bs, fn="generic")
+    assert torch.equal(got.isnan(), plain.isnan()) and bool(plain.isnan().any())
