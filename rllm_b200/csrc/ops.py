@@ -1905,16 +1905,20 @@ F32_TILE_ROWS = 32             # rows (tokens x query heads) of a tile of attent
 
 
 class F32AttentionPlan:
-    """Tokens and tiles of one float32 step for one group size (query heads per key/value head): requests of at most
-    DECODE_MAX_Q tokens go token by token, longer portions in tiles.  Built once per step, shared by its layers."""
+    """Tokens and tiles of one float32 step for one geometry: requests of at most DECODE_MAX_Q tokens go token by token,
+    longer portions in tiles or token by token, whichever `tiles_pay` estimates to end first (the two give equal bits).
+    Built once per step, shared by its layers.  span: an upper bound of the keys that a token of the step sees."""
 
-    def __init__(self, ctx, g, device):
+    def __init__(self, ctx, H, K, hd, span, device):
+        g = H // K
         self.GH = min(g, F32_TILE_ROWS)
         self.chunks = -(-g // self.GH)
         self.TT = F32_TILE_ROWS // self.GH
+        portions = [k for k in ctx.q_lens if k > DECODE_MAX_Q]
+        tiles = bool(portions) and self.tiles_pay(portions, g, K, hd, span, sm_count(device))
         toks, t_req, t_tok, at = [], [], [], 0
         for r, k in enumerate(ctx.q_lens):
-            if k <= DECODE_MAX_Q:
+            if k <= DECODE_MAX_Q or not tiles:
                 toks += range(at, at + k)
             else:
                 starts = range(at, at + k, self.TT)
@@ -1925,6 +1929,18 @@ class F32AttentionPlan:
         flat = torch.tensor(toks + t_req + t_tok + [0], dtype=torch.int32).to(device)
         a, b = self.n_rows, self.n_rows + self.n_tiles
         self.tokens, self.t_req, self.t_tok = flat[:a], flat[a:b], flat[b:b + self.n_tiles]
+
+    def tiles_pay(self, portions, g, K, hd, span, n_sm):
+        """A launch of tiles takes 4 us and 4.8 us per 32 keys for heads of 128 (2.7 for 64) with an SM to each block, a third
+        more beside another one, and two fit an SM; a block of the token kernel takes 7 us per round of its warps' chunks, one
+        block of 16 warps or four of 4 an SM.  (One portion of 64 tokens behind 4,096 keys, 16 heads on 8: 609 us in tiles,
+        227 token by token; one of 461 behind none: 89 us and 165.)"""
+        blocks = sum(-(-k // self.TT) for k in portions) * K * self.chunks
+        in_tiles = 4 + -(-span // 32) * (4.8 if hd > 64 else 2.7) * (1.35 if blocks > n_sm else 1.0) * max(1.0, blocks / (2 * n_sm))
+        warps = 4 if span <= 128 else 8 if span <= 256 else 16
+        waves = -(-sum(portions) * K * (-(-g // 4) if g > 2 else 1) * warps // (16 * n_sm))
+        rounds = -(-max(1, span - max(portions) // 2) // (32 * warps))
+        return in_tiles < waves * rounds * (7.0 if warps == 16 else 5.5)
 
 
 def paged_attention_f32(q, k_cache, v_cache, out, ctx, block_table, H, K, hd, block_size, scale, window=0, keep_first=0,
@@ -1938,10 +1954,13 @@ def paged_attention_f32(q, k_cache, v_cache, out, ctx, block_table, H, K, hd, bl
     assert block_table.dtype == torch.int32 and block_table.dim() == 2 and block_table.stride(1) == 1
     for w in (sink, slopes):
         assert w is None or (w.dtype == torch.float32 and w.numel() == H and w.is_contiguous())
-    key = ("float32", H // K)
+    span = block_table.shape[1] * block_size
+    if window or chunk:
+        span = min(span, min(window or span, chunk or span) + keep_first)
+    key = ("float32", H, K, hd, span)
     plan = ctx.plans.get(key)
     if plan is None:
-        plan = ctx.plans[key] = F32AttentionPlan(ctx, H // K, q.device)
+        plan = ctx.plans[key] = F32AttentionPlan(ctx, H, K, hd, span, q.device)
     tail = (c_int(window), c_int(keep_first), c_int(chunk), c_float(softcap), c_int(min(k_cache.shape[0], 0x7fffffff)),
             _ptr(error_word(q.device)), _ptr(sink), _ptr(slopes), _stream())
     if plan.n_tiles:
