@@ -40,8 +40,9 @@ def sample_rows(logits: torch.Tensor, params: Sequence[SamplingParams], counters
     dev = logits.device
     mask = (1 << 63) - 1
     temperature = torch.tensor([p.temperature for p in params], dtype=torch.float32).to(dev)
-    top_k = torch.tensor([p.top_k for p in params], dtype=torch.int32).to(dev)
-    top_p = torch.tensor([p.top_p for p in params], dtype=torch.float32).to(dev)
+    # None where no row asks for it: the launch then knows that it has fewer passes to make
+    top_k = torch.tensor([p.top_k for p in params], dtype=torch.int32).to(dev) if any(p.top_k > 0 for p in params) else None
+    top_p = torch.tensor([p.top_p for p in params], dtype=torch.float32).to(dev) if any(p.top_p < 1.0 for p in params) else None
     seed = torch.from_numpy(np.array([p.seed & ((1 << 64) - 1) for p in params], dtype=np.uint64).view(np.int64)).to(dev)
     counter = torch.tensor([c & mask for c in counters], dtype=torch.int64).to(dev)
     return ops.sample_rows(logits, out, temperature, top_k, top_p, seed, counter)
