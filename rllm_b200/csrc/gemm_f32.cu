@@ -10,11 +10,12 @@
 // in flight per warp.  NR grows with the rows of A because each 32 bytes of A that come out of L1 then serve NR
 // rows of W (22 bytes per clock and SM of W leave L1 room for about four times as many bytes of A).
 //
-// gemm_f32_kernel, more rows: bound by the FMA pipe (74 TFLOP/s).  cp.async tiles of 16 k values (two runs of one
-// class) in rows of 20 floats: eight rows' float4 then lie in eight different 16-byte bank groups, so no
+// gemm_f32_kernel, more rows: bound by the FMA pipe (74 TFLOP/s).  cp.async tiles of 16 k values (two runs, of one class
+// or of two neighbours) in rows of 20 floats: eight rows' float4 then lie in eight different 16-byte bank groups, so no
 // transposition is needed and every shared-memory read of a warp is one wavefront.  Per 4 k values a thread reads
-// TM + TN float4 for TM * TN * 4 multiply-adds.  128 x 64 tiles (8 x 8 a thread) where they fill the SMs, else 64 x 32
-// (4 x 4): a launch of fewer blocks than SMs is as slow as its one block.
+// TM + TN float4 for TM * TN * 4 multiply-adds.  128 x 64 tiles (8 x 8 a thread) where they fill the SMs, 64 x 64 (4 x 8) where
+// they do and there are no more rows than that, else 64 x 32 (4 x 4): a launch of fewer blocks than SMs is as slow as its
+// one block.
 //
 // Measured in place of one kernel for every shape (64 x 64 tiles, one chain over k, 16 shared-memory reads of 4 bytes per
 // 16 multiply-adds, a block per 64 columns also for a single row): float32 requests of 300 and 161 tokens at the 0.6B
@@ -141,19 +142,22 @@ gemm_f32_kernel(const float* A, const float* W, float* C, int m, int n, int k, i
     W += (size_t)blockIdx.z * sw;
     C += (size_t)blockIdx.z * sc;
 
-    const int per_class = ((k + F32_STEP - 1) / F32_STEP + 1) / 2;           // tiles of one class
-    const int classes = min(F32_CLASSES, (k + F32_RUN - 1) / F32_RUN);
-    const int tiles = per_class * classes;
+    const int per_class = (k + F32_STEP - 1) / F32_STEP;                      // runs of one class
+    const int runs = per_class * min(F32_CLASSES, (k + F32_RUN - 1) / F32_RUN);
+    const int tiles = (runs + 1) / 2;
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(&tile[0][0]);
 
+    constexpr int PARTS = VEC ? GEMM_BK / 4 : GEMM_BK;                        // copies per row of a tile
+    const int f = tid % PARTS * (GEMM_BK / PARTS);                            // a thread's place in its rows
     auto fetch = [&](int t) {
-        const int q = t / per_class, p = t - q * per_class;
+        // the tile's runs: number 2 t and the next one, of the same class or of the class behind it
+        const int q0 = 2 * t / per_class, p0 = 2 * t - q0 * per_class;
+        const bool turns = p0 + 1 == per_class;
+        const int e0 = p0 * F32_STEP + q0 * F32_RUN, e1 = 2 * t + 1 == runs ? k : turns ? (q0 + 1) * F32_RUN : e0 + F32_STEP;
         const uint32_t to = base + (t % GEMM_STAGES) * (ROWS * GEMM_LD * 4);
-        constexpr int PARTS = VEC ? GEMM_BK / 4 : GEMM_BK, WIDE = VEC ? 4 : 1;
-#pragma unroll 4
-        for (int x = tid; x < ROWS * PARTS; x += THREADS) {
-            const int r = x / PARTS, f = (x % PARTS) * WIDE;
-            const int e = (2 * p + f / F32_RUN) * F32_STEP + q * F32_RUN + f % F32_RUN;
+        const int e = (f < F32_RUN ? e0 : e1) + f % F32_RUN;
+#pragma unroll
+        for (int r = tid / PARTS; r < ROWS; r += THREADS / PARTS) {
             const bool is_a = r < BM;
             const int row = is_a ? m0 + r : n0 + r - BM;
             const bool in = row < (is_a ? m : n) && e < k;
@@ -201,16 +205,16 @@ gemm_f32_kernel(const float* A, const float* W, float* C, int m, int n, int k, i
 #pragma unroll
                 for (int i = 0; i < TM; ++i) acc[i][j] = fmaf(a[i].w, w.w, acc[i][j]);
             }
-        }
-        if (--left == 0) {                                 // the class ends
-            left = per_class;
+            if (f % F32_RUN != 0 && --left == 0) {         // a run ends, and the class with it
+                left = per_class;
 #pragma unroll
-            for (int i = 0; i < TM; ++i)
+                for (int i = 0; i < TM; ++i)
 #pragma unroll
-                for (int j = 0; j < TN; ++j) {
-                    total[i][j] += acc[i][j];
-                    acc[i][j] = 0.f;
-                }
+                    for (int j = 0; j < TN; ++j) {
+                        total[i][j] += acc[i][j];
+                        acc[i][j] = 0.f;
+                    }
+            }
         }
     }
 #pragma unroll
@@ -232,13 +236,17 @@ gemm_f32_kernel(const float* A, const float* W, float* C, int m, int n, int k, i
 // Rows up to which W is streamed by warps (in groups of 8 rows of A, each of which reads W again, from L2 where it fits):
 // 16 rows of 6,144 x 1,024 take 17 us this way, 24 rows take 53 us in tiles, which are mostly empty then.
 #define GEMV_ROWS 16
+// With less k most lanes of the streaming kernel have nothing to do: 16 rows of 8,192 x 16 take 5.7 us streamed, 2.5 in tiles.
+#define GEMV_MIN_K 32
+// Products of so little k are over before their blocks could be in the way: launched early, 16 rows of 8,192 x 16 2.85 -> 2.5 us.
+#define EARLY_MAX_K 64
 
 RLLM_API int rllm_gemm_f32_batched(const float* A, const float* W, float* C, int m, int n, int k, int lda, int ldw, int ldc,
                                    int accumulate, int batch, long long sa, long long sw, long long sc, cudaStream_t stream) {
     if (m <= 0 || n <= 0 || batch <= 0) return 0;
     if (k <= 0 || batch > 65535) return (int)cudaErrorInvalidValue;
     const bool vec = ((uintptr_t)A | (uintptr_t)W) % 16 == 0 && (k | lda | ldw) % 4 == 0 && (batch == 1 || (sa | sw) % 4 == 0);
-    const int n_sm = 148;
+    const int n_sm = rllm_sm_count();
 #define GEMV(M, NR, U)                                                                                                   \
     {                                                                                                                    \
         const int need = ((n + NR - 1) / NR + GEMV_WARPS - 1) / GEMV_WARPS, most = n_sm * (M >= 4 ? 2 : 3);               \
@@ -248,7 +256,7 @@ RLLM_API int rllm_gemm_f32_batched(const float* A, const float* W, float* C, int
                    : rllm_launch_after(gemv_f32_kernel<M, NR, U, false>, grid, dim3(GEMV_WARPS * 32), 0, stream, A, W, C, m, n, \
                                  k, lda, ldw, ldc, accumulate, sa, sw, sc);                                               \
     }
-    if (m <= GEMV_ROWS) {
+    if (m <= GEMV_ROWS && k > GEMV_MIN_K) {
         if (m == 1) GEMV(1, 1, 4)
         if (m == 2) GEMV(2, 1, 4)
         if (m <= 4) GEMV(4, 2, 2)
@@ -258,13 +266,16 @@ RLLM_API int rllm_gemm_f32_batched(const float* A, const float* W, float* C, int
 #define GEMM(TY, TX, TM, TN)                                                                                             \
     {                                                                                                                    \
         dim3 grid((n + TX * TN - 1) / (TX * TN), (m + TY * TM - 1) / (TY * TM), batch);                                   \
-        return vec ? rllm_launch_after(gemm_f32_kernel<TY, TX, TM, TN, true>, grid, dim3(TY * TX), 0, stream, A, W, C, m, n, k, \
-                                 lda, ldw, ldc, accumulate, sa, sw, sc)                                                   \
-                   : rllm_launch_after(gemm_f32_kernel<TY, TX, TM, TN, false>, grid, dim3(TY * TX), 0, stream, A, W, C, m, n,   \
-                                 k, lda, ldw, ldc, accumulate, sa, sw, sc);                                               \
+        auto kern = vec ? gemm_f32_kernel<TY, TX, TM, TN, true> : gemm_f32_kernel<TY, TX, TM, TN, false>;                 \
+        if (k <= EARLY_MAX_K)                                                                                            \
+            return rllm_launch(kern, grid, dim3(TY * TX), 0, stream, A, W, C, m, n, k, lda, ldw, ldc, accumulate, sa, sw, sc); \
+        return rllm_launch_after(kern, grid, dim3(TY * TX), 0, stream, A, W, C, m, n, k, lda, ldw, ldc, accumulate, sa, sw, sc); \
     }
     const long long large = (long long)((n + 63) / 64) * ((m + 127) / 128) * batch;
-    if (large >= n_sm) GEMM(16, 8, 8, 8)
+    if (large >= n_sm) {
+        if (m > 64) GEMM(16, 8, 8, 8)
+        GEMM(16, 8, 4, 8)
+    }
     GEMM(16, 8, 4, 4)
 #undef GEMM
 }
