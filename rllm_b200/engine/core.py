@@ -22,6 +22,7 @@ the same pre-checks before any mutation (86-100); graph replay keyed by the step
 from __future__ import annotations
 
 import contextlib
+import gc
 import math
 import os
 from typing import Optional, Sequence
@@ -368,12 +369,20 @@ class Engine:
         torch.cuda.synchronize()
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
-        with torch.cuda.stream(side):
-            graph.capture_begin(pool=self._graph_pool)
-            try:
-                yield
-            finally:
-                graph.capture_end()
+        # Not while the collector may run: a graph that an engine of the past left in a reference cycle must not be destroyed
+        # while a stream captures (the capture would fail).
+        collects = gc.isenabled()
+        gc.disable()
+        try:
+            with torch.cuda.stream(side):
+                graph.capture_begin(pool=self._graph_pool)
+                try:
+                    yield
+                finally:
+                    graph.capture_end()
+        finally:
+            if collects:
+                gc.enable()
         torch.cuda.current_stream().wait_stream(side)
 
     def _graph_step(self, items: Sequence[StepItem], device_tokens=None, portion: int = 0, n_dev: int = 0) -> Optional[torch.Tensor]:
