@@ -8,12 +8,20 @@ from test_f32_path_gpu import DEV, Step, attend64, ops, rnd
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("hd,H,K,bs", [(128, 16, 8, 32), (64, 6, 2, 16), (128, 40, 4, 8)])
+def blocks(o, step, H, K, window, keep, chunk):
+    """CTAs of the decode launch; with at most three per SM they have four warps."""
+    plan = o.AttentionPlan(step, H, K, window, torch.device(DEV), chunk)
+    assert plan.n_pre == 0
+    return plan.n_dec * K * plan.chunks_d * (plan.n_splits + (1 if keep else 0))
+
+
+@pytest.mark.parametrize("hd,H,K,bs,many", [(128, 16, 8, 32, 6), (64, 6, 2, 16, 18), (128, 40, 4, 8, 6)])
 @pytest.mark.parametrize("form", ["all", "window", "kept", "chunk", "extras"])
-@pytest.mark.parametrize("copies", [1, 6])
-def test_decode(hd, H, K, bs, form, copies):
-    """`copies` times the same requests: beyond 444 blocks the one-warp kernel runs.  Bound: weights and result are each
+@pytest.mark.parametrize("copied", [False, True])
+def test_decode(hd, H, K, bs, form, many, copied):
+    """`many` times the same requests: beyond three blocks an SM the one-warp kernel runs.  Bound: weights and result are each
     rounded to 9 bits, so 2^-8 of the largest value, and as much again for the exponentials and the sums."""
+    copies = many if copied else 1
     lens, q_lens = [1, 15, 16, 17, 33, 128, 129, 300, 515] * copies, [1, 1, 1, 1, 8, 1, 2, 1, 3] * copies
     window, keep, chunk, cap, sink, slopes = 0, 0, 0, 0.0, None, None
     if form in ("window", "kept"):
@@ -43,16 +51,18 @@ def test_decode(hd, H, K, bs, form, copies):
     dev = lambda x: None if x is None else x.to(DEV)                                     # noqa: E731
     out = torch.full((step.n_tokens, H * hd), float("nan"), dtype=torch.bfloat16, device=DEV)
     o = ops()
+    assert (blocks(o, step, H, K, window, keep, chunk) > 3 * o.sm_count(DEV)) or not copied
     o.paged_attention(q.view(-1, H * hd).to(DEV), kc.to(DEV), vc.to(DEV), out, step, table.to(DEV), H, K, hd, bs, hd ** -0.5,
                       window, keep, None, chunk, cap, dev(sink), dev(slopes))
     o.check_device_errors()
     top = max(float(v.abs().max()) for v in vs)
     assert float((out.cpu().double() - want).abs().max()) < 2.0 ** -7 * top
-    # a request alone (four warps a CTA) and in the batch: the same bits
+    # a request alone (four warps a CTA) and in the batch (copied: one warp): the same bits
     at = 0
     for r in range(9):
         one = Step([lens[r]], [q_lens[r]])
         one.start_pos = [lens[r] - q_lens[r]]
+        assert blocks(o, one, H, K, window, keep, chunk) <= 3 * o.sm_count(DEV)
         alone = torch.empty(q_lens[r], H * hd, dtype=torch.bfloat16, device=DEV)
         o.paged_attention(q[at:at + q_lens[r]].reshape(q_lens[r], -1).to(DEV), kc.to(DEV), vc.to(DEV), alone, one, table[r:r + 1].to(DEV), H,
                           K, hd, bs, hd ** -0.5, window, keep, None, chunk, cap, dev(sink), dev(slopes))
