@@ -552,8 +552,11 @@ RLLM_API int rllm_token_shift(const void* h, int act_dt, const float* mu, const 
 // which moves results by rounding only.
 #define WKV_PARTS 8
 // value columns a thread holds, and tokens per chunk (what a thread fetches ahead of a chunk lies in registers)
-__host__ __device__ constexpr int wkv_cols(int dmax) { return dmax <= 128 ? 4 : 2; }
-__host__ __device__ constexpr int wkv_tok(int dmax) { return dmax <= 128 ? 8 : 2; }
+// (heads of 32: with four columns a block has two warps only; 64 heads, 200 tokens, two columns and 16 tokens 64 us, four
+// and 8 97.  Heads of 64, 64 of them, 8 requests of 2, 5 and 7 tokens: 8.4, 9.2 and 9.3 us, a chunk of eight each time; with
+// two columns and a loop to the last token 10.6, 13.3 and 15.4.)
+__host__ __device__ constexpr int wkv_cols(int dmax) { return dmax <= 32 ? 2 : dmax <= 128 ? 4 : 2; }
+__host__ __device__ constexpr int wkv_tok(int dmax) { return dmax <= 32 ? 16 : dmax <= 128 ? 8 : 2; }
 // key channel of a thread's register ii: runs of four, so that the eight parts' 16-byte reads of a row lie side by side
 __device__ __forceinline__ int wkv_channel(int part, int ii) { return (ii / 4) * (4 * WKV_PARTS) + part * 4 + ii % 4; }
 __host__ __device__ constexpr int wkv_threads(int dmax) { return WKV_PARTS * dmax / wkv_cols(dmax); }
@@ -570,6 +573,7 @@ wkv_kernel(const float* rp, const float* kp, const float* vp, const float* wraw,
     constexpr int IPT = DMAX / WKV_PARTS;               // key channels per thread
     constexpr int COLS = wkv_cols(DMAX);                // neighbouring value channels per thread
     constexpr int NT = wkv_threads(DMAX);
+    constexpr bool STOPS = TOK > 8;
     constexpr int TD = TOK * DMAX;
     constexpr int PRE = (5 * TD + NT - 1) / NT;         // values a thread brings in per chunk
     extern __shared__ __align__(16) float sm_wkv[];      // r, k, w, v, gate: [5][TOK][DMAX]; o: [TOK][DMAX]; u: [DMAX]; bonus: [TOK]
@@ -649,7 +653,8 @@ wkv_kernel(const float* rp, const float* kp, const float* vp, const float* wraw,
         if (more) fetch(tb + TOK);
         // One token: only S carries over from the token before.  The loop is unrolled and a token's output stays in a
         // register until the chunk's end (a store to shared memory would hold back the next token's loads), so
-        // neighbouring tokens overlap.  Places behind the last token have zero keys and a decay of one.
+        // neighbouring tokens overlap.  Places behind the last token have zero keys and a decay of one, except where a chunk is
+        // long: that one stops at its tokens.
         float keep[TOK];
         int mycol = 0;                                     // the lane's column of the thread's COLS
         auto token = [&](int tt) {
@@ -701,8 +706,15 @@ wkv_kernel(const float* rp, const float* kp, const float* vp, const float* wraw,
             for (; m < WKV_PARTS; m <<= 1) o[0] += __shfl_xor_sync(0xffffffffu, o[0], m);
             keep[tt] = o[0];
         };
+        if (!STOPS || nt == TOK) {
 #pragma unroll
-        for (int tt = 0; tt < TOK; ++tt) token(tt);
+            for (int tt = 0; tt < TOK; ++tt) token(tt);
+        } else {
+#pragma unroll
+            for (int tt = 0; tt < TOK; ++tt)
+                if (tt < nt) token(tt);
+                else keep[tt] = 0.f;
+        }
         if (PASS != 1 && part < COLS) {
 #pragma unroll
             for (int tt = 0; tt < TOK; ++tt) s_o[tt * DMAX + j0 + mycol] =
