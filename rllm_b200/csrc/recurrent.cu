@@ -188,6 +188,39 @@ struct TimeSegments {
 #define SCAN_TOK 16           // tokens per chunk (1 where every request brings one token)
 #define SCAN_THREADS (SCAN_LANES * SCAN_CH)
 
+// A lane's states of a channel (places lane * NPT .. of the channel's N; zero beyond).  More than four: four at a time where
+// every channel's first one lies on 16 bytes; one at a time the lanes of a warp are NPT places apart, and 32 requests of 1,024 channels of
+// 64 states, one token each, took 21 us, now 9 (lanes that share a run of four places 16).
+__device__ __forceinline__ bool states_wide(const float* state, long long slot_stride, const float* A, const float* carry, int N) {
+    return N % 4 == 0 && slot_stride % 4 == 0 && (((uintptr_t)state | (uintptr_t)A | (uintptr_t)carry) & 15) == 0;
+}
+template <int NPT>
+__device__ __forceinline__ void load_states(float (&S)[NPT], const float* from, int lane, int N, bool wide) {
+    if (NPT > 4 && wide) {
+#pragma unroll
+        for (int k = 0; k < NPT; k += 4) {
+            const int n = lane * NPT + k;
+            const float4 v = n < N ? load4(from + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+            S[k] = v.x; S[k + 1] = v.y; S[k + 2] = v.z; S[k + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < NPT; ++k) S[k] = lane * NPT + k < N ? from[lane * NPT + k] : 0.f;
+    }
+}
+template <int NPT>
+__device__ __forceinline__ void store_states(float* to, const float (&S)[NPT], int lane, int N, bool wide) {
+    if (NPT > 4 && wide) {
+#pragma unroll
+        for (int k = 0; k < NPT; k += 4)
+            if (lane * NPT + k < N) store4(to + lane * NPT + k, make_float4(S[k], S[k + 1], S[k + 2], S[k + 3]));
+    } else {
+#pragma unroll
+        for (int k = 0; k < NPT; ++k)
+            if (lane * NPT + k < N) to[lane * NPT + k] = S[k];
+    }
+}
+
 template <typename TA, int NPT, int PASS, int TOK>
 __global__ void __launch_bounds__(SCAN_THREADS)
 selective_scan_kernel(const TA* x, const float* xz, long long ld_xz, const float* low, long long ld_low, int b_off,
@@ -222,13 +255,13 @@ selective_scan_kernel(const TA* x, const float* xz, long long ld_xz, const float
     const float* from = (first && last) ? st : seg.carry + (size_t)src * inner * N;
     float S[NPT], a[NPT];
     float sum_dt = 0.f;
+    const bool wide = NPT > 4 && states_wide(state, slot_stride, A, seg.carry, N);
+    if (PASS != 1) load_states<NPT>(S, from + (size_t)c * N, lane, N, wide);
+    else {
 #pragma unroll
-    for (int k = 0; k < NPT; ++k) {
-        const int n = lane * NPT + k;
-        const bool on = n < N;
-        S[k] = (on && PASS != 1) ? from[(size_t)c * N + n] : 0.f;
-        a[k] = on ? A[(size_t)c * N + n] : 0.f;
+        for (int k = 0; k < NPT; ++k) S[k] = 0.f;
     }
+    load_states<NPT>(a, A + (size_t)c * N, lane, N, wide);
     const float dd = Dp[c];
     float px[PRE_X], pbc[PRE_BC];
     // element e of the x/dt/z part: which (0 x, 1 dt, 2 z), token, channel of the block
@@ -317,21 +350,12 @@ selective_scan_kernel(const TA* x, const float* xz, long long ld_xz, const float
     }
     if (!live) return;
     if (PASS == 1) {
-        float* to = seg.carry + (size_t)item * inner * N;
-#pragma unroll
-        for (int k = 0; k < NPT; ++k) {
-            const int n = lane * NPT + k;
-            if (n < N) to[(size_t)c * N + n] = S[k];
-        }
+        store_states<NPT>(seg.carry + ((size_t)item * inner + c) * N, S, lane, N, wide);
         if (lane == 0) seg.decay[(size_t)item * inner + c] = sum_dt;
         return;
     }
     if (!last) return;
-#pragma unroll
-    for (int k = 0; k < NPT; ++k) {
-        const int n = lane * NPT + k;
-        if (n < N) st[(size_t)c * N + n] = S[k];
-    }
+    store_states<NPT>(st + (size_t)c * N, S, lane, N, wide);
     if (lane == 0 && taps > 1) {
         // kept inputs: the last taps-1 of (old kept inputs ++ this step's inputs), oldest first
         float* cs = st + conv_off + (size_t)c * (taps - 1);
