@@ -63,19 +63,24 @@ conv_silu4_kernel(const float* xz, long long ld, const float* __restrict__ w, co
         wt[i][0] = v.x; wt[i][1] = v.y; wt[i][2] = v.z; wt[i][3] = v.w;
         bias[i] = on && b ? b[c + i] : 0.f;
     }
+    // the step's indices were uploaded before its first kernel: the chain to the kept inputs starts ahead of the wait
+    const int ta = blockIdx.x * tok, tb = min(n, ta + tok);
+    int r = seq_ids[ta], first = cu_q[r], slot = slots[r];
+    bool begins = true;
     pdl_wait();
     pdl_launch_dependents();
     if (!on) return;
-    const int ta = blockIdx.x * tok, tb = min(n, ta + tok);
     float4 h3 = make_float4(0.f, 0.f, 0.f, 0.f), h2 = h3, h1 = h3;      // the inputs three, two and one token back
-    int r = -1;
     for (int t = ta; t < tb; ++t) {
         const float4 x = load4(xz + (size_t)t * ld + c);
-        const int rt = seq_ids[t];
-        if (rt != r) {                                     // a request begins, here or before this block's tokens
-            r = rt;
-            const int i = t - cu_q[r];
-            const float* st = state + (size_t)slots[r] * slot_stride + conv_off + (size_t)c * 3;
+        if (t > ta) {
+            const int rt = seq_ids[t];
+            begins = rt != r;
+            if (begins) { r = rt; first = cu_q[r]; slot = slots[r]; }
+        }
+        if (begins) {                                      // a request begins, here or before this block's tokens
+            const int i = t - first;
+            const float* st = state + (size_t)slot * slot_stride + conv_off + (size_t)c * 3;
             // the input `back` tokens before t: a row of this step, or place 3 - back + i of the kept inputs (oldest first)
             auto before = [&](int back) {
                 if (back <= i) return load4(xz + (size_t)(t - back) * ld + c);
