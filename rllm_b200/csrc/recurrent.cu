@@ -20,6 +20,7 @@
 //           four floats of which the first is the running maximum m.  Heads beyond the kernel's sizes: S
 //           [dk][dv + 1] row-major and the four floats.
 #include "common.cuh"
+#include <type_traits>
 #include "recurrent.cuh"
 
 // ------------------------------------------------------------------ causal convolution + silu
@@ -267,6 +268,9 @@ selective_scan_kernel(const TA* x, const float* xz, long long ld_xz, const float
         for (int k = 0; k < NPT; ++k) S[k] = 0.f;
     }
     load_states<NPT>(a, A + (size_t)c * N, lane, N, wide);
+    // This lane's states that there are.  The places behind them hold zeros, which an infinite input turns into NaN, so that a
+    // number of states that does not fill the lanes (N < NP) leaves them out of the sum.
+    const int mine = N - lane * NPT;
     const float dd = Dp[c];
     float px[PRE_X], pbc[PRE_BC];
     // element e of the x/dt/z part: which (0 x, 1 dt, 2 z), token, channel of the block
@@ -319,7 +323,7 @@ selective_scan_kernel(const TA* x, const float* xz, long long ld_xz, const float
         if (more) fetch(tb + TOK);
         // One token: only S carries over from the token before, so with the loop unrolled the
         // exponentials, loads and shuffles of neighbouring tokens overlap.
-        auto token = [&](int tt) {
+        auto token = [&](int tt, auto ragged) {
             const float xv = s_x[tt * SCAN_CH + cl];
             const float dt = s_dt[tt * SCAN_CH + cl];
             const float dx = dt * xv;
@@ -334,7 +338,7 @@ selective_scan_kernel(const TA* x, const float* xz, long long ld_xz, const float
 #pragma unroll
                 for (int x = 0; x < 4; ++x) {
                     S[k + x] = fmaf(expf(dt * a[k + x]), S[k + x], __fmul_rn(dx, bb[x]));      // written out: every instance rounds alike
-                    if (PASS != 1) part = fmaf(S[k + x], cc[x], part);
+                    if (PASS != 1 && (!decltype(ragged)::value || k + x < mine)) part = fmaf(S[k + x], cc[x], part);
                 }
             }
             if (PASS == 1) return;
@@ -343,11 +347,13 @@ selective_scan_kernel(const TA* x, const float* xz, long long ld_xz, const float
             if (lane == 0 && live)
                 out[(size_t)(tb + tt) * inner + c] = from_f<TA>(fmaf(dd, xv, part) * s_z[tt * SCAN_CH + cl]);
         };
-        if (nt == TOK) {
+        if (N < NP) {
+            for (int tt = 0; tt < nt; ++tt) token(tt, std::true_type());
+        } else if (nt == TOK) {
 #pragma unroll 4
-            for (int tt = 0; tt < TOK; ++tt) token(tt);
+            for (int tt = 0; tt < TOK; ++tt) token(tt, std::false_type());
         } else {
-            for (int tt = 0; tt < nt; ++tt) token(tt);
+            for (int tt = 0; tt < nt; ++tt) token(tt, std::false_type());
         }
         __syncthreads();                                 // everyone is done with this chunk
         if (more) stash();
