@@ -1,7 +1,7 @@
 // Paged causal attention, plain form: one block per (token, query head), float32
 // arithmetic, any head size up to 512 (keys: 2048), any page size, any
-// number of heads and groups, optional sliding window.  It is the float32 path of
-// the engine and the reference the tensor-core kernels are tested against.
+// number of heads and groups, optional sliding window.  It takes the heads that the other
+// kernels do not (float32 heads of 64 and 128: attention_f32.cu) and is the reference they are tested against.
 //
 // Token t of request r = seq_ids[t] at absolute position pos sees keys p with
 // max(0, pos+1-window) <= p <= pos (window 0: all keys) and, with keep_first > 0, also the

@@ -19,7 +19,7 @@
 //
 // Measured in place of one kernel for every shape (64 x 64 tiles, one chain over k, 16 shared-memory reads of 4 bytes per
 // 16 multiply-adds, a block per 64 columns also for a single row): float32 requests of 300 and 161 tokens at the 0.6B
-// sizes with 8 decode steps 259 -> 63 ms; the head of 151,936 x 1,024 for one row 94 us (6.6 TB/s), 4,096 columns of
+// sizes with 8 decode steps 258 -> 65.5 ms; the head of 151,936 x 1,024 for one row 94 us (6.6 TB/s), 4,096 columns of
 // 1,024 for 1,024 rows 30 TFLOP/s.
 //
 // Both are launched behind the kernel before, not early beside its end: they fill the SMs, and blocks that wait there keep

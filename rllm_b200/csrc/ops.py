@@ -1804,7 +1804,7 @@ def defers_norm(m: int, w_before, w_after, swiglu_after: bool = False, w_lead=No
 def linear(a, w, out=None, out_dtype=None, accumulate=False, stream=None, follow=None, then_norm=None):
     """out (+)= a . w^T, choosing the kernel by element type and shape.
 
-    float32 operands always take the plain CUDA-core product (the true 32-bit path).
+    float32 operands always take the CUDA-core products of gemm_f32.cu (the true 32-bit path).
     bfloat16 operands: up to 64 rows take the weight-streaming tensor-core kernel, more rows the
     library product; shapes neither can take (a row length that is not a multiple of 8
     elements) take the plain product with the same operand types."""
