@@ -409,20 +409,13 @@ __global__ void __launch_bounds__(NW * 32) paged_decode_attention_kernel(const F
     int lo = p.window > 0 ? max(0, pos_first + 1 - p.window) : 0;
     if (p.chunk > 0) lo = max(lo, pos_first - pos_first % p.chunk);      // the first token's run starts first
     lo = lo / BN * BN;
-    // The kept first keys that lie before the first window tile: [0, sink_end).  Without splits they are
-    // extra tiles ahead of the window's; with splits the last split is theirs (and may be empty).  Kept
-    // keys inside the window tiles are let through by the mask there.
+    // The kept first keys that lie before the first window tile: [0, sink_end).  The last split is theirs
+    // (and may be empty).  Kept keys inside the window tiles are let through by the mask there.
     const int keepv = p.window > 0 ? p.keep_first : 0;
     const int sink_end = min(keepv, lo);
-    const bool sink_split = p.split_keys > 0 && keepv > 0 && blockIdx.z == gridDim.z - 1;
-    int kb = lo, ke = pos_last + 1;
-    if (sink_split) {
-        kb = 0;
-        ke = sink_end;
-    } else if (p.split_keys > 0) {
-        kb = lo + blockIdx.z * p.split_keys;
-        ke = min(ke, kb + p.split_keys);
-    }
+    const bool sink_split = keepv > 0 && blockIdx.z == gridDim.z - 1;
+    const int kb = sink_split ? 0 : lo + blockIdx.z * p.split_keys;
+    const int ke = sink_split ? sink_end : min(pos_last + 1, kb + p.split_keys);
     const size_t part_base = (((size_t)tile * gridDim.y + blockIdx.y) * gridDim.z + blockIdx.z) * p.part_rows;
 
     // the two columns (query rows) of this lane's accumulators: 2t and 2t + 1
@@ -779,12 +772,13 @@ static int launch_flash(const FlashParams& p, int mode, int n_tiles, int n_split
         // (measured at batch 8 and 64, context 2,048: 32-key tiles x 2 stages 24.8 / 109 us,
         // 16 x 3: 21.0 / 104, 16 x 4: 25.6 / 112, 32 x 4: 30.8 / 166).
         constexpr int BN = 16;
-        if ((long long)grid.x * grid.y * grid.z <= 3 * 148) {
+        if ((long long)grid.x * grid.y * grid.z <= 3LL * rllm_sm_count()) {
             // Few CTAs: four warps each, 64 KB, three CTAs an SM.  The line is where they no longer all run at once; then
-            // nine one-warp CTAs an SM keep more in flight.  Whole decode steps, one warp against four (CTAs): 0.6B sizes, 1
-            // request of 128 tokens 890 -> 789 us (16); 8B sizes, 1 of 700 3,317 -> 3,246 (48).  Beyond the line, with a first
-            // form of the four warps that merged their own partial sums: 16 of 400 1,130 / 1,132 (512), 40 of 600 1,851 / 1,940
-            // (1,920), 8B sizes, 8 of 2,048 3,519 / 3,800 (1,088).
+            // nine one-warp CTAs an SM keep more in flight.  One warp / four, us a call with its merge (CTAs), 32 heads on 8 of
+            // 128: 9.7 / 7.7 (8), 10.4 / 7.8 (48), 11.0 / 8.5 (96), 11.2 / 9.9 (192), 12.3 / 11.1 (288), 13.7 / 11.1 (384),
+            // 13.5 / 12.3 (432); 8 heads on 2 of 64: 8.4 / 6.6 (2), 13.5 / 10.8 (96).  All sizes measured below the line: 0.74 to
+            // 0.97 of one warp's time.  Beyond it, with a first form of the four warps that merged their own partial sums, whole
+            // steps: 16 of 400 1,130 / 1,132 (512), 40 of 600 1,851 / 1,940 (1,920), 8 of 2,048 at the 8B sizes 3,519 / 3,800 (1,088).
             constexpr int NS = 2, NW = 4, smem = NW * NS * 2 * BN * HD * 2;
             auto kern = paged_decode_attention_kernel<HD, BN, NS, NW>;
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

@@ -109,7 +109,7 @@ conv_silu4_kernel(const float* xz, long long ld, const float* __restrict__ w, co
 // tokens per thread of the kernels that keep rows in registers: enough threads for the SMs, at most 16 tokens
 static int row4_tokens(int n, int columns) {
     const long long quads = (long long)n * ((columns + 3) / 4);
-    const long long t = quads / (148LL * 1024);
+    const long long t = quads / (1024LL * rllm_sm_count());
     return t < 1 ? 1 : t > 16 ? 16 : (int)t;
 }
 
@@ -443,7 +443,7 @@ static int launch_scan(int n_requests, cudaStream_t stream, const void* x, const
 // seg_* / carry / decay: the cut along time (TimeSegments; n_items 0: none).  carry needs n_items * inner * N
 // floats, decay n_items * inner.  one_token: every request brings exactly one token (a decode step).  A chunk is then one
 // token, so that nothing is done for the fifteen that are not there: the same sums, 8 requests of 8,192 channels of 16
-// states 20.8 -> 8.4 us.
+// states 20.8 -> 8.3 us.
 RLLM_API int rllm_selective_scan(const void* x, int act_dt, const float* xz, long long ld_xz, const float* low,
                                  long long ld_low, int b_off, int c_off, const float* dtr, const float* dt_b,
                                  const float* A, const float* Dp, float* state, long long slot_stride,
@@ -829,16 +829,8 @@ static int launch_wkv_pass(dim3 grid, cudaStream_t stream, const float* rp, cons
                            const float* u, const float* norm_w, float eps, float* state, long long slot_stride,
                            long long prev_off, const void* h, int width, const int* cu_q, const int* slots, void* out,
                            int H, int D, const TimeSegments& seg) {
-    const size_t smem = ((size_t)(6 * TOK + 1) * DMAX + TOK) * sizeof(float);
-    if (smem > 48 * 1024) {
-        static bool raised = false;                      // once per instantiation: more dynamic shared memory than the default
-        if (!raised) {
-            cudaError_t e = cudaFuncSetAttribute(wkv_kernel<TA, DMAX, PASS, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem);
-            if (e != cudaSuccess) return (int)e;
-            raised = true;
-        }
-    }
+    constexpr size_t smem = ((size_t)(6 * TOK + 1) * DMAX + TOK) * sizeof(float);
+    static_assert(smem <= 48 * 1024, "more shared memory than a launch gets without asking");
     return rllm_launch(wkv_kernel<TA, DMAX, PASS, TOK>, grid, dim3(wkv_threads(DMAX)), smem, stream, rp, kp, vp, wraw,
                        gp, ld, w0, u, norm_w, eps, state, slot_stride, prev_off, (const TA*)h, width, cu_q, slots, (TA*)out,
                        H, D, seg);
@@ -867,7 +859,7 @@ static int launch_wkv(int n_requests, cudaStream_t stream, const float* rp, cons
 
 // seg_* / carry / decay: the cut along time (TimeSegments; n_items 0: none).  carry needs n_items * H * DMAX * DMAX
 // floats, decay n_items * H * DMAX (DMAX as in rllm_wkv_state_floats).  one_token: every request brings exactly one
-// token (a decode step): chunks of one token, the same sums; 8 requests of 64 heads of 64 22.8 -> 7.2 us.
+// token (a decode step): chunks of one token, the same sums; 8 requests of 64 heads of 64 22.8 -> 7.0 us.
 RLLM_API int rllm_wkv(const float* rp, const float* kp, const float* vp, const float* wraw, const float* gp,
                       long long ld, const float* w0, const float* u, const float* norm_w, float eps, float* state,
                       long long slot_stride, long long prev_off, const void* h, int act_dt, int width,
