@@ -39,16 +39,32 @@ __device__ __forceinline__ float warp_max(float v) {
 // Block-wide sum in a fixed order (butterfly inside a warp, then warps in index
 // order), so the result does not depend on scheduling.  `red` holds >= 33 floats.
 // All threads of the block must call it; every thread gets the total.
+// The warps' sums are read side by side and then added: up to eight by every thread (no second round through shared memory),
+// more by the first warp, a sum a lane.  (One thread that reads and adds them in turn: 0.5 us for 32 warps.)
 __device__ __forceinline__ float block_sum(float v, float* red) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
     v = warp_sum(v);
     __syncthreads();
     if (lane == 0) red[warp] = v;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.f;
-        for (int i = 0; i < nw; ++i) t += red[i];
-        red[32] = t;
+    float t = 0.f;
+    if (nw <= 8) {
+        float s[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s[i] = i < nw ? red[i] : 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (i < nw) t += s[i];
+        return t;
+    }
+    if (warp == 0) {
+        const float mine = lane < nw ? red[lane] : 0.f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            const float s = __shfl_sync(0xffffffffu, mine, i);
+            if (i < nw) t += s;
+        }
+        if (lane == 0) red[32] = t;
     }
     __syncthreads();
     return red[32];

@@ -318,8 +318,9 @@ qkv_rownorm_store_kernel(const TI* qkv, const float* __restrict__ bias, const fl
 
 // The same without a rotation, on float32 rows that can be read four entries at a time: the q and k columns stay in
 // registers (NV float4 a thread) between the sums and the stores, both sums are taken in one exchange.  Bound by its bytes;
-// 2,048 rows of 4,096 + 1,024 + 1,024: 51 us through shared memory an entry at a time, now 32 us; 8 rows 9.9 -> 5.9 us.
-template <typename TO, int NV>
+// 2,048 rows of 4,096 + 1,024 + 1,024: 51 us through shared memory an entry at a time, now 32 us; 8 rows 9.9 -> 5.9 us, with
+// the weights and values on their way early (EARLY) 4.1 -> 2.7 us between kernels of its own kind.
+template <typename TO, int NV, bool EARLY>
 __global__ void __launch_bounds__(1024)
 qkv_rownorm_store4_kernel(const float* qkv, const float* __restrict__ bias, const float* __restrict__ q_norm_w,
                           const float* __restrict__ k_norm_w, const int* __restrict__ slots, TO* q_out, TO* k_cache, TO* v_cache,
@@ -327,21 +328,48 @@ qkv_rownorm_store4_kernel(const float* qkv, const float* __restrict__ bias, cons
                           int n_slots, int* err, int v_off) {
     __shared__ float red[2][32];
     pdl_launch_dependents();
-    pdl_wait();
     const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    // EARLY: few tokens wait for memory, not for bandwidth: biases and norm weights, which do not depend on the kernels before,
+    // are here when the rows are, and the first value columns when they are stored.  With many tokens the registers that
+    // takes cost more (2,048 rows of 1,024 + 256 + 256: 8.7 -> 9.8 us).
+    float4 wgt[EARLY ? NV : 1], off4[EARLY ? NV : 1];
+    auto norm_weight = [&](int c) {
+        const float* w = c < wq ? q_norm_w : k_norm_w;
+        return w ? ld4(w + (c < wq ? c : c - wq)) : make_float4(1.f, 1.f, 1.f, 1.f);
+    };
+    if (EARLY) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int c = 4 * (tid + i * blockDim.x);
+            wgt[EARLY ? i : 0] = c < wq + wk ? norm_weight(c) : make_float4(1.f, 1.f, 1.f, 1.f);
+            off4[EARLY ? i : 0] = bias && c < wq + wk ? ld4(bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    pdl_wait();
     const float* row = qkv + (size_t)t * ld;
     auto biased = [&](int c) {
         float4 v = ld4(row + c);
         if (bias) { v.x += bias[c]; v.y += bias[c + 1]; v.z += bias[c + 2]; v.w += bias[c + 3]; }
         return v;
     };
+    int slot = write_kv ? slots[t] : -1;
     float4 val[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int c = 4 * (tid + i * blockDim.x);
+        if (c < wq + wk) val[i] = ld4(row + c);
+    }
+    float4 first_v = make_float4(0.f, 0.f, 0.f, 0.f);           // a thread's first four value columns, on their way meanwhile
+    if (EARLY && 4 * tid < wv) first_v = biased(v_off + 4 * tid);
     float sq = 0.f, sk = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         const int c = 4 * (tid + i * blockDim.x);
         if (c >= wq + wk) continue;
-        val[i] = biased(c);
+        if (bias) {
+            const float4 b = EARLY ? off4[EARLY ? i : 0] : ld4(bias + c);
+            val[i].x += b.x; val[i].y += b.y; val[i].z += b.z; val[i].w += b.w;
+        }
         const float s = val[i].x * val[i].x + val[i].y * val[i].y + val[i].z * val[i].z + val[i].w * val[i].w;
         if (c < wq) sq += s; else sk += s;
     }
@@ -353,7 +381,6 @@ qkv_rownorm_store4_kernel(const float* qkv, const float* __restrict__ bias, cons
     sq = warp_sum(in ? red[0][lane] : 0.f);
     sk = warp_sum(in ? red[1][lane] : 0.f);
     const float rq = 1.0f / sqrtf(sq / (float)wq + eps), rk = 1.0f / sqrtf(sk / (float)wk + eps);
-    int slot = write_kv ? slots[t] : -1;
     if (slot >= n_slots) {
         if (tid == 0 && err) atomicExch(err, RLLM_ERR_SLOT);
         slot = -1;
@@ -364,19 +391,19 @@ qkv_rownorm_store4_kernel(const float* qkv, const float* __restrict__ bias, cons
         int c = 4 * (tid + i * blockDim.x);
         if (c >= wq + wk) continue;
         const bool is_q = c < wq;
-        if (!is_q) c -= wq;
-        const float* w = is_q ? q_norm_w : k_norm_w;
         float4 v = val[i];
-        if (w) {
+        if (is_q ? q_norm_w != nullptr : k_norm_w != nullptr) {
             const float r = is_q ? rq : rk;
-            v = make_float4(v.x * r * w[c], v.y * r * w[c + 1], v.z * r * w[c + 2], v.w * r * w[c + 3]);
+            const float4 w = EARLY ? wgt[EARLY ? i : 0] : norm_weight(c);
+            v = make_float4(v.x * r * w.x, v.y * r * w.y, v.z * r * w.z, v.w * r * w.w);
         }
+        if (!is_q) c -= wq;
         if (is_q) st4(q_out + (size_t)t * wq + c, v);
         else if (slot >= 0) st4(k_cache + ((page * G + c / dk) * bs + off) * dk + c % dk, v);
     }
     if (slot < 0) return;
     for (int c = 4 * tid; c < wv; c += 4 * blockDim.x)
-        st4(v_cache + ((page * G + c / dv) * bs + off) * dv + c % dv, biased(v_off + c));
+        st4(v_cache + ((page * G + c / dv) * bs + off) * dv + c % dv, EARLY && c == 4 * tid ? first_v : biased(v_off + c));
 }
 
 RLLM_API int rllm_qkv_rownorm_store(const void* qkv, int in_dt, long long ld, const float* bias, const float* q_norm_w,
@@ -394,17 +421,19 @@ RLLM_API int rllm_qkv_rownorm_store(const void* qkv, int in_dt, long long ld, co
     const int threads = n < 128 ? 1024 : 256;
     const int qk = (H + G) * dk, nv = (qk / 4 + threads - 1) / threads;
     if (in_dt == RLLM_F32 && !rot && nv <= 8 && ld % 4 == 0 && dk % 4 == 0 && dv % 4 == 0 && v_off % 4 == 0 && al16(qkv) &&
-        al16(q_out) && al16(k_cache) && al16(v_cache)) {
-#define LAUNCH4(TO, NV)                                                                                                        \
-    return rllm_launch(qkv_rownorm_store4_kernel<TO, NV>, dim3(n), dim3(threads), 0, stream, (const float*)qkv, bias, q_norm_w, \
+        al16(q_out) && al16(k_cache) && al16(v_cache) && al16(bias) && al16(q_norm_w) && al16(k_norm_w)) {
+#define LAUNCH4(TO, NV, EARLY)                                                                                                        \
+    return rllm_launch(qkv_rownorm_store4_kernel<TO, NV, EARLY>, dim3(n), dim3(threads), 0, stream, (const float*)qkv, bias, q_norm_w, \
                        k_norm_w, slots, (TO*)q_out, (TO*)k_cache, (TO*)v_cache, ld, H * dk, G * dk, G * dv, G, dk, dv, bs, eps, \
                        write_kv, ns, err, v_off)
         if (out_dt == RLLM_F32) {
-            if (nv <= 2) { LAUNCH4(float, 2); }
-            LAUNCH4(float, 8);
+            if (nv <= 2 && n < 128) { LAUNCH4(float, 2, true); }
+            if (nv <= 2) { LAUNCH4(float, 2, false); }
+            LAUNCH4(float, 8, false);
         }
-        if (nv <= 2) { LAUNCH4(bf16, 2); }
-        LAUNCH4(bf16, 8);
+        if (nv <= 2 && n < 128) { LAUNCH4(bf16, 2, true); }
+        if (nv <= 2) { LAUNCH4(bf16, 2, false); }
+        LAUNCH4(bf16, 8, false);
 #undef LAUNCH4
     }
     const size_t smem = (size_t)(H + G) * dk * sizeof(float);

@@ -1,0 +1,68 @@
+"""The norms of whole rows that keep a row in registers: every number of columns a thread holds, the longest rows, delta and rows
+of either alignment, rows of which several groups of warps add their sums."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def ops():
+    from rllm_b200.csrc import ops as o
+    return o
+
+
+def rnd(*shape, seed):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed))
+
+
+def close(got, want, bits):
+    """A few roundings of float32 on the way, the sum of squares in any order (its relative error is halved by the root), and
+    one rounding to `bits` bits at the end."""
+    bound = (want.abs() * (2.0 ** -bits + 24 * 2.0 ** -24) + 1e-30)
+    assert bool(((got.cpu().double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("n", [1, 130])
+@pytest.mark.parametrize("d", [4, 8, 32, 252, 1024, 1028, 2048, 4092, 4096, 4100, 8192, 8196, 12288])
+@pytest.mark.parametrize("low", [torch.float32, torch.bfloat16])
+def test_norm_rows(n, d, low):
+    a, x, w = rnd(n, d, seed=1), rnd(n, d, seed=2), rnd(d, seed=3)
+    unit = a.double() / torch.sqrt((a.double() ** 2).mean(1, keepdim=True) + 1e-6) * w.double()
+    xs, out = x.to(DEV), torch.full((n, d + 4), float("nan"), dtype=low, device=DEV)
+    ops().norm_rows(a.to(DEV), w.to(DEV), 1e-6, x=xs, add=True, low=out[:, :d])
+    total = x.double() + unit
+    assert bool(((xs.cpu().double() - total).abs() <= (x.double().abs() + unit.abs()) * 24 * 2.0 ** -24 + 1e-30).all())
+    close(out[:, :d], xs.cpu().double(), 8 if low is torch.bfloat16 else 24)
+    assert bool(out[:, d:].isnan().all())
+    alone = torch.empty(n, d, dtype=low, device=DEV)
+    ops().norm_rows(a.to(DEV), None, 1e-6, low=alone)
+    close(alone, a.double() / torch.sqrt((a.double() ** 2).mean(1, keepdim=True) + 1e-6), 8 if low is torch.bfloat16 else 24)
+    own = a.to(DEV)
+    ops().norm_rows(own, w.to(DEV), 1e-6, x=own)                      # the rows are the stream itself
+    close(own, unit, 24)
+
+
+@pytest.mark.parametrize("n", [1, 9, 130])
+@pytest.mark.parametrize("d", [4, 1024, 1028, 2052, 4096, 4100, 8192, 8196])
+@pytest.mark.parametrize("dt,shift", [(torch.float32, 0), (torch.float32, 1), (torch.bfloat16, 0), (torch.bfloat16, 1)])
+def test_add_rms_norm(n, d, dt, shift):
+    """shift: the sublayer's output starts one entry behind an aligned address."""
+    x, delta, w = rnd(n, d, seed=4), rnd(n, d, seed=5).to(dt), rnd(d, seed=6)
+    base = torch.zeros(n * d + 1, dtype=dt, device=DEV)
+    moved = base[shift:shift + n * d].view(n, d)
+    moved.copy_(delta)
+    total = x.double() + 0.5 * delta.double()
+    unit = total / torch.sqrt((total ** 2).mean(1, keepdim=True) + 1e-5) * w.double()
+    for out_dt, bits in ((torch.float32, 24), (torch.bfloat16, 8)):
+        xs, out = x.to(DEV), torch.empty(n, d, dtype=out_dt, device=DEV)
+        ops().add_rms_norm(xs, moved, w.to(DEV), out, 1e-5, delta_scale=0.5)
+        size = x.double().abs() + 0.5 * delta.double().abs()
+        assert bool(((xs.cpu().double() - total).abs() <= size * 2.0 ** -23 + 1e-30).all())
+        exact = xs.cpu().double()
+        close(out, exact / torch.sqrt((exact ** 2).mean(1, keepdim=True) + 1e-5) * w.double(), bits)
+    rows = torch.tensor([n - 1, 0], dtype=torch.int32, device=DEV)
+    kept, out = x.to(DEV), torch.empty(2, d, device=DEV)
+    ops().add_rms_norm(kept, moved, w.to(DEV), out, 1e-5, rows=rows, write_x=False, delta_scale=0.5)
+    assert torch.equal(kept.cpu(), x)
+    assert bool(((out.cpu().double() - unit[[n - 1, 0]]).abs() <= (unit[[n - 1, 0]].abs() + 1) * 1e-5).all())
