@@ -1,7 +1,8 @@
 // Blackwell tensor-core product for many rows: D[M,N] = A[M,K] . B[N,K]^T, bfloat16 operands,
 // float32 accumulation in tensor memory (TMEM), operands staged in shared memory by TMA.
 //
-//   * persistent CTAs (one per SM) walk over 128 x 256 output tiles; K is walked in blocks of 64
+//   * persistent CTAs (one per SM) walk over 128 x 256 output tiles (the gated product of few tiles or little K: 128 x 128 or
+//     128 x 64, two CTAs an SM: ops._gated_tile has the rule and both sides' times); K is walked in blocks of 64
 //     elements through a ring of shared-memory stages, each holding a [128 x 64] A tile and a
 //     [256 x 64] B tile in the 128-byte-swizzled K-major layout that both TMA writes and
 //     tcgen05.mma reads; two accumulators in TMEM let one tile's epilogue overlap the next tile's MMAs;
@@ -66,7 +67,7 @@ template <> __device__ __forceinline__ void store_row32<bf16>(bf16* dst, const f
 // buffers in TMEM (2 x BN columns): the epilogue of one tile overlaps the MMAs of the next, and the
 // operand ring never drains between tiles.
 template <int BN, int EPI, typename TC, int STAGES>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+__global__ void __launch_bounds__(TC_THREADS, BN < 256 ? 2 : 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, TC* __restrict__ C,
                int ldc, int M, int N, int K, int up_row_offset, int* __restrict__ err, const GluForm glu) {
     constexpr int A_BYTES = TC_BM * TC_BK * 2;
@@ -104,12 +105,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_slot;
-    pdl_wait();                                    // the A operand is written by the kernel before
 
     if (warp == 0 && lane == 0) {
-        // ---- TMA producer: one continuous ring over all of this CTA's tiles
+        // ---- TMA producer: one continuous ring over all of this CTA's tiles.  The weights of the first tile's first stages do
+        // not depend on the kernel before; the A operand does.
         int it = 0, issued = 0;
         bool ok = true;
+        const int head = blockIdx.x < total_tiles ? min(STAGES, nkb) : 0;
+        {
+            const int n0 = ((int)blockIdx.x / m_tiles) * BN_OUT;
+            for (int s = 0; s < head; ++s) {
+                unsigned char* b_s = smem + (size_t)s * STAGE_BYTES + A_BYTES;
+                mbar_expect_tx(&full_bar[s], STAGE_BYTES);
+                tma_load_2d(b_s, &tmB, s * TC_BK, n0, &full_bar[s]);
+                if (EPI == TC_EPI_SWIGLU) tma_load_2d(b_s + B_BYTES / 2, &tmB, s * TC_BK, up_row_offset + n0, &full_bar[s]);
+            }
+        }
+        pdl_wait();
         for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
             const int m0 = (tile % m_tiles) * TC_BM, n0 = (tile / m_tiles) * BN_OUT;
             for (int kb = 0; kb < nkb; ++kb, ++it) {
@@ -122,13 +134,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
                 unsigned char* a_s = smem + (size_t)s * STAGE_BYTES;
                 unsigned char* b_s = a_s + A_BYTES;
-                mbar_expect_tx(&full_bar[s], STAGE_BYTES);
+                if (it >= head) mbar_expect_tx(&full_bar[s], STAGE_BYTES);
                 tma_load_2d(a_s, &tmA, kb * TC_BK, m0, &full_bar[s]);
-                if (EPI == TC_EPI_SWIGLU) {
+                if (it >= head) {
                     tma_load_2d(b_s, &tmB, kb * TC_BK, n0, &full_bar[s]);
-                    tma_load_2d(b_s + B_BYTES / 2, &tmB, kb * TC_BK, up_row_offset + n0, &full_bar[s]);
-                } else {
-                    tma_load_2d(b_s, &tmB, kb * TC_BK, n0, &full_bar[s]);
+                    if (EPI == TC_EPI_SWIGLU) tma_load_2d(b_s + B_BYTES / 2, &tmB, kb * TC_BK, up_row_offset + n0, &full_bar[s]);
                 }
                 issued = it + 1;
             }
@@ -173,6 +183,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
     } else if (warp >= 2) {
         // ---- epilogue: warp w may touch TMEM lanes 32 * (w % 4) .. + 31
+        pdl_wait();                                // C belongs to the kernels before until here
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;
         int local = 0;
@@ -188,6 +199,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             tc_fence_after();
             if (first && tile + (int)gridDim.x >= total_tiles) { pdl_launch_dependents(); first = false; }
             const uint32_t taddr = tmem_base + buf * BN + ((uint32_t)(quarter * 32) << 16);
+            if (m0 + quarter * 32 >= M) {                    // none of the warp's rows exists
+                tc_fence_before();
+                mbar_arrive(&acc_empty[buf]);
+                continue;
+            }
 #pragma unroll 1
             for (int c0 = 0; c0 < BN_OUT; c0 += 32) {
                 uint32_t r[32];
@@ -199,7 +215,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     tmem_ld_wait();
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
-                        const float g = __uint_as_float(r[j]);
+                        // a row behind the last one: its gate is 0, and dividing 0 takes the division's slow path
+                        const float g = gm < M ? __uint_as_float(r[j]) : 1.f;
                         v[j] = glu_apply(glu, g, __uint_as_float(u[j]));
                     }
                 } else {
@@ -255,6 +272,8 @@ static int make_tmap(CUtensorMap* map, const void* base, int rows, int cols, int
     return r == CUDA_SUCCESS ? 0 : 30000 + (int)r;
 }
 
+// BN 256: one CTA an SM.  BN 128 and 64: two, one's epilogue beside the other's MMAs, each with half the shared memory for its
+// ring, or, where there are no more tiles than SMs, one with all of it.
 template <int BN, int EPI, typename TC, int STAGES>
 static int launch_tc(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int ldc, int M, int N, int K, int up,
                      int* err, cudaStream_t stream, const GluForm glu = GluForm{0.f, 1.f, 0.f}) {
@@ -275,7 +294,8 @@ static int launch_tc(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int 
         if (n_sm <= 0) n_sm = 148;
     }
     const int tiles = ((M + TC_BM - 1) / TC_BM) * ((N + BN_OUT - 1) / BN_OUT);
-    dim3 grid(tiles < n_sm ? tiles : n_sm);
+    const int most = smem > 110 * 1024 ? n_sm : 2 * n_sm;
+    dim3 grid(tiles < most ? tiles : most);
     return rllm_launch(kern, grid, dim3(TC_THREADS), smem, stream, ta, tb, (TC*)C, ldc, M, N, K, up, err, glu);
 }
 
@@ -285,20 +305,21 @@ static int launch_tc(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int 
 // K a multiple of 8.  `err` is a device int that receives a code if a bounded wait ran out.
 // Returns 0, a cudaError_t, 30000 + CUresult of the tensor-map encoder, or cudaErrorInvalidValue.
 // glu_*: the constants of the gated epilogue (GluForm in common.cuh); rllm_gemm_tc is SwiGLU's {0, 1, 0}.
-RLLM_API int rllm_gemm_tc_glu(const void* A, const void* B, void* C, int c_dtype, int M, int N, int K, int lda, int ldb,
-                              int ldc, int epilogue, int up_row_offset, float glu_limit, float glu_alpha,
-                              float glu_shift, int* err, cudaStream_t stream) {
+// bn: rows of B per tile, 256, or with the gated epilogue (half of them gate and half up) also 128 or 64.
+RLLM_API int rllm_gemm_tc_tile(const void* A, const void* B, void* C, int c_dtype, int M, int N, int K, int lda, int ldb,
+                               int ldc, int epilogue, int up_row_offset, float glu_limit, float glu_alpha,
+                               float glu_shift, int bn, int* err, cudaStream_t stream) {
     const GluForm glu = GluForm{glu_limit, glu_alpha, glu_shift};
     if (M <= 0 || N <= 0) return 0;
-    if (K <= 0 || (K & 7) || (lda & 7) || (ldb & 7) || ((uintptr_t)A & 15) || ((uintptr_t)B & 15) || !err)
+    if (K <= 0 || (K & 7) || (lda & 7) || (ldb & 7) || ((uintptr_t)A & 15) || ((uintptr_t)B & 15) || !err ||
+        (bn != 256 && (epilogue != TC_EPI_SWIGLU || (bn != 128 && bn != 64))))
         return (int)cudaErrorInvalidValue;
     if (epilogue == TC_EPI_ACCUM && c_dtype != RLLM_F32) return (int)cudaErrorInvalidValue;
     CUtensorMap ta, tb;
     int st = make_tmap(&ta, A, M, K, lda, TC_BM);
     if (st) return st;
     const int b_rows = epilogue == TC_EPI_SWIGLU ? up_row_offset + N : N;
-    const int b_box = epilogue == TC_EPI_SWIGLU ? 128 : 256;
-    st = make_tmap(&tb, B, b_rows, K, ldb, b_box);
+    st = make_tmap(&tb, B, b_rows, K, ldb, epilogue == TC_EPI_SWIGLU ? bn / 2 : bn);
     if (st) return st;
     if (epilogue == TC_EPI_STORE) {
         return c_dtype == RLLM_F32 ? launch_tc<256, TC_EPI_STORE, float, 4>(ta, tb, C, ldc, M, N, K, 0, err, stream)
@@ -306,11 +327,29 @@ RLLM_API int rllm_gemm_tc_glu(const void* A, const void* B, void* C, int c_dtype
     } else if (epilogue == TC_EPI_ACCUM) {
         return launch_tc<256, TC_EPI_ACCUM, float, 4>(ta, tb, C, ldc, M, N, K, 0, err, stream);
     } else if (epilogue == TC_EPI_SWIGLU) {
-        return c_dtype == RLLM_F32
-                   ? launch_tc<256, TC_EPI_SWIGLU, float, 4>(ta, tb, C, ldc, M, N, K, up_row_offset, err, stream, glu)
-                   : launch_tc<256, TC_EPI_SWIGLU, bf16, 4>(ta, tb, C, ldc, M, N, K, up_row_offset, err, stream, glu);
+#define GATED(BN_, TC_, STAGES_) \
+    return launch_tc<BN_, TC_EPI_SWIGLU, TC_, STAGES_>(ta, tb, C, ldc, M, N, K, up_row_offset, err, stream, glu)
+        const bool alone = (long long)((M + TC_BM - 1) / TC_BM) * ((N + bn / 2 - 1) / (bn / 2)) <= rllm_sm_count();
+        if (c_dtype == RLLM_F32) {
+            if (bn == 256) { GATED(256, float, 4); }
+            if (bn == 128) { if (alone) { GATED(128, float, 6); } GATED(128, float, 3); }
+            if (alone) { GATED(64, float, 8); }
+            GATED(64, float, 4);
+        }
+        if (bn == 256) { GATED(256, bf16, 4); }
+        if (bn == 128) { if (alone) { GATED(128, bf16, 6); } GATED(128, bf16, 3); }
+        if (alone) { GATED(64, bf16, 8); }
+        GATED(64, bf16, 4);
+#undef GATED
     }
     return (int)cudaErrorInvalidValue;
+}
+
+RLLM_API int rllm_gemm_tc_glu(const void* A, const void* B, void* C, int c_dtype, int M, int N, int K, int lda, int ldb,
+                              int ldc, int epilogue, int up_row_offset, float glu_limit, float glu_alpha,
+                              float glu_shift, int* err, cudaStream_t stream) {
+    return rllm_gemm_tc_tile(A, B, C, c_dtype, M, N, K, lda, ldb, ldc, epilogue, up_row_offset, glu_limit, glu_alpha, glu_shift,
+                             256, err, stream);
 }
 
 RLLM_API int rllm_gemm_tc(const void* A, const void* B, void* C, int c_dtype, int M, int N, int K, int lda, int ldb,
@@ -783,4 +822,5 @@ TC_DEFINE_WAIT_CONTROLS(rllm_tc)
 // the packed-argument forms (common.cuh) for the host runtime's replay of recorded launches
 RLLM_PACKED(rllm_gemm_tc)
 RLLM_PACKED(rllm_gemm_tc_glu)
+RLLM_PACKED(rllm_gemm_tc_tile)
 RLLM_PACKED(rllm_gemm_tc_swap)

@@ -1500,10 +1500,10 @@ def _tc_ok(a, w, _meta=False) -> bool:
             and (_meta or a.data_ptr() % 16 == 0) and w.data_ptr() % 16 == 0)
 
 
-def gemm_tc(a, w, out, epilogue=EPI_STORE, up_row_offset=0, glu=None):
+def gemm_tc(a, w, out, epilogue=EPI_STORE, up_row_offset=0, glu=None, tile=256):
     """out (+)= a . w^T on the tcgen05 tensor cores (TMA-fed, accumulators in tensor memory).
     epilogue as for skinny_gemm; glu = (limit, alpha, shift): the gated epilogue's constants (None:
-    SwiGLU).  See gemm_tc.cu."""
+    SwiGLU); tile: rows of w per tile, 256, or 128 or 64 with the gated epilogue.  See gemm_tc.cu."""
     _need_cuda(a, w, out)
     if not _tc_ok(a, w):
         raise KernelError("gemm_tc needs bfloat16 operands, k a multiple of 8 and 16-byte aligned rows")
@@ -1515,10 +1515,10 @@ def gemm_tc(a, w, out, epilogue=EPI_STORE, up_row_offset=0, glu=None):
     else:
         assert w.shape[0] == n
     limit, alpha, shift = glu or (0.0, 1.0, 0.0)
-    st = _lib("tc").rllm_gemm_tc_glu(
+    st = _lib("tc").rllm_gemm_tc_tile(
         _ptr(a), _ptr(w), _ptr(out), c_int(_code(out)), c_int(m), c_int(n), c_int(k), c_int(a.stride(0)),
         c_int(w.stride(0)), c_int(out.stride(0)), c_int(epilogue), c_int(up_row_offset), c_float(limit),
-        c_float(alpha), c_float(shift), _ptr(error_word(a.device)), _stream())
+        c_float(alpha), c_float(shift), c_int(tile), _ptr(error_word(a.device)), _stream())
     if st >= 30000:
         raise KernelError(f"gemm_tc: tensor map encoding failed (CUresult {st - 30000}) for m={m} n={n} k={k}")
     _check(st, "gemm_tc")
@@ -1862,6 +1862,34 @@ def _prefer_tc2(m: int, n_col_tiles: int, n_sm: int = 148) -> bool:
 USE_TC2 = True
 
 
+def _gated_tile(m: int, F: int, k: int, n_sm: int = 148) -> int:
+    """Which kernel takes a gated product of m > 64 rows and F features: 64, 128 or 256 rows of the stacked matrix per 128-row
+    tile of gemm_tc, or 2 for gemm_tc2.  While all 128-wide tiles run at once, two an SM, nothing is as fast: every SM streams
+    weights, and a tile's epilogue has another tile's MMAs beside it.  64-wide ones, as long as they too run at once and K is so
+    short that a launch is mostly its start and its end.  With k up to 1,024 the epilogue decides at every size.  us, 64 / 128 /
+    256 wide / two SMs:
+        F 3,072,  k 1,024:   77 rows 9.8 / 11.7 / 17.1 / 12.7, 384 rows 11.0 / 12.9 / 17.5 / 19.0, 512 rows 15.4 / 14.7 / 18.0 / 19.1,
+                             2,048 rows 38.5 / 28.6 / 38.7 / 40.9
+        F 6,144,  k 2,048:   77 rows 16.6 / 17.8 / 24.3 / 24.8, 384 rows 27.1 / 22.1 / 25.3 / 30.8, 512 rows 37.3 / 33.4 / 36.3 / 30.9
+        F 8,192,  k 4,096:   77 rows 33.5 / 33.4 / 43.9 / 42.0, 256 rows 50.5 / 40.2 / 42.4 / 40.8, 300 rows 68.5 / 61.2 / 63.1 / 57.6
+        F 12,288, k 4,096:   77 rows 53.1 / 44.2 / 47.9 / 53.2, 200 rows 70.7 / 63.7 / 66.8 / 54.7, 384 rows 92.7 / 73.2 / 70.0 / 80.9
+        F 25,600, k 5,120:   77 rows 110 / 106 / 110 / 117, 200 rows 169 / 132 / 125 / 114"""
+    rows, most = -(-m // 128), 2 * n_sm
+    if k <= 2048 and rows * -(-F // 32) <= most:
+        return 64
+    if k <= 1024 or rows * -(-F // 64) <= most:
+        return 128
+    return 2 if _prefer_tc2(m, -(-F // 128), n_sm) else 256
+
+
+def _gemm_gated(h, w_gate_up, out, glu=None):
+    F = out.shape[1]
+    tile = _gated_tile(h.shape[0], F, h.shape[1], sm_count(h.device))
+    if tile == 2:
+        return gemm_tc2(h, w_gate_up, out, EPI_SWIGLU, up_row_offset=F, glu=glu)
+    return gemm_tc(h, w_gate_up, out, EPI_SWIGLU, up_row_offset=F, glu=glu, tile=tile)
+
+
 def gate_up_swiglu(h, w_gate_up, out, glu=None):
     """out[m, F] = silu(h . Wg^T) * (h . Wu^T) with w_gate_up = [Wg; Wu] stacked ([2F, k]).
     bfloat16: one kernel (the weight-streaming kernel up to 64 rows, the tcgen05 kernel above);
@@ -1874,8 +1902,7 @@ def gate_up_swiglu(h, w_gate_up, out, glu=None):
     rows = h.xw if isinstance(h, NormedRows) else h
     if glu is not None:
         if not _skinny_ok(rows, w_gate_up) and _tc_ok(h, w_gate_up) and out.data_ptr() % 16 == 0:
-            many = gemm_tc2 if _prefer_tc2(m, -(-F // 128), sm_count(h.device)) else gemm_tc
-            return many(h, w_gate_up, out, EPI_SWIGLU, up_row_offset=F, glu=glu)
+            return _gemm_gated(h, w_gate_up, out, glu)
         return glu_clamped(linear(h, w_gate_up, out_dtype=torch.float32), out, *glu)
     if _skinny_ok(rows, w_gate_up):
         if _prefer_stream(rows, w_gate_up, 2 * F, swiglu=True):
@@ -1886,9 +1913,7 @@ def gate_up_swiglu(h, w_gate_up, out, glu=None):
     if isinstance(h, NormedRows):
         raise KernelError("gate_up_swiglu: a deferred norm needs a product that one of the few-row kernels takes")
     if _tc_ok(h, w_gate_up) and out.data_ptr() % 16 == 0:
-        # tcgen05, activation in the epilogue; two SMs per tile where that takes fewer waves
-        many = gemm_tc2 if _prefer_tc2(m, -(-F // 128), sm_count(h.device)) else gemm_tc
-        return many(h, w_gate_up, out, EPI_SWIGLU, up_row_offset=F)
+        return _gemm_gated(h, w_gate_up, out)            # tcgen05, activation in the epilogue
     gu = linear(h, w_gate_up, out_dtype=torch.float32)     # same rounding points as the fused kernels
     return silu_mul(gu, out)
 
