@@ -57,6 +57,7 @@ class PagedGroup:
         self.allocator = BlockAllocator(n_blocks)
         self.pool = None                               # device tensor, see CacheManager.allocate_device
         self.pool_k = self.pool_v = None               # in place of `pool` when value heads have a size of their own
+        self._planes = None                            # the pool's tensors and the views that `planes` has made of them
 
     def first_needed_block(self, length: int) -> int:
         """Logical index of the first block that tokens at positions >= length can still read
@@ -71,12 +72,19 @@ class PagedGroup:
         return -(-self.need.keep_first // self.block_size) if self.need.window > 0 else 0
 
     def planes(self, plane: int):
-        """(keys, values) of one run entry: [pages, kv_heads, block_size, head size]."""
-        if self.pool is not None:
-            return self.pool[plane, 0], self.pool[plane, 1]
-        if self.pool_v is None:                        # the values lie in the key rows
-            return self.pool_k[plane], self.pool_k[plane]
-        return self.pool_k[plane], self.pool_v[plane]
+        """(keys, values) of one run entry: [pages, kv_heads, block_size, head size].  The views are made once per pool."""
+        owner = (self.pool, self.pool_k, self.pool_v)
+        if self._planes is None or any(a is not b for a, b in zip(self._planes[0], owner)):
+            self._planes = (owner, {})
+        views = self._planes[1]
+        if plane not in views:
+            if self.pool is not None:
+                views[plane] = self.pool[plane, 0], self.pool[plane, 1]
+            elif self.pool_v is None:                  # the values lie in the key rows
+                views[plane] = self.pool_k[plane], self.pool_k[plane]
+            else:
+                views[plane] = self.pool_k[plane], self.pool_v[plane]
+        return views[plane]
 
 
 # Pages of a windowed group are given back in runs of this many keys: the attention kernels round

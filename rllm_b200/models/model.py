@@ -170,7 +170,10 @@ class DecoderModel:
             nxt = self.blocks[self.run_order[i + 1].layer] if i + 1 < len(self.run_order) else None
             if nxt is not None and self.run_order[i + 1].junction is not None:
                 nxt = None                               # a junction follows: the block prepares nothing beyond itself
-            defers = getattr(block, "DEFERS_NORM", False) and getattr(nxt, "DEFERS_NORM", False)
+            # (with more rows than a block defers norms for, its launches do not depend on what follows: the last layer then
+            # replays the record of the others too)
+            defers = (getattr(block, "DEFERS_NORM", False) and getattr(nxt, "DEFERS_NORM", False)
+                      and x.shape[0] <= getattr(block, "DEFER_MAX_ROWS", x.shape[0]))
             key = None
             if traces is not None and self._builds[e.layer] is not None:
                 view = views[i]

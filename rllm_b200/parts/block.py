@@ -76,6 +76,7 @@ class PreNormBlock:
         return ps
 
     DEFERS_NORM = True
+    DEFER_MAX_ROWS = ops.SKINNY_MAX_ROWS       # beyond it `deferral` answers no whatever the parts are
     CAPTURE_SAFE = True
     TRACEABLE = True
 
