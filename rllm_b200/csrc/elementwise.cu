@@ -372,13 +372,30 @@ qk_norm_rope_store_token_kernel(const TI* qkv, const float* __restrict__ q_norm_
     // grid has completed, and so the product before it) it reads only the step's index arrays and
     // keys of earlier steps, and that part of it then runs beside this kernel and the end of the one before.
     pdl_launch_dependents();
-    pdl_wait();
     const int t = blockIdx.x;
     const int half = hd >> 1;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n_heads = write_kv ? H + 2 * K : H;
     const size_t width = (size_t)(H + 2 * K) * hd;
     const int units = half >> 1;                  // float2 units per half head
+    // what no kernel of this step writes: the token's slot (uploaded before the first one) and this lane's norm weights
+    int slot = slots[t];
+    float2 wlo[HPW][U], whi[HPW][U];
+#pragma unroll
+    for (int i = 0; i < HPW; ++i) {
+        const int hx = (blockIdx.y * HPW + i) * 8 + warp;
+        const float* nw = hx < H ? q_norm_w : hx < H + K ? k_norm_w : nullptr;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            wlo[i][u] = whi[i][u] = make_float2(1.f, 1.f);
+            if (nw && lane + 32 * u < units) {
+                const int j = (lane + 32 * u) * 2;
+                wlo[i][u] = make_float2(nw[j], nw[j + 1]);
+                whi[i][u] = make_float2(nw[j + half], nw[j + half + 1]);
+            }
+        }
+    }
+    pdl_wait();
     // this warp's heads are asked for first: their values arrive while the rest is worked out
     float a[HPW][U][2], b[HPW][U][2];
     float2 cs[U][2];                              // (cos, sin) of this lane's pairs
@@ -405,7 +422,6 @@ qk_norm_rope_store_token_kernel(const TI* qkv, const float* __restrict__ q_norm_
             }
         }
     }
-    int slot = slots[t];
     if (slot >= n_slots) {
         if (tid == 0 && blockIdx.y == 0 && err) atomicExch(err, RLLM_ERR_SLOT);
         slot = -1;
@@ -438,7 +454,7 @@ qk_norm_rope_store_token_kernel(const TI* qkv, const float* __restrict__ q_norm_
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     float av = a[i][u][e], bv = b[i][u][e];
-                    if (nw) { av = av * rs * nw[j + e]; bv = bv * rs * nw[j + e + half]; }
+                    if (nw) { av = av * rs * (e ? wlo[i][u].y : wlo[i][u].x); bv = bv * rs * (e ? whi[i][u].y : whi[i][u].x); }
                     if (kind != 2) {
                         const float2 c = cs[u][e];
                         const float a2 = av * c.x - bv * c.y, b2 = av * c.y + bv * c.x;

@@ -292,14 +292,18 @@ latent_rope_store_kernel(const TQ* q, long long ld_q, const float* kv, long long
                          const float* __restrict__ kv_norm_w, const float2* cs_table, float cs_mult,
                          const int* __restrict__ slots, TO* q_att, TO* cache, int H, int dq, int r, int rank, int bs,
                          float eps, int write_kv, int n_slots, int* err, int pairs) {
+    // Blocks y > 0: 256 (head, pair)s of the queries each.  Block y = 0: the latent, its norm and the shared key part.  (One block
+    // a token went through its 1,024 pairs four at a time, a round trip each, and through the latent behind them: 6.3 us.)
     __shared__ float red[33];
+    constexpr int NR = 4;                               // columns of the latent a thread holds (rank up to 1,024)
     pdl_launch_dependents();
-    pdl_wait();
     const int t = blockIdx.x, tid = threadIdx.x;
     const int half = r >> 1, W = rank + r;
     const float2* cs = cs_table + (size_t)t * half;
-    // queries: every (head, pair)
-    for (int i = tid; i < H * half; i += blockDim.x) {
+    if (blockIdx.y > 0) {
+        pdl_wait();
+        const int i = (blockIdx.y - 1) * 256 + tid;
+        if (i >= H * half) return;
         const int h = i / half, j = i - h * half;
         const TQ* src = q + (size_t)t * ld_q + (size_t)h * (dq + r) + dq;
         const float2 a = cs[j];
@@ -309,22 +313,27 @@ latent_rope_store_kernel(const TQ* q, long long ld_q, const float* kv, long long
         TO* dst = q_att + ((size_t)t * H + h) * W + rank;
         dst[iu] = from_f<TO>(u * c - w * s);
         dst[iv] = from_f<TO>(w * c + u * s);
+        return;
     }
-    const float* row = kv + (size_t)t * ld_kv;
-    float ss = 0.f;
-    for (int i = tid; i < rank; i += blockDim.x) ss += row[i] * row[i];
-    ss = block_sum(ss, red);
-    if (!write_kv) return;
-    int slot = slots[t];
+    int slot = write_kv ? slots[t] : -1;
+    float wn[NR], v[NR];
+#pragma unroll
+    for (int k = 0; k < NR; ++k) wn[k] = tid + 256 * k < rank ? kv_norm_w[tid + 256 * k] : 0.f;
+    pdl_wait();
     if (slot >= n_slots) {
         if (tid == 0 && err) atomicExch(err, RLLM_ERR_SLOT);
         slot = -1;
     }
     if (slot < 0) return;
-    const float rs = 1.0f / sqrtf(ss / (float)rank + eps);
+    const float* row = kv + (size_t)t * ld_kv;
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < NR; ++k) v[k] = tid + 256 * k < rank ? row[tid + 256 * k] : 0.f;
+#pragma unroll
+    for (int k = 0; k < NR; ++k) ss += v[k] * v[k];
+    for (int i = tid + 256 * NR; i < rank; i += 256) ss += row[i] * row[i];
     TO* dst = cache + (size_t)slot * W;                 // one head: page * bs + offset is the row
-    for (int i = tid; i < rank; i += blockDim.x) dst[i] = from_f<TO>(row[i] * rs * kv_norm_w[i]);
-    for (int j = tid; j < half; j += blockDim.x) {
+    for (int j = tid; j < half; j += 256) {
         const float2 a = cs[j];
         const float c = a.x * cs_mult, s = a.y * cs_mult;
         const int iu = pairs ? 2 * j : j, iv = pairs ? 2 * j + 1 : j + half;
@@ -332,6 +341,12 @@ latent_rope_store_kernel(const TQ* q, long long ld_q, const float* kv, long long
         dst[rank + iu] = from_f<TO>(u * c - w * s);
         dst[rank + iv] = from_f<TO>(w * c + u * s);
     }
+    ss = block_sum(ss, red);
+    const float rs = 1.0f / sqrtf(ss / (float)rank + eps);
+#pragma unroll
+    for (int k = 0; k < NR; ++k)
+        if (tid + 256 * k < rank) dst[tid + 256 * k] = from_f<TO>(v[k] * rs * wn[k]);
+    for (int i = tid + 256 * NR; i < rank; i += 256) dst[i] = from_f<TO>(row[i] * rs * kv_norm_w[i]);
 }
 
 RLLM_API int rllm_latent_rope_store(const void* q, int q_dt, long long ld_q, const float* kv, long long ld_kv,
@@ -344,8 +359,11 @@ RLLM_API int rllm_latent_rope_store(const void* q, int q_dt, long long ld_q, con
         ld_q < (long long)H * (dq + r) || ld_kv < rank + r)
         return (int)cudaErrorInvalidValue;
     const int ns = (int)(n_slots > 0x7fffffffLL ? 0x7fffffffLL : n_slots);
+    const long long pairs_of_token = (long long)H * (r / 2);
+    if (pairs_of_token > 256LL * 65534) return (int)cudaErrorInvalidValue;
+    const dim3 grid(n, 1 + (unsigned)((pairs_of_token + 255) / 256));
 #define LAUNCH(TQ, TO)                                                                                           \
-    return rllm_launch(latent_rope_store_kernel<TQ, TO>, dim3(n), dim3(256), 0, stream, (const TQ*)q, ld_q, kv,   \
+    return rllm_launch(latent_rope_store_kernel<TQ, TO>, grid, dim3(256), 0, stream, (const TQ*)q, ld_q, kv,      \
                        ld_kv, kv_norm_w, (const float2*)cs_table, cs_mult, slots, (TO*)q_att, (TO*)cache, H, dq, r, \
                        rank, bs, eps, write_kv, ns, err, pairs)
     if (q_dt == RLLM_F32 && out_dt == RLLM_F32) { LAUNCH(float, float); }

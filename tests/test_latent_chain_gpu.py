@@ -1,0 +1,95 @@
+"""Merging the splits of attention through latents and storing its rotated parts, where their loops end: one split and more than are in
+flight at once, splits without keys, values narrower and wider than a block's columns, latents longer than the threads hold."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def ops():
+    from rllm_b200.csrc import ops as o
+    return o
+
+
+@pytest.mark.parametrize("L", [1, 33, 130, 700, 2500])
+@pytest.mark.parametrize("H,rank,rot", [(1, 64, 64), (32, 512, 64), (40, 512, 0), (8, 128, 64)])
+def test_latent_decode(L, H, rank, rot):
+    """Two tokens of one context of L keys and of one of 5 keys: the longer one decides the number of splits."""
+    o, W, bs = ops(), rank + rot, 32
+    g = torch.Generator().manual_seed(L + H)
+    lens = [L, 5]
+    rows = [torch.randn(n, W, generator=g).bfloat16() for n in lens]
+    q = torch.randn(2, H * W, generator=g).bfloat16()
+    if not o.latent_decode_ok(q.to(DEV), W, rank):
+        pytest.skip("not a size of this kernel")
+    blocks = [-(-n // bs) for n in lens]
+    cache = torch.full((sum(blocks), 1, bs, W), float("nan")).bfloat16()
+    table = torch.zeros(2, max(blocks), dtype=torch.int32)
+    at = 0
+    for r, x in enumerate(rows):
+        table[r, :blocks[r]] = torch.arange(at, at + blocks[r])
+        flat = torch.zeros(blocks[r] * bs, W).bfloat16()
+        flat[:lens[r]] = x
+        cache[at:at + blocks[r], 0] = flat.view(blocks[r], bs, W)
+        at += blocks[r]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)                       # noqa: E731
+    out = torch.empty(2, H * rank, dtype=torch.bfloat16, device=DEV)
+    scale = W ** -0.5
+    span = 128 if L <= 128 else -(-L // 128) * 128
+    o.latent_decode_attention(q.to(DEV), cache.to(DEV), out, i32([n - 1 for n in lens]), i32([0, 1]), table.to(DEV), H, W, rank, bs,
+                              scale, 0.0, span)
+    o.check_device_errors()
+    for r, x in enumerate(rows):
+        k = x.double()
+        p = torch.softmax(q[r].double().view(H, W) @ k.t() * scale, -1)
+        want = (p @ k[:, :rank]).reshape(-1)
+        # probabilities and the result in bfloat16: 2^-8 of sums of |p v|, twice
+        size = (p @ k[:, :rank].abs()).reshape(-1)
+        assert bool(((out[r].cpu().double() - want).abs() <= 2.0 ** -7 * size + 1e-6).all()), r
+
+
+@pytest.mark.parametrize("H,rank,r", [(1, 64, 2), (5, 250, 64), (32, 512, 64), (128, 1100, 32), (16, 1024, 64)])
+@pytest.mark.parametrize("pairs", [False, True])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_latent_rope_store(H, rank, r, pairs, dt):
+    o, n, dq, bs = ops(), 3, 16, 4
+    g = torch.Generator().manual_seed(rank + r)
+    q, kv, w = torch.randn(n, H * (dq + r), generator=g), torch.randn(n, rank + r, generator=g), torch.randn(rank, generator=g)
+    ang = torch.rand(n, r // 2, generator=g) * 6.0
+    cs = torch.stack([torch.cos(ang), torch.sin(ang)], -1).contiguous()
+    slots = torch.tensor([6, -1, 1], dtype=torch.int32)
+    W = rank + r
+    q_att, cache = torch.full((n, H * W), 7.0, dtype=dt), torch.full((2, 1, bs, W), 7.0, dtype=dt)
+    got_q, got_c = q_att.to(DEV), cache.to(DEV)
+    o.latent_rope_store(q.to(DEV), kv.to(DEV), w.to(DEV), cs.to(DEV), 1.5, slots.to(DEV), got_q, got_c, H, dq, r, rank, bs, 1e-6,
+                        pairs=pairs)
+    o.check_device_errors()
+
+    def rotate(x, c):                                                                    # x [..., r], c [r / 2, 2]
+        co, si = c[..., 0].double() * 1.5, c[..., 1].double() * 1.5
+        out = torch.empty_like(x, dtype=torch.float64)
+        u, v = (x[..., 0::2], x[..., 1::2]) if pairs else (x[..., :r // 2], x[..., r // 2:])
+        a, b = u.double() * co - v.double() * si, v.double() * co + u.double() * si
+        if pairs:
+            out[..., 0::2], out[..., 1::2] = a, b
+        else:
+            out[..., :r // 2], out[..., r // 2:] = a, b
+        return out
+
+    eps = 2.0 ** -8 if dt is torch.bfloat16 else 2.0 ** -20
+    for t in range(n):
+        head = got_q[t].cpu().view(H, W)
+        assert bool((head[:, :rank] == 7.0).all())
+        want = rotate(q[t].view(H, dq + r)[:, dq:], cs[t])
+        assert bool(((head[:, rank:].double() - want).abs() <= eps * (want.abs() + 4.0)).all())
+        if slots[t] < 0:
+            continue
+        row = got_c.cpu().view(-1, W)[slots[t]].double()
+        lat = kv[t, :rank].double()
+        want = lat / torch.sqrt((lat ** 2).mean() + 1e-6) * w.double()
+        assert bool(((row[:rank] - want).abs() <= eps * want.abs() + 1e-5 * want.abs()).all())
+        want = rotate(kv[t, rank:], cs[t])
+        assert bool(((row[rank:] - want).abs() <= eps * (want.abs() + 4.0)).all())
+    rest = [s for s in range(2 * bs) if s not in (6, 1)]
+    assert bool((got_c.cpu().view(-1, W)[rest] == 7.0).all())
