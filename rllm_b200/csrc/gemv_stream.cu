@@ -88,6 +88,15 @@ struct SvNorm {
     float inv_d, eps;
 };
 
+// Products of one shape on inputs of their own, run as one (store epilogue): W is their matrices one behind the other, X and C
+// their planes likewise.  A share may reach from one matrix into the next, not further; its chunks end where a matrix ends.
+// (One launch in place of several: their starts and ends, 2 to 4 us each, happen once.)
+struct SvStack {
+    int gran;                 // granules of one matrix (0: a single product)
+    int m;                    // rows of X and of C per plane
+    long long plane;          // elements from one plane of C to the next
+};
+
 // The share of CTA `c` of `G`: granules [first, last).
 __device__ __forceinline__ void sv_share(int n_gran, int c, int G, int& first, int& last) {
     first = (int)(((long long)n_gran * c) / G);
@@ -106,7 +115,7 @@ __device__ __forceinline__ void sv_share(int n_gran, int c, int G, int& first, i
 template <int NT, int EPI, typename TC, int ATOMS, int STAGES>
 __global__ void __launch_bounds__(SV_THREADS)
 gemv_stream_kernel(const __grid_constant__ SvMaps maps, TC* __restrict__ C, int ldc, int m, int n, int K,
-                   int up_row_offset, int* err, const SvNorm nm) {
+                   int up_row_offset, int* err, const SvNorm nm, const SvStack sk) {
     constexpr int ROWS = 128 / ATOMS;
     constexpr int SLOTS = ROWS / 16;
     constexpr int BK = ATOMS * SV_ATOM;
@@ -129,7 +138,15 @@ gemv_stream_kernel(const __grid_constant__ SvMaps maps, TC* __restrict__ C, int 
     int g_first, g_last;
     sv_share(n_gran, blockIdx.x, gridDim.x, g_first, g_last);
     const int nkb = (K + BK - 1) / BK;
-    const int n_chunks = (g_last - g_first + GRAN_PER_CHUNK - 1) / GRAN_PER_CHUNK;
+    // chunks [g_first, g_cut) and [g_cut, g_last): the cut lies where the share passes from one stacked matrix into the next
+    const int plane0 = sk.gran ? g_first / sk.gran : 0;
+    const int g_cut = sk.gran ? min(g_last, (plane0 + 1) * sk.gran) : g_last;
+    const int n_before = (g_cut - g_first + GRAN_PER_CHUNK - 1) / GRAN_PER_CHUNK;
+    const int n_chunks = n_before + (g_last - g_cut + GRAN_PER_CHUNK - 1) / GRAN_PER_CHUNK;
+    auto chunk_first = [&](int chunk) {
+        return chunk < n_before ? g_first + chunk * GRAN_PER_CHUNK : g_cut + (chunk - n_before) * GRAN_PER_CHUNK;
+    };
+    auto chunk_size = [&](int chunk, int g0) { return min(GRAN_PER_CHUNK, (chunk < n_before ? g_cut : g_last) - g0); };
     const int total = n_chunks * nkb;                     // stages this CTA streams
 
     // Every thread signals at once that the next kernel of the stream may be scheduled: all CTAs of
@@ -154,8 +171,8 @@ gemv_stream_kernel(const __grid_constant__ SvMaps maps, TC* __restrict__ C, int 
         // (one in all for a whole chunk), twice that with SwiGLU, and one for the batch rows.
         auto issue_w = [&](int it) {
             const int s = it % STAGES, chunk = it / nkb, kb = it - chunk * nkb;
-            const int g0 = g_first + chunk * GRAN_PER_CHUNK;
-            const int ng = min(GRAN_PER_CHUNK, g_last - g0);
+            const int g0 = chunk_first(chunk);
+            const int ng = chunk_size(chunk, g0);
             unsigned char* st = smem + (size_t)s * STAGE_BYTES;
             mbar_expect_tx(&full_bar[s], ATOMS * (HALVES * ng * SV_GRAN_BYTES + XATOM_BYTES));
 #pragma unroll
@@ -174,7 +191,8 @@ gemv_stream_kernel(const __grid_constant__ SvMaps maps, TC* __restrict__ C, int 
         };
         auto issue_x = [&](int it) {
             const int s = it % STAGES, kb = it % nkb;
-            tma_load_3d(smem + (size_t)s * STAGE_BYTES + SV_W_BYTES, &maps.x, 0, 0, kb * ATOMS, &full_bar[s]);
+            const int x0 = sk.gran ? (plane0 + (it / nkb >= n_before)) * sk.m : 0;
+            tma_load_3d(smem + (size_t)s * STAGE_BYTES + SV_W_BYTES, &maps.x, 0, x0, kb * ATOMS, &full_bar[s]);
         };
         if (lane != 0) return;
         const int head = min(STAGES, total);
@@ -249,8 +267,8 @@ gemv_stream_kernel(const __grid_constant__ SvMaps maps, TC* __restrict__ C, int 
     float acc[SLOTS][NT][4];
     int it = 0;
     for (int chunk = 0; chunk < n_chunks; ++chunk) {
-        const int g0 = g_first + chunk * GRAN_PER_CHUNK;
-        const int ng = min(GRAN_PER_CHUNK, g_last - g0);
+        const int g0 = chunk_first(chunk);
+        const int ng = chunk_size(chunk, g0);
         const int n_slots = (EPI == SV_EPI_SWIGLU) ? ng : (ng + 1) >> 1;
         // where slot sl lies in a stage: the chunk's boxes follow one another, largest first, each as
         // [atom][rows of the box]; a slot lies in one box (an odd last granule is a box of its own)
@@ -368,7 +386,12 @@ gemv_stream_kernel(const __grid_constant__ SvMaps maps, TC* __restrict__ C, int 
         }
         if (!waited) { pdl_wait(); waited = true; }      // C belongs to the kernels before until here
         // rows of this lane in slot `warp`: row g (sums 0, 1) and row g + 8 (sums 2, 3); batch columns 8j + 2t, + 1
-        const int row_end = min(n, g_last * SV_GRAN);
+        const int row_end = min(n, (g0 + ng) * SV_GRAN);
+        TC* Cp = C;                                       // row r of stacked matrix p goes to column r - p * rows of plane p
+        if (EPI == SV_EPI_STORE && sk.gran) {
+            const long long plane = plane0 + (chunk >= n_before);
+            Cp += plane * sk.plane - plane * sk.gran * SV_GRAN;
+        }
         if (EPI == SV_EPI_SWIGLU) {
             const int f = (g0 + warp) * SV_GRAN + g;
             if (f < row_end) {
@@ -395,7 +418,7 @@ gemv_stream_kernel(const __grid_constant__ SvMaps maps, TC* __restrict__ C, int 
                     for (int e = 0; e < 2; ++e) {
                         const int b = 8 * j + 2 * t + e;
                         if (b < m) {
-                            TC* c = C + (size_t)b * ldc + row;
+                            TC* c = Cp + (size_t)b * ldc + row;
                             const float val = v[j][2 * h + e];
                             if (EPI == SV_EPI_ACCUM) {
                                 const float sum = c_old[j][2 * h + e] + val;
@@ -447,11 +470,12 @@ struct SvProblem {
     int m, n, K, ldw, ldx, ldc, up, grid, nt, w_rows, stages;
     int* err;
     SvNorm nm;
+    SvStack sk;
 };
 
 template <int NT, int EPI, typename TC, int ATOMS, int STAGES>
 static int launch_sv_stages(const SvMaps& maps, void* C, int ldc, int m, int n, int K, int up, int grid, int* err,
-                            const SvNorm& nm, cudaStream_t stream) {
+                            const SvNorm& nm, const SvStack& sk, cudaStream_t stream) {
     constexpr int SLOTS = 128 / ATOMS / 16;
     constexpr size_t smem = (size_t)STAGES * (SV_W_BYTES + ATOMS * NT * SV_GRAN_BYTES) +
                             2 * (SV_WARPS * SLOTS * NT * 32 * 4) * sizeof(float) + 1024;
@@ -462,7 +486,7 @@ static int launch_sv_stages(const SvMaps& maps, void* C, int ldc, int m, int n, 
         if (e != cudaSuccess) return (int)e;
         attr_set = true;
     }
-    return rllm_launch(kern, dim3(grid), dim3(SV_THREADS), smem, stream, maps, (TC*)C, ldc, m, n, K, up, err, nm);
+    return rllm_launch(kern, dim3(grid), dim3(SV_THREADS), smem, stream, maps, (TC*)C, ldc, m, n, K, up, err, nm, sk);
 }
 
 template <int NT, int EPI, typename TC, int ATOMS>
@@ -472,13 +496,13 @@ static int launch_sv_atoms(const SvProblem& p, cudaStream_t stream) {
         int st = sv_tmap(&maps.w[lvl], p.W, p.w_rows, p.K, p.ldw, (8 >> lvl) * SV_GRAN, ATOMS);
         if (st) return st;
     }
-    int st = sv_tmap(&maps.x, p.X, p.m, p.K, p.ldx, 8 * NT, ATOMS);
+    int st = sv_tmap(&maps.x, p.X, p.sk.gran ? p.m * (p.n / (p.sk.gran * SV_GRAN)) : p.m, p.K, p.ldx, 8 * NT, ATOMS);
     if (st) return st;
     if (p.stages == 10 && ATOMS * NT <= 4)           // ten stages of the widest shapes do not fit; they get five
-        return launch_sv_stages<NT, EPI, TC, ATOMS, 10>(maps, p.C, p.ldc, p.m, p.n, p.K, p.up, p.grid, p.err, p.nm, stream);
+        return launch_sv_stages<NT, EPI, TC, ATOMS, 10>(maps, p.C, p.ldc, p.m, p.n, p.K, p.up, p.grid, p.err, p.nm, p.sk, stream);
     if (p.stages == 3)
-        return launch_sv_stages<NT, EPI, TC, ATOMS, 3>(maps, p.C, p.ldc, p.m, p.n, p.K, p.up, p.grid, p.err, p.nm, stream);
-    return launch_sv_stages<NT, EPI, TC, ATOMS, 5>(maps, p.C, p.ldc, p.m, p.n, p.K, p.up, p.grid, p.err, p.nm, stream);
+        return launch_sv_stages<NT, EPI, TC, ATOMS, 3>(maps, p.C, p.ldc, p.m, p.n, p.K, p.up, p.grid, p.err, p.nm, p.sk, stream);
+    return launch_sv_stages<NT, EPI, TC, ATOMS, 5>(maps, p.C, p.ldc, p.m, p.n, p.K, p.up, p.grid, p.err, p.nm, p.sk, stream);
 }
 
 // The stage shape follows the share of a CTA: few rows, more k-columns per stage.
@@ -523,6 +547,7 @@ RLLM_API int rllm_gemv_stream(const void* W, const void* X, void* C, int c_dtype
     p.up = up_row_offset; p.grid = grid; p.stages = stages; p.nt = m <= 8 ? 1 : 2; p.err = err;
     p.w_rows = epilogue == SV_EPI_SWIGLU ? up_row_offset + n : n;
     p.nm = SvNorm{};
+    p.sk = SvStack{};
     if (xw_out || ssq_out || w_next) {
         if (epilogue != SV_EPI_ACCUM || !xw_out || !ssq_out || !w_next) return (int)cudaErrorInvalidValue;
         p.nm.xw_out = (bf16*)xw_out; p.nm.w_next = w_next; p.nm.ssq_out = ssq_out; p.nm.ld_xw = ld_xw;
@@ -551,7 +576,28 @@ RLLM_API int rllm_gemv_stream(const void* W, const void* X, void* C, int c_dtype
     return (int)cudaErrorInvalidValue;
 }
 
+// C[i] = X[i] . W[i]^T for the `planes` contiguous planes of X [planes, m, K], W [planes, n, K] and C [planes, m, n] (float32), m
+// <= 16, n a multiple of 8, K of 64.  grid CTAs (at most all granules of 8 rows, and so many that a share is no longer than one
+// matrix); stages as above.
+RLLM_API int rllm_gemv_stream_stack(const void* W, const void* X, float* C, int m, int n, int K, int planes, int grid, int stages,
+                                    int* err, cudaStream_t stream) {
+    if (m <= 0 || n <= 0 || planes <= 0) return 0;
+    if (m > 16 || n % SV_GRAN || K <= 0 || (K % SV_ATOM) || ((uintptr_t)W & 15) || ((uintptr_t)X & 15) || !err || grid <= 0 ||
+        (stages != 3 && stages != 5 && stages != 10) || (long long)planes * n > 0x7fffffffLL)
+        return (int)cudaErrorInvalidValue;
+    const int n_gran = planes * (n / SV_GRAN);
+    if (grid > n_gran) grid = n_gran;
+    if ((n_gran + grid - 1) / grid > n / SV_GRAN) return (int)cudaErrorInvalidValue;
+    SvProblem p;
+    p.W = W; p.X = X; p.C = C; p.m = m; p.n = planes * n; p.K = K; p.ldw = K; p.ldx = K; p.ldc = n; p.up = 0; p.grid = grid;
+    p.stages = stages; p.nt = m <= 8 ? 1 : 2; p.err = err; p.w_rows = planes * n;
+    p.nm = SvNorm{};
+    p.sk = SvStack{n / SV_GRAN, m, (long long)m * n};
+    return p.nt == 1 ? launch_sv<1, SV_EPI_STORE, float>(p, stream) : launch_sv<2, SV_EPI_STORE, float>(p, stream);
+}
+
 TC_DEFINE_WAIT_CONTROLS(rllm_stream)
 
 // the packed-argument forms (common.cuh) for the host runtime's replay of recorded launches
 RLLM_PACKED(rllm_gemv_stream)
+RLLM_PACKED(rllm_gemv_stream_stack)

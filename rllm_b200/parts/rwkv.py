@@ -30,6 +30,7 @@ STREAMS = "rkvgw"
 @register_part("mixer", "rwkv_time_mix")
 class RWKVTimeMix(Mixer):
     CAPTURE_SAFE = True
+    OUTPUT_MATRIX = "w_o"         # the product behind the heads; a mixer made of mixers may run it with its neighbour's
 
     def __init__(self, params, prefix, runtime):
         super().__init__(params, prefix, runtime)
@@ -56,7 +57,7 @@ class RWKVTimeMix(Mixer):
     def load(self, tensors):
         p, f32 = self.prefix, torch.float32
         self.mu = self._to_device(torch.stack([tensors[p + "mu." + s].to(f32) for s in STREAMS], 0), f32)
-        self.w_r, self.w_k, self.w_v, self.w_g = (self._to_device(tensors[p + s]) for s in "rkvg")
+        self.w_rkvg = self._to_device(torch.stack([tensors[p + s].to(self.runtime.dtype) for s in "rkvg"], 0))
         self.w_1, self.w_2, self.w_o = (self._to_device(tensors[p + s]) for s in ("w1", "w2", "o"))
         if self.w_1.shape[0] != self.w_2.shape[1]:
             raise PartError(f"{p}w1 {tuple(self.w_1.shape)} and {p}w2 {tuple(self.w_2.shape)} do not fit together")
@@ -65,19 +66,36 @@ class RWKVTimeMix(Mixer):
         self.u = self._to_device(tensors[p + "u"], f32)
         self.norm_w = self._to_device(tensors[p + "norm"], f32)
 
-    def forward(self, h, ctx, cache, position=None, residual=None):
+        self._scaled = {}
+
+    @property
+    def output_columns(self):
+        return self.H * self.D
+
+    def scaled_norm(self, factor):
+        """The norm's weight times a constant (made once)."""
+        if factor == 1.0:
+            return self.norm_w
+        if factor not in self._scaled:
+            self._scaled[factor] = self.norm_w * factor
+        return self._scaled[factor]
+
+    def forward(self, h, ctx, cache, position=None, residual=None, into=None, factor=1.0):
+        """`into`, `factor`: the rows that the output projection would read, times `factor`, go to the matrix `into` and the
+        projection is left to the caller (OUTPUT_MATRIX)."""
         n, dt, dev, HD = h.shape[0], self.runtime.dtype, h.device, self.H * self.D
         mixed = torch.empty((len(STREAMS), n, self.hidden_size), dtype=dt, device=dev)
         ops.token_shift(h, self.mu, cache.state, self.prev_off, ctx.seq_ids, ctx.cu_q, cache.slots, mixed)
         proj = torch.empty((5, n, HD), dtype=torch.float32, device=dev)           # r, k, v, gate, decay (raw)
-        for i, w in enumerate((self.w_r, self.w_k, self.w_v, self.w_g)):
-            ops.linear(mixed[i], w, out=proj[i])
+        ops.linear_stack(mixed[:4], self.w_rkvg, proj[:4])
         low = ops.linear(mixed[4], self.w_1, out_dtype=torch.float32)
         low_t = torch.empty((n, self.low), dtype=dt, device=dev)
         ops.rows_act(low, low_t, act="tanh")
         ops.linear(low_t, self.w_2, out=proj[4])
-        out = torch.empty((n, HD), dtype=dt, device=dev)
-        ops.wkv(proj[0], proj[1], proj[2], proj[4], proj[3], self.w0, self.u.view(-1), self.norm_w, self.eps,
+        out = torch.empty((n, HD), dtype=dt, device=dev) if into is None else into
+        ops.wkv(proj[0], proj[1], proj[2], proj[4], proj[3], self.w0, self.u.view(-1), self.scaled_norm(factor), self.eps,
                 cache.state, self.prev_off, h, ctx.cu_q, cache.slots, out, ctx.n_requests, self.H, self.D,
                 segments=ops.time_segments(ctx, dev), one_token=ctx.max_q_len == 1)
+        if into is not None:
+            return None
         return ops.linear(out, self.w_o, out_dtype=torch.float32)
