@@ -68,6 +68,13 @@ struct SgNorm {
 };
 
 
+// What lies at the output of this thread when a block has 16 x 8 of them.
+template <typename TC>
+__device__ __forceinline__ float old_output(const TC* C, int ldc, int r0, int m, int n) {
+    const int row = threadIdx.x & 15, b = threadIdx.x >> 4;
+    return b < m && r0 + row < n ? to_f<TC>(C[(size_t)b * ldc + r0 + row]) : 0.f;
+}
+
 // NT: batch columns / 8.  RT: weight row tiles per CTA (2 for SwiGLU).  U: k steps fetched ahead.
 template <int NT, int EPI, typename TC, int U>
 __global__ void __launch_bounds__(SG_THREADS)
@@ -87,6 +94,13 @@ skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* X, TC* C, int m,
     const int r0 = blockIdx.x * 16;
     const bool norm_out = EPI == EPI_ACCUM && nm.ssq_out != nullptr;
     const bool norm_in = EPI != EPI_ACCUM && nm.ssq_in != nullptr;
+    // Accumulating, up to 8 batch rows: the old value of the one output this thread writes (threads 0..127), fetched beside the
+    // first batch rows.  Read where it is added to, it was a round trip to L2 at the end of every kernel (16 tokens of one
+    // request at the 0.6B sizes 12.34 -> 11.29 ms, with the norm's parts behind the first batch rows' load, which their sum no
+    // longer holds back).  With more rows the loop's own loads are worth the registers (12 rows of 1,024 x 2,048: 4.4 us, with
+    // early old values 4.6 to 5.4; 24 rows of 4,096 x 4,096: 12.5 and 18.8).
+    constexpr bool EARLY_OLD = EPI == EPI_ACCUM && NT == 1;
+    float c_old = 0.f;
     // the following norm's weight at the output column this thread writes (a weight: no need to wait for it)
     const float wn = (norm_out && r0 + (threadIdx.x & 15) < n) ? nm.w_next[r0 + (threadIdx.x & 15)] : 0.f;
     float nsum[GPT];
@@ -156,21 +170,39 @@ skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* X, TC* C, int m,
         // The weights do not depend on the kernel before this one, the activations do: with a
         // programmatic dependent launch the first weight loads are already in flight while the
         // previous kernel drains.  (Without that launch attribute the wait returns at once.)
-        if (s0 == warp) {
-            pdl_wait();
-            load_norm();               // beside the batch rows' loads, while the weights arrive
-        }
+        if constexpr (NT == 1) {
+            if (s0 == warp) pdl_wait();
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int kk = (s0 + u * SG_WARPS) << 5;
-            const bool ok = kk + 8 * t + 8 <= k;
-#pragma unroll
-            for (int j = 0; j < NT; ++j) {
-                const uint4 b = (ok && xok[j]) ? ldg_cached(xrow[j] + kk) : zero;
+            for (int u = 0; u < U; ++u) {
+                const int kk = (s0 + u * SG_WARPS) << 5;
+                const uint4 b = (kk + 8 * t + 8 <= k && xok[0]) ? ldg_cached(xrow[0] + kk) : zero;
+                if (u == 0 && s0 == warp) {
+                    load_norm();           // beside the batch rows' loads, while the weights arrive
+                    if constexpr (EARLY_OLD) c_old = old_output<TC>(C, ldc, r0, m, n);
+                }
 #pragma unroll
                 for (int rt = 0; rt < RT; ++rt) {
-                    mma16816(acc[rt][j], a[u][rt][0].x, a[u][rt][1].x, a[u][rt][0].y, a[u][rt][1].y, b.x, b.y);
-                    mma16816(acc[rt][j], a[u][rt][0].z, a[u][rt][1].z, a[u][rt][0].w, a[u][rt][1].w, b.z, b.w);
+                    mma16816(acc[rt][0], a[u][rt][0].x, a[u][rt][1].x, a[u][rt][0].y, a[u][rt][1].y, b.x, b.y);
+                    mma16816(acc[rt][0], a[u][rt][0].z, a[u][rt][1].z, a[u][rt][0].w, a[u][rt][1].w, b.z, b.w);
+                }
+            }
+        } else {
+            if (s0 == warp) {
+                pdl_wait();
+                load_norm();               // beside the batch rows' loads, while the weights arrive
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int kk = (s0 + u * SG_WARPS) << 5;
+                const bool ok = kk + 8 * t + 8 <= k;
+#pragma unroll
+                for (int j = 0; j < NT; ++j) {
+                    const uint4 b = (ok && xok[j]) ? ldg_cached(xrow[j] + kk) : zero;
+#pragma unroll
+                    for (int rt = 0; rt < RT; ++rt) {
+                        mma16816(acc[rt][j], a[u][rt][0].x, a[u][rt][1].x, a[u][rt][0].y, a[u][rt][1].y, b.x, b.y);
+                        mma16816(acc[rt][j], a[u][rt][0].z, a[u][rt][1].z, a[u][rt][0].w, a[u][rt][1].w, b.z, b.w);
+                    }
                 }
             }
         }
@@ -178,6 +210,9 @@ skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* X, TC* C, int m,
     pdl_wait();                 // warps that had no k step still have to wait before they write
     pdl_launch_dependents();    // the next kernel may start to fill the SMs that this one leaves
     load_norm();
+    if constexpr (EARLY_OLD) {
+        if (warp >= steps) c_old = old_output<TC>(C, ldc, r0, m, n);
+    }
     if (norm_in) {
 #pragma unroll
         for (int j = 0; j < GPT; ++j) nred[(threadIdx.x / NCOL) * GPT + j][threadIdx.x % NCOL] = nsum[j];
@@ -220,6 +255,7 @@ skinny_gemm_kernel(const bf16* __restrict__ W, const bf16* X, TC* C, int m,
         float x_new = 0.f;
         if (ok) {
             if (EPI == EPI_STORE) *c = from_f<TC>(v[0]);
+            else if constexpr (EARLY_OLD) { x_new = c_old + v[0]; *c = from_f<TC>(x_new); }
             else if (EPI == EPI_ACCUM) { x_new = to_f<TC>(*c) + v[0]; *c = from_f<TC>(x_new); }
             else *c = from_f<TC>(v[0] / (1.0f + expf(-v[0])) * v[RT - 1]);
         }
