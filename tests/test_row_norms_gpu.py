@@ -43,6 +43,22 @@ def test_norm_rows(n, d, low):
     close(own, unit, 24)
 
 
+@pytest.mark.parametrize("n,d", [(1, 4), (8, 252), (127, 1024), (8, 2048), (130, 2048), (1, 4096), (130, 4096), (127, 8192), (130, 8192),
+                                 (1, 8196), (130, 12288)])
+def test_a_row_is_joined_in_one_rounding(n, d):
+    """Bit for bit, in every form that reads four columns at a time: v * (rs * w) + x with one rounding behind the product rs * w.
+    The rows are whole numbers, so that their sum of squares is exact in any order; the sum in 64 bits of a 48-bit product is
+    rounded twice, which matters in one of 2^29 cases."""
+    a = torch.randint(-6, 7, (n, d), generator=torch.Generator().manual_seed(7)).float()
+    a[:, 0] = 3.0
+    x, w = rnd(n, d, seed=8), rnd(d, seed=9)
+    xs, low = x.to(DEV), torch.empty(n, d, dtype=torch.bfloat16, device=DEV)
+    ops().norm_rows(a.to(DEV), w.to(DEV), 1e-6, x=xs, add=True, low=low)
+    rs = 1.0 / torch.sqrt((a.double() ** 2).sum(1, keepdim=True).float() / torch.tensor(float(d)) + torch.tensor(1e-6))
+    want = (a.double() * (rs * w).double() + x.double()).float()
+    assert torch.equal(xs.cpu(), want) and torch.equal(low.cpu(), want.bfloat16())
+
+
 @pytest.mark.parametrize("n", [1, 9, 130])
 @pytest.mark.parametrize("d", [4, 1024, 1028, 2052, 4096, 4100, 8192, 8196])
 @pytest.mark.parametrize("dt,shift", [(torch.float32, 0), (torch.float32, 1), (torch.bfloat16, 0), (torch.bfloat16, 1)])
