@@ -862,8 +862,8 @@ def time_segments(ctx, device, length=SEGMENT_TOKENS, shortest=SEGMENT_FROM):
 def wkv(r, k, v, wraw, g, w0, u, norm_w, eps, state, prev_off, h, cu_q, slots, out, n_requests, H, D, segments=None,
         one_token=False):
     """The RWKV recurrence with data-dependent decay, unit norm per head, norm weight and silu gate; see
-    recurrent.cu.  r, k, v, wraw, g float32 [n, H*D] (equal row strides); out activation type (any row
-    stride).  segments: the step's TimeSegments (long portions are then worked through segment by segment, side
+    recurrent.cu.  r, k, v, wraw, g float32 [n, H*D] (equal row strides); out activation type.
+    segments: the step's TimeSegments (long portions are then worked through segment by segment, side
     by side) or None.  one_token: the caller says that every request brings exactly one token."""
     _need_cuda(r, k, v, wraw, g, w0, u, norm_w, state, h, out)
     n = out.shape[0]
@@ -871,8 +871,8 @@ def wkv(r, k, v, wraw, g, w0, u, norm_w, eps, state, prev_off, h, cu_q, slots, o
     for name, t in (("r", r), ("k", k), ("v", v), ("wraw", wraw), ("g", g)):
         _rows2d(t, name)
         assert t.dtype == torch.float32 and t.shape == (n, H * D) and t.stride(0) == r.stride(0)
-    _need_contig(h=h, w0=w0, u=u, norm_w=norm_w)
-    assert _rows2d(out, "out").shape == (n, H * D) and h.dtype == out.dtype and h.shape[0] == n
+    _need_contig(out=out, h=h, w0=w0, u=u, norm_w=norm_w)
+    assert out.shape == (n, H * D) and h.dtype == out.dtype and h.shape[0] == n
     assert w0.dtype == u.dtype == norm_w.dtype == torch.float32
     assert w0.numel() == u.numel() == norm_w.numel() == H * D
     if D > 256:
@@ -888,7 +888,7 @@ def wkv(r, k, v, wraw, g, w0, u, norm_w, eps, state, prev_off, h, cu_q, slots, o
     _check(_lib("recur").rllm_wkv(_ptr(r), _ptr(k), _ptr(v), _ptr(wraw), _ptr(g), c_longlong(r.stride(0)), _ptr(w0),
                                   _ptr(u), _ptr(norm_w), c_float(eps), _ptr(st), c_longlong(st.stride(0)),
                                   c_longlong(prev_off), _ptr(h), c_int(_code(h)), c_int(h.shape[1]), _ptr(cu_q),
-                                  _ptr(slots), _ptr(out), c_longlong(out.stride(0)), c_int(n_requests), c_int(H), c_int(D),
+                                  _ptr(slots), _ptr(out), c_int(n_requests), c_int(H), c_int(D),
                                   _ptr(sg.t0 if sg else None), _ptr(sg.t1 if sg else None), _ptr(sg.req if sg else None),
                                   _ptr(sg.flags if sg else None), _ptr(sg.item0 if sg else None),
                                   _ptr(sg.items if sg else None), c_int(sg.n_items if sg else 0), _ptr(carry),

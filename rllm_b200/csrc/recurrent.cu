@@ -603,7 +603,7 @@ __global__ void __launch_bounds__(wkv_threads(DMAX), DMAX <= 64 ? 4 : 1)
 wkv_kernel(const float* rp, const float* kp, const float* vp, const float* wraw, const float* gp, long long ld,
            const float* __restrict__ w0, const float* __restrict__ u, const float* __restrict__ norm_w, float eps,
            float* state, long long slot_stride, long long prev_off, const TA* h, int width,
-           const int* __restrict__ cu_q, const int* __restrict__ slots, TA* out, long long ld_out, int H, int D,
+           const int* __restrict__ cu_q, const int* __restrict__ slots, TA* out, int H, int D,
            const TimeSegments seg) {
     constexpr int IPT = DMAX / WKV_PARTS;               // key channels per thread
     constexpr int COLS = wkv_cols(DMAX);                // neighbouring value channels per thread
@@ -761,7 +761,7 @@ wkv_kernel(const float* rp, const float* kp, const float* vp, const float* wraw,
             for (int i = lane; i < D; i += 32) ss += s_o[tt * DMAX + i] * s_o[tt * DMAX + i];
             const float rs = 1.0f / sqrtf(warp_sum(ss) / (float)D + eps);
             for (int i = lane; i < D; i += 32)
-                out[(size_t)(tb + tt) * ld_out + col + i] =
+                out[(size_t)(tb + tt) * H * D + col + i] =
                     from_f<TA>(s_o[tt * DMAX + i] * rs * norm_w[col + i] * silu_f(s_g[tt * DMAX + i]));
         }
         __syncthreads();                                 // everyone is done with this chunk
@@ -828,22 +828,22 @@ static int launch_wkv_pass(dim3 grid, cudaStream_t stream, const float* rp, cons
                            const float* vp, const float* wraw, const float* gp, long long ld, const float* w0,
                            const float* u, const float* norm_w, float eps, float* state, long long slot_stride,
                            long long prev_off, const void* h, int width, const int* cu_q, const int* slots, void* out,
-                           long long ld_out, int H, int D, const TimeSegments& seg) {
+                           int H, int D, const TimeSegments& seg) {
     constexpr size_t smem = ((size_t)(6 * TOK + 1) * DMAX + TOK) * sizeof(float);
     static_assert(smem <= 48 * 1024, "more shared memory than a launch gets without asking");
     return rllm_launch(wkv_kernel<TA, DMAX, PASS, TOK>, grid, dim3(wkv_threads(DMAX)), smem, stream, rp, kp, vp, wraw,
                        gp, ld, w0, u, norm_w, eps, state, slot_stride, prev_off, (const TA*)h, width, cu_q, slots, (TA*)out,
-                       ld_out, H, D, seg);
+                       H, D, seg);
 }
 
 template <typename TA, int DMAX>
 static int launch_wkv(int n_requests, cudaStream_t stream, const float* rp, const float* kp, const float* vp,
                       const float* wraw, const float* gp, long long ld, const float* w0, const float* u,
                       const float* norm_w, float eps, float* state, long long slot_stride, long long prev_off,
-                      const void* h, int width, const int* cu_q, const int* slots, void* out, long long ld_out, int H, int D,
+                      const void* h, int width, const int* cu_q, const int* slots, void* out, int H, int D,
                       int one_token, const TimeSegments& seg) {
     constexpr int TOK = wkv_tok(DMAX);
-#define WKV_ARGS rp, kp, vp, wraw, gp, ld, w0, u, norm_w, eps, state, slot_stride, prev_off, h, width, cu_q, slots, out, ld_out, H, D, seg
+#define WKV_ARGS rp, kp, vp, wraw, gp, ld, w0, u, norm_w, eps, state, slot_stride, prev_off, h, width, cu_q, slots, out, H, D, seg
     if (one_token) return launch_wkv_pass<TA, DMAX, 0, 1>(dim3(H, n_requests), stream, WKV_ARGS);
     if (seg.n_items <= 0)
         return launch_wkv_pass<TA, DMAX, 0, TOK>(dim3(H, n_requests), stream, WKV_ARGS);
@@ -863,12 +863,12 @@ static int launch_wkv(int n_requests, cudaStream_t stream, const float* rp, cons
 RLLM_API int rllm_wkv(const float* rp, const float* kp, const float* vp, const float* wraw, const float* gp,
                       long long ld, const float* w0, const float* u, const float* norm_w, float eps, float* state,
                       long long slot_stride, long long prev_off, const void* h, int act_dt, int width,
-                      const int* cu_q, const int* slots, void* out, long long ld_out, int n_requests, int H, int D,
+                      const int* cu_q, const int* slots, void* out, int n_requests, int H, int D,
                       const int* seg_t0, const int* seg_t1, const int* seg_req, const int* seg_flags,
                       const int* req_item0, const int* req_items, int n_items, float* carry, float* decay,
                       int one_token, cudaStream_t stream) {
     if (n_requests <= 0) return 0;
-    if (D <= 0 || D > 256 || H <= 0 || ld_out < (long long)H * D) return (int)cudaErrorInvalidValue;
+    if (D <= 0 || D > 256 || H <= 0) return (int)cudaErrorInvalidValue;
     const int dmax = D <= 32 ? 32 : D <= 64 ? 64 : D <= 128 ? 128 : 256;
     if (prev_off < (long long)H * dmax * dmax) return (int)cudaErrorInvalidValue;
     TimeSegments seg = {seg_t0, seg_t1, seg_req, seg_flags, req_item0, req_items, carry, decay, n_items};
@@ -876,7 +876,7 @@ RLLM_API int rllm_wkv(const float* rp, const float* kp, const float* vp, const f
         return (int)cudaErrorInvalidValue;
 #define LAUNCH(TA, DMAX)                                                                                        \
     return launch_wkv<TA, DMAX>(n_requests, stream, rp, kp, vp, wraw, gp, ld, w0, u, norm_w, eps, state,  \
-                                slot_stride, prev_off, h, width, cu_q, slots, out, ld_out, H, D, one_token, seg)
+                                slot_stride, prev_off, h, width, cu_q, slots, out, H, D, one_token, seg)
 #define BY_D(TA)                                                                                               \
     do {                                                                                                       \
         if (dmax == 32) { LAUNCH(TA, 32); }                                                                    \

@@ -11,8 +11,8 @@ import plain_falalix as pf
 from rllm_b200.cache import CacheManager
 from rllm_b200.cache.native import NativeCacheManager
 from rllm_b200.config import ConfigError, FalalixConfig, config_from_dict
-from rllm_b200.models.model import expected_tensors
-from rllm_b200.parts import PagedKVNeed, StateNeed
+from rllm_b200.models.model import DecoderModel, expected_tensors
+from rllm_b200.parts import PagedKVNeed, Runtime, StateNeed
 from rllm_b200.weights.loader import shape_fits
 
 
@@ -140,3 +140,16 @@ def test_random_weights_mode_makes_a_falalix_folder(tmp_path):
     assert set(got) == set(exp)
     mu = got["l1.mix.right.mu.k"].float()
     assert 0 < float(mu.min()) and float(mu.max()) < 1
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_the_sides_of_a_parallel_layer_keep_their_output_products(dtype):
+    """The attention's rows and the time mixing's are rounded as they are and multiplied by matrices of their own; the scales meet
+    the float32 products.  (One product of both, over rows scaled in front of their rounding, is further from 64 bits.)"""
+    cfg = fc.CASES["heads64"]
+    model = DecoderModel(config_from_dict(cfg).model_spec(), Runtime(torch.device("cpu"), dtype))
+    weights = fc.make_weights(cfg, 1, dtype)
+    model.load_tensors(dict(weights))
+    mixer = model.blocks[0].mixer
+    assert mixer.w_ends is None
+    assert torch.equal(mixer.left.w_o, weights["l0.mix.left.o"]) and torch.equal(mixer.right.w_o, weights["l0.mix.right.o"])
