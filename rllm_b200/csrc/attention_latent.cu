@@ -29,6 +29,7 @@
 #define LAT_TILE 32         // keys per tile
 #define LAT_PAD 8           // bf16 elements of padding per shared-memory row
 #define LAT_MAX_NT 32       // n8 tiles of value columns per warp (V / 2 / 8)
+#define LAT_MAX_SPLITS 8192 // splits of a launch
 
 __device__ __forceinline__ uint32_t lat_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void lat_cp16(uint32_t dst, const void* src, int bytes) {
@@ -329,7 +330,7 @@ RLLM_API int rllm_latent_decode_attention(const void* q, const void* cache, void
                                           int window, cudaStream_t stream) {
     if (n <= 0) return 0;
     if (H <= 0 || W % 16 || V % 64 || V <= 0 || V > 16 * LAT_MAX_NT || V > W || bs <= 0 || split_keys <= 0 ||
-        split_keys % LAT_TILE || n_splits <= 0 || n_splits > 8192 || !part_o || !part_ml || softcap < 0.f || window < 0)
+        split_keys % LAT_TILE || n_splits <= 0 || n_splits > LAT_MAX_SPLITS || !part_o || !part_ml || softcap < 0.f || window < 0)
         return (int)cudaErrorInvalidValue;
     const size_t smem = latent_smem(W);
     if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
@@ -339,6 +340,13 @@ RLLM_API int rllm_latent_decode_attention(const void* q, const void* cache, void
         if (e != cudaSuccess) return (int)e;
         configured = smem;
     }
+    // the merge keeps 8 bytes a split: more than the 48 KB that a launch gets without asking from 6,143 splits on (786,176 keys).
+    // Asked for here, in front of the first launch, so that a refusal leaves nothing half done.
+    const size_t merge_smem = (size_t)n_splits * 2 * sizeof(float);
+    if (merge_smem > 40 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(latent_combine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LAT_MAX_SPLITS * 8);
+        if (e != cudaSuccess) return (int)e;
+    }
     LatentParams p;
     p.q = (const bf16*)q; p.cache = (const bf16*)cache; p.part_o = part_o; p.part_ml = part_ml;
     p.positions = positions; p.seq_ids = seq_ids; p.block_table = block_table; p.table_stride = table_stride;
@@ -347,7 +355,7 @@ RLLM_API int rllm_latent_decode_attention(const void* q, const void* cache, void
     const int chunks = (H + LAT_HEADS - 1) / LAT_HEADS;
     int st = rllm_launch(latent_decode_kernel, dim3(n, chunks, n_splits), dim3(128), smem, stream, p);
     if (st) return st;
-    return rllm_launch(latent_combine_kernel, dim3(n, H), dim3(128), (size_t)n_splits * 2 * sizeof(float), stream, (const float*)part_o,
+    return rllm_launch(latent_combine_kernel, dim3(n, H), dim3(128), merge_smem, stream, (const float*)part_o,
                        (const float*)part_ml, (bf16*)out, H, V, chunks, n_splits);
 }
 

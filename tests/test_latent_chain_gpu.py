@@ -93,3 +93,31 @@ def test_latent_rope_store(H, rank, r, pairs, dt):
         assert bool(((row[rank:] - want).abs() <= eps * (want.abs() + 4.0)).all())
     rest = [s for s in range(2 * bs) if s not in (6, 1)]
     assert bool((got_c.cpu().view(-1, W)[rest] == 7.0).all())
+
+
+@pytest.mark.parametrize("n_splits", [6143, 6144, 8192])
+def test_the_longest_contexts(n_splits):
+    """As many splits as the kernels take.  The context's logical pages go round eight pages of the cache, so that a key counts as
+    often as its page; beside it a token that sees only the first few keys of as many splits."""
+    o, W, bs = ops(), 64, 64
+    L = n_splits * o.LATENT_SPLIT_KEYS
+    g = torch.Generator().manual_seed(n_splits)
+    cache = torch.randn(8, 1, bs, W, generator=g).bfloat16()
+    q = torch.randn(2, W, generator=g).bfloat16()
+    table = (torch.arange(L // bs, dtype=torch.int32) % 8).repeat(2, 1)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)                       # noqa: E731
+    out = torch.full((2, W), float("nan"), dtype=torch.bfloat16, device=DEV)
+    o.latent_decode_attention(q.to(DEV), cache.to(DEV), out, i32([L - 1, 4]), i32([0, 1]), table.to(DEV), 1, W, W, bs, W ** -0.5,
+                              0.0, L)
+    o.check_device_errors()
+    keys = cache.double().view(-1, W)
+    for r, k in enumerate((keys, keys[:5])):
+        times = torch.ones(len(k), dtype=torch.float64)
+        if r == 0:
+            pages = torch.bincount(table[0].long(), minlength=8).double()
+            times = pages.repeat_interleave(bs)
+        s = q[r].double() @ k.t() * W ** -0.5
+        e = times * torch.exp(s - s.max())
+        want, size = (e @ k) / e.sum(), (e @ k.abs()) / e.sum()
+        # probabilities and the result in bfloat16: 2^-8 of sums of |p v|, twice; a million keys' sums in float32
+        assert bool(((out[r].cpu().double() - want).abs() <= (2.0 ** -7 + 2e-4) * size + 1e-6).all()), r
