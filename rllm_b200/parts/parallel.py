@@ -72,7 +72,19 @@ class ParallelMixer(Mixer):
         rows = ops.linear(h, self.w_both, out_dtype=torch.float32)
         return {"rows": rows[:, :self.split]}, {"rows": rows[:, self.split:]}
 
+    def _ends(self, h, ctx, cache, position):
+        """What the stacked output product reads: both sides' rows, each times its scale."""
+        k = self.left.output_columns
+        ends = torch.empty((h.shape[0], self.w_ends.shape[1]), dtype=self.runtime.dtype, device=h.device)
+        rows = self._rows(h)
+        self.left.forward(h, ctx, cache[0], position, into=ends[:, :k], factor=self.left_scale, **rows[0])
+        self.right.forward(h, ctx, cache[1], position, into=ends[:, k:], factor=self.right_scale, **rows[1])
+        return ends
+
     def join(self, h, ctx, cache, position, x, extra=None, mult=1.0, copy=None, add=True):
+        if self.w_ends is not None:                      # the sides have no product of their own then
+            a = ops.linear(self._ends(h, ctx, cache, position), self.w_ends, out_dtype=torch.float32)
+            return ops.join_sum_rows(a, x, mult, add, c=extra, low=copy)
         a, b = self._sides(h, ctx, cache, position)
         form = lambda n: (n.weight, n.eps) if n is not None else None
         return ops.join_sum_rows(a, x, mult, add, form(self.left_norm), self.left_scale, b, form(self.right_norm),
@@ -80,11 +92,7 @@ class ParallelMixer(Mixer):
 
     def forward(self, h, ctx, cache, position=None, residual=None):
         if self.w_ends is not None:
-            k = self.left.output_columns
-            ends = torch.empty((h.shape[0], self.w_ends.shape[1]), dtype=self.runtime.dtype, device=h.device)
-            rows = self._rows(h)
-            self.left.forward(h, ctx, cache[0], position, into=ends[:, :k], factor=self.left_scale, **rows[0])
-            self.right.forward(h, ctx, cache[1], position, into=ends[:, k:], factor=self.right_scale, **rows[1])
+            ends = self._ends(h, ctx, cache, position)
             if residual is not None:
                 ops.linear(ends, self.w_ends, out=residual, accumulate=True)
                 return None

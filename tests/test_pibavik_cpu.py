@@ -242,3 +242,45 @@ def test_plain_experts_weigh_their_input():
     out = pp.experts(torch.tensor([[3.0]], dtype=F64), w, "m.", {"router": {"top": 1}})
     assert torch.allclose(out, torch.tensor([[(0.5 * 6.0) ** 2]], dtype=F64))                # sigmoid(0) = 1/2 inside the square
     assert pp.choose(torch.tensor([0.3, 0.9, 0.5], dtype=F64), 2)[0] == [1, 2]
+
+
+@pytest.mark.parametrize("name", ["pair", "pair_wide_state"])
+def test_sides_without_norms_join_the_stream(name, monkeypatch):
+    """What a block that joins its mixer's output itself asks for (shared_norm), of a mixer whose output products are stacked: the
+    kernels' places are taken by plain products, the sides' by products with random matrices."""
+    cfg = CASES[name]
+    model = DecoderModel(config_from_dict(cfg).model_spec(), Runtime(torch.device("cpu"), torch.float32))
+    weights = pc.make_weights(cfg, 1)
+    model.load_tensors(dict(weights))
+    at = [i for i, ly in enumerate(cfg["layers"]) if ly["type"] == "parallel"][0]
+    mixer = model.blocks[at].mixer
+    assert mixer.w_ends is not None
+    g = torch.Generator().manual_seed(2)
+    n, d = 5, cfg["width"]
+    h, x, extra = (torch.randn(n, d, generator=g) for _ in range(3))
+    mats = {}
+    for key in ("left", "right"):
+        side = getattr(mixer, key)
+        mats[key] = torch.randn(d, side.output_columns, generator=g)
+
+        def forward(h, ctx, cache, position=None, residual=None, rows=None, into=None, factor=1.0, m=mats[key]):
+            into.copy_(factor * (h @ m))
+        side.forward = forward
+
+    def join_sum_rows(a, x, mult=1.0, add=True, norm_a=None, scale_a=1.0, b=None, norm_b=None, scale_b=1.0, c=None, low=None):
+        assert norm_a is None and norm_b is None
+        y = mult * (scale_a * a + (scale_b * b if b is not None else 0.0) + (c if c is not None else 0.0))
+        x.copy_(x + y if add else y)
+        if low is not None:
+            low.copy_(x)
+    monkeypatch.setattr(ops, "linear", lambda a, w, out=None, out_dtype=None, **kw: (a.float() @ w.float().t()).to(out_dtype or a.dtype))
+    monkeypatch.setattr(ops, "join_sum_rows", join_sum_rows)
+    sums = sum(scale * (h.double() @ mats[key].double()) @ weights[f"l{at}.mix.{key}.o"].double().t()
+               for key, scale in (("left", mixer.left_scale), ("right", mixer.right_scale)))
+    for add, mult, more in ((True, 0.5, extra), (True, 1.0, None), (False, 1.0, None)):
+        stream, copy = x.clone(), torch.empty(n, d)
+        mixer.join(h, None, (None, None), None, stream, more, mult, copy, add)
+        want = mult * (sums + (more.double() if more is not None else 0.0)) + (x.double() if add else 0.0)
+        size = float(want.abs().max())
+        # float32 sums of at most some hundred products of size `size`
+        assert float((stream.double() - want).abs().max()) <= 1e-4 * size and torch.equal(copy, stream)
