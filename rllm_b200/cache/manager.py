@@ -51,13 +51,21 @@ class _Request:
     state_slot: Optional[int] = None
 
 
+def _pool_tensor(name):
+    def put(group, tensor):
+        group.__dict__[name], group._planes = tensor, {}
+    return property(lambda group: group.__dict__[name], put)
+
+
 class PagedGroup:
     def __init__(self, need: PagedKVNeed, entries: list, n_blocks: int, block_size: int):
         self.need, self.entries, self.block_size, self.n_blocks = need, entries, block_size, n_blocks
         self.allocator = BlockAllocator(n_blocks)
         self.pool = None                               # device tensor, see CacheManager.allocate_device
         self.pool_k = self.pool_v = None               # in place of `pool` when value heads have a size of their own
-        self._planes = None                            # the pool's tensors and the views that `planes` has made of them
+
+    # the pool's tensors; setting one lets go of the views that `planes` has made, and so of the memory behind them
+    pool, pool_k, pool_v = (_pool_tensor(name) for name in ("pool", "pool_k", "pool_v"))
 
     def first_needed_block(self, length: int) -> int:
         """Logical index of the first block that tokens at positions >= length can still read
@@ -73,10 +81,7 @@ class PagedGroup:
 
     def planes(self, plane: int):
         """(keys, values) of one run entry: [pages, kv_heads, block_size, head size].  The views are made once per pool."""
-        owner = (self.pool, self.pool_k, self.pool_v)
-        if self._planes is None or any(a is not b for a, b in zip(self._planes[0], owner)):
-            self._planes = (owner, {})
-        views = self._planes[1]
+        views = self._planes
         if plane not in views:
             if self.pool is not None:
                 views[plane] = self.pool[plane, 0], self.pool[plane, 1]

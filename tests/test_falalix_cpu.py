@@ -153,3 +153,27 @@ def test_the_sides_of_a_parallel_layer_keep_their_output_products(dtype):
     mixer = model.blocks[0].mixer
     assert mixer.w_ends is None
     assert torch.equal(mixer.left.w_o, weights["l0.mix.left.o"]) and torch.equal(mixer.right.w_o, weights["l0.mix.right.o"])
+
+
+@pytest.mark.parametrize("need", [PagedKVNeed(2, 8), PagedKVNeed(2, 8, v_head_dim=12)])
+def test_a_pool_that_is_replaced_is_given_back(need):
+    """The views of a pool's planes do not outlive it, neither when another one takes its place nor when it is taken away."""
+    import gc
+    import weakref
+    cm = CacheManager([need, need], [None] * 2, block_size=4, max_tokens=32, max_requests=2)
+    for _ in range(2):
+        cm.allocate_device("cpu", torch.float32)
+        grp = cm.paged[0]
+        k, v = grp.planes(1)
+        assert grp.planes(1)[0] is k and (k.shape[-1], v.shape[-1]) == (need.head_dim, need.value_dim)
+        assert all(a.data_ptr() == b.data_ptr() for a, b in zip((k, v), (grp.pool[1, 0], grp.pool[1, 1]) if grp.pool is not None
+                                                                 else (grp.pool_k[1], grp.pool_v[1])))
+        old = [weakref.ref(t) for t in (k, v)]
+        del k, v
+        cm.allocate_device("cpu", torch.float32)
+        gc.collect()
+        assert all(ref() is None for ref in old)
+    grp.planes(0)
+    old = [weakref.ref(t) for t in grp.planes(1)]
+    grp.pool = grp.pool_k = grp.pool_v = None
+    assert all(ref() is None for ref in old)
