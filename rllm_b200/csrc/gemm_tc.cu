@@ -62,7 +62,7 @@ template <> __device__ __forceinline__ void store_row32<bf16>(bf16* dst, const f
     }
 }
 
-// Persistent: the grid is one CTA per SM; CTA c takes tiles c, c + grid, c + 2 grid, ... (m fastest, so
+// Persistent: the grid is one CTA per SM (two with BN 128 and 64); CTA c takes tiles c, c + grid, c + 2 grid, ... (m fastest, so
 // the CTAs running together share few weight rows and the whole of A stays in L2).  Two accumulator
 // buffers in TMEM (2 x BN columns): the epilogue of one tile overlaps the MMAs of the next, and the
 // operand ring never drains between tiles.
@@ -304,7 +304,7 @@ static int launch_tc(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int 
 // silu(gate) * up).  A, B bfloat16 row-major with 16-byte aligned bases and lda, ldb multiples of 8;
 // K a multiple of 8.  `err` is a device int that receives a code if a bounded wait ran out.
 // Returns 0, a cudaError_t, 30000 + CUresult of the tensor-map encoder, or cudaErrorInvalidValue.
-// glu_*: the constants of the gated epilogue (GluForm in common.cuh); rllm_gemm_tc is SwiGLU's {0, 1, 0}.
+// glu_*: the constants of the gated epilogue (GluForm in common.cuh); SwiGLU's are {0, 1, 0}.
 // bn: rows of B per tile, 256, or with the gated epilogue (half of them gate and half up) also 128 or 64.
 RLLM_API int rllm_gemm_tc_tile(const void* A, const void* B, void* C, int c_dtype, int M, int N, int K, int lda, int ldb,
                                int ldc, int epilogue, int up_row_offset, float glu_limit, float glu_alpha,
@@ -343,18 +343,6 @@ RLLM_API int rllm_gemm_tc_tile(const void* A, const void* B, void* C, int c_dtyp
 #undef GATED
     }
     return (int)cudaErrorInvalidValue;
-}
-
-RLLM_API int rllm_gemm_tc_glu(const void* A, const void* B, void* C, int c_dtype, int M, int N, int K, int lda, int ldb,
-                              int ldc, int epilogue, int up_row_offset, float glu_limit, float glu_alpha,
-                              float glu_shift, int* err, cudaStream_t stream) {
-    return rllm_gemm_tc_tile(A, B, C, c_dtype, M, N, K, lda, ldb, ldc, epilogue, up_row_offset, glu_limit, glu_alpha, glu_shift,
-                             256, err, stream);
-}
-
-RLLM_API int rllm_gemm_tc(const void* A, const void* B, void* C, int c_dtype, int M, int N, int K, int lda, int ldb,
-                          int ldc, int epilogue, int up_row_offset, int* err, cudaStream_t stream) {
-    return rllm_gemm_tc_glu(A, B, C, c_dtype, M, N, K, lda, ldb, ldc, epilogue, up_row_offset, 0.f, 1.f, 0.f, err, stream);
 }
 
 // =====================================================================================================
@@ -820,7 +808,5 @@ RLLM_API int rllm_gemm_tc_swap(const void* W, const void* X, void* C, int c_dtyp
 TC_DEFINE_WAIT_CONTROLS(rllm_tc)
 
 // the packed-argument forms (common.cuh) for the host runtime's replay of recorded launches
-RLLM_PACKED(rllm_gemm_tc)
-RLLM_PACKED(rllm_gemm_tc_glu)
 RLLM_PACKED(rllm_gemm_tc_tile)
 RLLM_PACKED(rllm_gemm_tc_swap)

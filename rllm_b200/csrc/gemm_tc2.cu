@@ -468,7 +468,7 @@ static int launch_tc2(const T2Maps& maps, void* C, int ldc, int M, int N, int K,
 }
 
 // C[M,N] (+)= A[M,K] . B[N,K]^T with two SMs per 256 x 256 tile.  Arguments, epilogues and return
-// values as rllm_gemm_tc (gemm_tc.cu).
+// values as rllm_gemm_tc_tile (gemm_tc.cu).
 // glu_*: the constants of the gated epilogue (GluForm in common.cuh); rllm_gemm_tc2 is SwiGLU's {0, 1, 0}.
 RLLM_API int rllm_gemm_tc2_glu(const void* A, const void* B, void* C, int c_dtype, int M, int N, int K, int lda,
                                int ldb, int ldc, int epilogue, int up_row_offset, float glu_limit, float glu_alpha,
