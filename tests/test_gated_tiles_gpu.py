@@ -44,6 +44,26 @@ def test_gated_tiles(tile, m, F, k):
             assert bool(base[m].isnan().all()) and bool(base[:, F:].isnan().all())
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("tile,m,F,k", [(64, 900, 4800, 520), (128, 900, 4800, 520), (64, 333, 6400, 1024), (128, 2048, 3072, 1024),
+                                        (256, 2048, 3072, 1024)])
+def test_three_tiles_a_cta_and_more(tile, m, F, k):
+    """Both accumulators and every stage of the ring are used again: at least three tiles a CTA, more blocks of K than stages, and
+    in the last row of tiles warps without a row."""
+    a = torch.randn(m, k, generator=torch.Generator().manual_seed(m)).bfloat16()
+    w = (2.0 * torch.randn(2 * F, k, generator=torch.Generator().manual_seed(F)) * k ** -0.5).bfloat16()
+    ctas = ops().sm_count(torch.device(DEV)) * (1 if tile == 256 else 2)
+    assert -(-m // 128) * -(-F // (tile // 2)) > 2 * ctas and k > 8 * 64
+    want = gated(a.double() @ w.double().t(), F, None)
+    for dt, rel in ((torch.float32, 2e-5), (torch.bfloat16, 2.0 ** -8)):
+        base = torch.full((m + 1, F + 8), float("nan"), dtype=dt, device=DEV)
+        ops().gemm_tc(a.to(DEV), w.to(DEV), base[:m, :F], ops().EPI_SWIGLU, up_row_offset=F, tile=tile)
+        ops().check_device_errors()
+        # as above
+        assert bool(((base[:m, :F].cpu().double() - want).abs() <= want.abs() * rel + 40 * k * 2.0 ** -24).all())
+        assert bool(base[m].isnan().all()) and bool(base[:, F:].isnan().all())
+
+
 def test_the_rule():
     tile = ops()._gated_tile
     assert [tile(m, 3072, 1024) for m in (65, 128, 384, 385, 512, 4096)] == [64, 64, 64, 128, 128, 128]

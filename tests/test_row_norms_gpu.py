@@ -82,3 +82,50 @@ def test_add_rms_norm(n, d, dt, shift):
     ops().add_rms_norm(kept, moved, w.to(DEV), out, 1e-5, rows=rows, write_x=False, delta_scale=0.5)
     assert torch.equal(kept.cpu(), x)
     assert bool(((out.cpu().double() - unit[[n - 1, 0]]).abs() <= (unit[[n - 1, 0]].abs() + 1) * 1e-5).all())
+
+
+def odd_rows(n, d):
+    """Rows with an infinity, with a NaN, with a square beyond float32, and ordinary ones; their weights."""
+    a = rnd(n, d, seed=10)
+    a[0, d // 2], a[1, d - 1], a[2, 0] = float("inf"), float("nan"), 3e20
+    return a, rnd(d, seed=11)
+
+
+def formula(a, w, eps=1e-6):
+    return a * (1.0 / torch.sqrt((a * a).sum(1, keepdim=True) / a.shape[1] + eps)) * w
+
+
+def alike(got, want, bits):
+    """NaN where the formula has it (an infinity times 0 too), 0 beside an infinity or a square beyond the range."""
+    got = got.cpu().double()
+    assert torch.equal(got.isnan(), want.isnan())
+    ok = ~want.isnan()
+    assert bool(((got - want.double()).abs() <= want.double().abs() * (2.0 ** -bits + 64 * 2.0 ** -24) + 1e-30)[ok].all())
+
+
+@pytest.mark.parametrize("n", [4, 130])
+@pytest.mark.parametrize("d", [64, 1024, 4096, 8192])
+def test_infinities_and_nans_stay_in_their_rows(n, d):
+    """float32's own rules: the sum of squares of an ordinary row is short of 64 roundings of its value by far (any order)."""
+    a, w = odd_rows(n, d)
+    want = formula(a, w)
+    for low, bits in ((torch.float32, 24), (torch.bfloat16, 8)):
+        out = torch.empty(n, d, dtype=low, device=DEV)
+        ops().norm_rows(a.to(DEV), w.to(DEV), 1e-6, low=out)
+        alike(out, want, bits)
+        ops().add_rms_norm(a.to(DEV), None, w.to(DEV), out, 1e-6)
+        alike(out, want, bits)
+    stream = torch.zeros(n, d, device=DEV)
+    ops().norm_rows(a.to(DEV), w.to(DEV), 1e-6, x=stream, add=True)
+    alike(stream, want, 24)
+    # the same columns as the query row of a projection; keys and values are ordinary
+    G, dk, bs = 1, 64, 8
+    H = d // dk
+    other = rnd(n, 2 * dk, seed=12)
+    q = torch.empty(n, d, device=DEV)
+    kc, vc = (torch.zeros(n // bs + 1, G, bs, dk, device=DEV) for _ in range(2))
+    ops().qkv_rownorm_store(torch.cat([a, other], 1).to(DEV), None, w.to(DEV), w[:dk].contiguous().to(DEV),
+                            torch.arange(n, dtype=torch.int32, device=DEV), q, kc, vc, H, G, dk, dk, bs, 1e-6)
+    alike(q, want, 24)
+    alike(kc.view(-1, dk)[:n], formula(other[:, :dk], w[:dk]), 24)
+    assert torch.equal(vc.view(-1, dk)[:n].cpu(), other[:, dk:])
