@@ -291,7 +291,7 @@ latent_rope_store_kernel(const TQ* q, long long ld_q, const float* kv, long long
                          const float* __restrict__ kv_norm_w, const float2* cs_table, float cs_mult,
                          const int* __restrict__ slots, TO* q_att, TO* cache, int H, int dq, int r, int rank, int bs,
                          float eps, int write_kv, int n_slots, int* err, int pairs) {
-    // Blocks y > 0: 256 (head, pair)s of the queries each.  Block y = 0: the latent, its norm and the shared key part.  (One block
+    // Blocks y > 0: 256 (head, pair)s of the queries at a time.  Block y = 0: the latent, its norm and the shared key part.  (One block
     // a token went through its 1,024 pairs four at a time, a round trip each, and through the latent behind them: 6.3 us.)
     __shared__ float red[33];
     constexpr int NR = 4;                               // columns of the latent a thread holds (rank up to 1,024)
@@ -301,17 +301,18 @@ latent_rope_store_kernel(const TQ* q, long long ld_q, const float* kv, long long
     const float2* cs = cs_table + (size_t)t * half;
     if (blockIdx.y > 0) {
         pdl_wait();
-        const int i = (blockIdx.y - 1) * 256 + tid;
-        if (i >= H * half) return;
-        const int h = i / half, j = i - h * half;
-        const TQ* src = q + (size_t)t * ld_q + (size_t)h * (dq + r) + dq;
-        const float2 a = cs[j];
-        const float c = a.x * cs_mult, s = a.y * cs_mult;
-        const int iu = pairs ? 2 * j : j, iv = pairs ? 2 * j + 1 : j + half;
-        const float u = to_f<TQ>(src[iu]), w = to_f<TQ>(src[iv]);
-        TO* dst = q_att + ((size_t)t * H + h) * W + rank;
-        dst[iu] = from_f<TO>(u * c - w * s);
-        dst[iv] = from_f<TO>(w * c + u * s);
+        const unsigned all = (unsigned)H * half;
+        for (unsigned i = (blockIdx.y - 1) * 256 + tid; i < all; i += (gridDim.y - 1) * 256) {
+            const int h = i / half, j = i - h * half;
+            const TQ* src = q + (size_t)t * ld_q + (size_t)h * (dq + r) + dq;
+            const float2 a = cs[j];
+            const float c = a.x * cs_mult, s = a.y * cs_mult;
+            const int iu = pairs ? 2 * j : j, iv = pairs ? 2 * j + 1 : j + half;
+            const float u = to_f<TQ>(src[iu]), w = to_f<TQ>(src[iv]);
+            TO* dst = q_att + ((size_t)t * H + h) * W + rank;
+            dst[iu] = from_f<TO>(u * c - w * s);
+            dst[iv] = from_f<TO>(w * c + u * s);
+        }
         return;
     }
     int slot = write_kv ? slots[t] : -1;
@@ -358,9 +359,8 @@ RLLM_API int rllm_latent_rope_store(const void* q, int q_dt, long long ld_q, con
         ld_q < (long long)H * (dq + r) || ld_kv < rank + r)
         return (int)cudaErrorInvalidValue;
     const int ns = (int)(n_slots > 0x7fffffffLL ? 0x7fffffffLL : n_slots);
-    const long long pairs_of_token = (long long)H * (r / 2);
-    if (pairs_of_token > 256LL * 65534) return (int)cudaErrorInvalidValue;
-    const dim3 grid(n, 1 + (unsigned)((pairs_of_token + 255) / 256));
+    const long long blocks = ((long long)H * (r / 2) + 255) / 256;        // of queries; more than a grid has go round
+    const dim3 grid(n, 1 + (unsigned)(blocks < 65534 ? blocks : 65534));
 #define LAUNCH(TQ, TO)                                                                                           \
     return rllm_launch(latent_rope_store_kernel<TQ, TO>, grid, dim3(256), 0, stream, (const TQ*)q, ld_q, kv,      \
                        ld_kv, kv_norm_w, (const float2*)cs_table, cs_mult, slots, (TO*)q_att, (TO*)cache, H, dq, r, \

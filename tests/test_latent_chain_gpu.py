@@ -121,3 +121,24 @@ def test_the_longest_contexts(n_splits):
         want, size = (e @ k) / e.sum(), (e @ k.abs()) / e.sum()
         # probabilities and the result in bfloat16: 2^-8 of sums of |p v|, twice; a million keys' sums in float32
         assert bool(((out[r].cpu().double() - want).abs() <= (2.0 ** -7 + 2e-4) * size + 1e-6).all()), r
+
+
+def test_more_pairs_a_token_than_a_grid_has_blocks():
+    """65,534 blocks of 256 pairs and some more: the blocks go round."""
+    o, H, dq, r, rank = ops(), (1 << 18) + 77, 1, 130, 2
+    assert H * (r // 2) > 65534 * 256
+    g = torch.Generator(device=DEV).manual_seed(3)
+    q = torch.randn(1, H * (dq + r), generator=g, device=DEV)
+    kv = torch.randn(1, rank + r, generator=g, device=DEV)
+    ang = torch.rand(1, r // 2, generator=g, device=DEV) * 6.0
+    q_att = torch.full((1, H * (rank + r)), 7.0, device=DEV)
+    cache = torch.zeros(1, 1, 4, rank + r, device=DEV)
+    o.latent_rope_store(q, kv, torch.ones(rank, device=DEV), torch.stack([torch.cos(ang), torch.sin(ang)], -1).contiguous(), 1.0,
+                        torch.zeros(1, dtype=torch.int32, device=DEV), q_att, cache, H, dq, r, rank, 4, 1e-6)
+    o.check_device_errors()
+    u, w = q.view(H, dq + r)[:, dq:].split(r // 2, 1)
+    c, s = torch.cos(ang), torch.sin(ang)
+    want = torch.cat([u * c - w * s, w * c + u * s], 1)
+    got = q_att.view(H, rank + r)
+    assert bool((got[:, :rank] == 7.0).all())
+    assert bool(((got[:, rank:] - want).abs() <= 2.0 ** -20 * (want.abs() + 4.0)).all())
