@@ -308,10 +308,15 @@ latent_combine_kernel(const float* part_o, const float* part_ml, bf16* out, int 
             }
         }
         const __nv_bfloat162 lo = __floats2bfloat162_rn(o.x * inv, o.y * inv), hi = __floats2bfloat162_rn(o.z * inv, o.w * inv);
-        uint2 u;
-        u.x = *reinterpret_cast<const uint32_t*>(&lo);
-        u.y = *reinterpret_cast<const uint32_t*>(&hi);
-        *reinterpret_cast<uint2*>(out + ((size_t)tok * H + head) * V + c) = u;
+        bf16* dst = out + ((size_t)tok * H + head) * V + c;
+        if (((uintptr_t)out & 7) == 0) {
+            uint2 u;
+            u.x = *reinterpret_cast<const uint32_t*>(&lo);
+            u.y = *reinterpret_cast<const uint32_t*>(&hi);
+            *reinterpret_cast<uint2*>(dst) = u;
+        } else {                                                    // a caller's rows that begin anywhere
+            dst[0] = lo.x; dst[1] = lo.y; dst[2] = hi.x; dst[3] = hi.y;
+        }
     }
 }
 

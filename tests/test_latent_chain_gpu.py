@@ -142,3 +142,23 @@ def test_more_pairs_a_token_than_a_grid_has_blocks():
     got = q_att.view(H, rank + r)
     assert bool((got[:, :rank] == 7.0).all())
     assert bool(((got[:, rank:] - want).abs() <= 2.0 ** -20 * (want.abs() + 4.0)).all())
+
+
+@pytest.mark.parametrize("shift", [1, 2, 3])
+@pytest.mark.parametrize("H,rank", [(3, 64), (33, 512)])
+def test_output_rows_that_begin_anywhere(shift, H, rank):
+    """The same bits as at an aligned address, and nothing beside them."""
+    o, W, bs, L = ops(), rank + 64, 16, 300
+    g = torch.Generator().manual_seed(H)
+    cache = torch.randn(-(-L // bs), 1, bs, W, generator=g).bfloat16().to(DEV)
+    q = torch.randn(2, H * W, generator=g).bfloat16().to(DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)                       # noqa: E731
+    table = torch.arange(len(cache), dtype=torch.int32, device=DEV).repeat(2, 1)
+    size = 2 * H * rank
+    aligned, base = (torch.full((size + 8,), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    for out in (aligned[:size], base[shift:shift + size]):
+        o.latent_decode_attention(q, cache, out.view(2, H * rank), i32([L - 1, 40]), i32([0, 1]), table, H, W, rank, bs, W ** -0.5,
+                                  0.0, L)
+    o.check_device_errors()
+    assert torch.equal(base[shift:shift + size], aligned[:size])
+    assert bool((base[:shift] == 7.0).all()) and bool((base[shift + size:] == 7.0).all())
