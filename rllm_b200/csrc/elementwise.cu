@@ -165,16 +165,24 @@ template <> __device__ __forceinline__ void store2<bf16>(bf16* p, float a, float
     *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b);
 }
 
-// four elements from a 16-byte (float32) or 8-byte (bfloat16) boundary, as loaded and as floats
-template <typename T> struct Four;
-template <> struct Four<float> {
+// four elements, as loaded and as floats; AL: they lie at a 16-byte (float32) or 8-byte (bfloat16) boundary
+template <typename T, bool AL> struct Four;
+template <bool AL> struct Four<float, AL> {
     float4 r;
-    __device__ __forceinline__ void load(const float* p) { r = *reinterpret_cast<const float4*>(p); }
+    __device__ __forceinline__ void load(const float* p) {
+        if (AL) r = *reinterpret_cast<const float4*>(p);
+        else r = make_float4(p[0], p[1], p[2], p[3]);
+    }
     __device__ __forceinline__ float4 get() const { return r; }
 };
-template <> struct Four<bf16> {
+template <bool AL> struct Four<bf16, AL> {
     uint2 r;
-    __device__ __forceinline__ void load(const bf16* p) { r = *reinterpret_cast<const uint2*>(p); }
+    __device__ __forceinline__ void load(const bf16* p) {
+        if (AL) { r = *reinterpret_cast<const uint2*>(p); return; }
+        const __nv_bfloat162 a = __halves2bfloat162(p[0], p[1]), b = __halves2bfloat162(p[2], p[3]);
+        r.x = *reinterpret_cast<const uint32_t*>(&a);
+        r.y = *reinterpret_cast<const uint32_t*>(&b);
+    }
     __device__ __forceinline__ float4 get() const {
         const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.x));
         const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.y));
@@ -188,7 +196,9 @@ template <> struct Four<bf16> {
 // all of a thread's x and delta before the first sum is stored (x may be what delta points at for all the compiler knows, so
 // that a store between them holds the next loads back: one round trip per four columns).  8 rows of 4,096 with a float32 delta
 // 3.40 -> 1.96 us, 512 rows 7.2 -> 3.8, 2,048 rows 13.1 -> 11.5 (7.3 TB/s, mostly out of L2).
-template <typename TD, typename TO, int NV>
+// AL: delta can be read four columns at a time (elsewhere one at a time: 8 rows of 4,096 2.00 us, 2,048 rows 12.4; by the
+// kernel above, which adds in another order, 3.6 and 30).
+template <typename TD, typename TO, int NV, bool AL>
 __global__ void __launch_bounds__(256)
 add_rms_norm_vec_kernel(float* x, const TD* delta, const int* __restrict__ rows,
                         const float* __restrict__ w, TO* __restrict__ out, int d, float eps, int write_x,
@@ -207,7 +217,7 @@ add_rms_norm_vec_kernel(float* x, const TD* delta, const int* __restrict__ rows,
     float* xr = x + (size_t)src * d;
     const TD* dr = delta ? delta + (size_t)src * d : nullptr;
     float4 v[NV];
-    Four<TD> add[NV];
+    Four<TD, AL> add[NV];
 #pragma unroll
     for (int it = 0; it < NV; ++it) {
         const int i = (it * 256 + threadIdx.x) * 4;
@@ -247,11 +257,12 @@ add_rms_norm_vec_kernel(float* x, const TD* delta, const int* __restrict__ rows,
 template <typename TD, typename TO>
 static int launch_norm(float* x, const void* delta, const int* rows, const float* w, void* out, int n_rows, int d,
                        float eps, int write_x, float delta_scale, cudaStream_t stream) {
-    const bool vec = d % 4 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)w & 15) == 0 &&
-                     ((uintptr_t)delta & (4 * sizeof(TD) - 1)) == 0;
-#define VEC(NV)                                                                                        \
-    return rllm_launch(add_rms_norm_vec_kernel<TD, TO, NV>, dim3(n_rows), dim3(256), 0, stream, x,     \
-                       (const TD*)delta, rows, w, (TO*)out, d, eps, write_x, delta_scale)
+    const bool vec = d % 4 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)w & 15) == 0;
+    const bool al = ((uintptr_t)delta & (4 * sizeof(TD) - 1)) == 0;
+#define VEC(NV)                                                                                                      \
+    return rllm_launch(al ? add_rms_norm_vec_kernel<TD, TO, NV, true> : add_rms_norm_vec_kernel<TD, TO, NV, false>,  \
+                       dim3(n_rows), dim3(256), 0, stream, x, (const TD*)delta, rows, w, (TO*)out, d, eps, write_x,  \
+                       delta_scale)
     if (vec && d <= 1024) VEC(1);
     if (vec && d <= 2048) VEC(2);
     if (vec && d <= 4096) VEC(4);

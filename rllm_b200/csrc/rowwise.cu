@@ -320,7 +320,9 @@ qkv_rownorm_store_kernel(const TI* qkv, const float* __restrict__ bias, const fl
 // registers (NV float4 a thread) between the sums and the stores, both sums are taken in one exchange.  Bound by its bytes;
 // 2,048 rows of 4,096 + 1,024 + 1,024: 51 us through shared memory an entry at a time, now 32 us; 8 rows 9.9 -> 5.9 us, with
 // the weights and values on their way early (EARLY) 4.1 -> 2.7 us between kernels of its own kind.
-template <typename TO, int NV, bool EARLY>
+// AL: biases and norm weights can be read four columns at a time (elsewhere one at a time: 8 rows of 4,096 + 1,024 + 1,024 2.6 us,
+// 2,048 rows 18.4 against 16.9; by the kernel above, which adds in another order, 5.3 and 39).
+template <typename TO, int NV, bool EARLY, bool AL>
 __global__ void __launch_bounds__(1024)
 qkv_rownorm_store4_kernel(const float* qkv, const float* __restrict__ bias, const float* __restrict__ q_norm_w,
                           const float* __restrict__ k_norm_w, const int* __restrict__ slots, TO* q_out, TO* k_cache, TO* v_cache,
@@ -333,16 +335,17 @@ qkv_rownorm_store4_kernel(const float* qkv, const float* __restrict__ bias, cons
     // are here when the rows are, and the first value columns when they are stored.  With many tokens the registers that
     // takes cost more (2,048 rows of 1,024 + 256 + 256: 8.7 -> 9.8 us).
     float4 wgt[EARLY ? NV : 1], off4[EARLY ? NV : 1];
+    auto four = [](const float* p) { return AL ? ld4(p) : make_float4(p[0], p[1], p[2], p[3]); };
     auto norm_weight = [&](int c) {
         const float* w = c < wq ? q_norm_w : k_norm_w;
-        return w ? ld4(w + (c < wq ? c : c - wq)) : make_float4(1.f, 1.f, 1.f, 1.f);
+        return w ? four(w + (c < wq ? c : c - wq)) : make_float4(1.f, 1.f, 1.f, 1.f);
     };
     if (EARLY) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int c = 4 * (tid + i * blockDim.x);
             wgt[EARLY ? i : 0] = c < wq + wk ? norm_weight(c) : make_float4(1.f, 1.f, 1.f, 1.f);
-            off4[EARLY ? i : 0] = bias && c < wq + wk ? ld4(bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            off4[EARLY ? i : 0] = bias && c < wq + wk ? four(bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     }
     pdl_wait();
@@ -367,7 +370,7 @@ qkv_rownorm_store4_kernel(const float* qkv, const float* __restrict__ bias, cons
         const int c = 4 * (tid + i * blockDim.x);
         if (c >= wq + wk) continue;
         if (bias) {
-            const float4 b = EARLY ? off4[EARLY ? i : 0] : ld4(bias + c);
+            const float4 b = EARLY ? off4[EARLY ? i : 0] : four(bias + c);
             val[i].x += b.x; val[i].y += b.y; val[i].z += b.z; val[i].w += b.w;
         }
         const float s = val[i].x * val[i].x + val[i].y * val[i].y + val[i].z * val[i].z + val[i].w * val[i].w;
@@ -421,11 +424,12 @@ RLLM_API int rllm_qkv_rownorm_store(const void* qkv, int in_dt, long long ld, co
     const int threads = n < 128 ? 1024 : 256;
     const int qk = (H + G) * dk, nv = (qk / 4 + threads - 1) / threads;
     if (in_dt == RLLM_F32 && !rot && nv <= 8 && ld % 4 == 0 && dk % 4 == 0 && dv % 4 == 0 && v_off % 4 == 0 && al16(qkv) &&
-        al16(q_out) && al16(k_cache) && al16(v_cache) && al16(bias) && al16(q_norm_w) && al16(k_norm_w)) {
-#define LAUNCH4(TO, NV, EARLY)                                                                                                        \
-    return rllm_launch(qkv_rownorm_store4_kernel<TO, NV, EARLY>, dim3(n), dim3(threads), 0, stream, (const float*)qkv, bias, q_norm_w, \
-                       k_norm_w, slots, (TO*)q_out, (TO*)k_cache, (TO*)v_cache, ld, H * dk, G * dk, G * dv, G, dk, dv, bs, eps, \
-                       write_kv, ns, err, v_off)
+        al16(q_out) && al16(k_cache) && al16(v_cache)) {
+        const bool al = al16(bias) && al16(q_norm_w) && al16(k_norm_w);
+#define LAUNCH4(TO, NV, EARLY)                                                                                                 \
+    return rllm_launch(al ? qkv_rownorm_store4_kernel<TO, NV, EARLY, true> : qkv_rownorm_store4_kernel<TO, NV, EARLY, false>,  \
+                       dim3(n), dim3(threads), 0, stream, (const float*)qkv, bias, q_norm_w, k_norm_w, slots, (TO*)q_out,      \
+                       (TO*)k_cache, (TO*)v_cache, ld, H * dk, G * dk, G * dv, G, dk, dv, bs, eps, write_kv, ns, err, v_off)
         if (out_dt == RLLM_F32) {
             if (nv <= 2 && n < 128) { LAUNCH4(float, 2, true); }
             if (nv <= 2) { LAUNCH4(float, 2, false); }

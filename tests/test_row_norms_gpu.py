@@ -129,3 +129,41 @@ def test_infinities_and_nans_stay_in_their_rows(n, d):
     alike(q, want, 24)
     alike(kc.view(-1, dk)[:n], formula(other[:, :dk], w[:dk]), 24)
     assert torch.equal(vc.view(-1, dk)[:n].cpu(), other[:, dk:])
+
+
+@pytest.mark.parametrize("n", [1, 130])
+@pytest.mark.parametrize("d", [1024, 2052, 4096, 8192])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shift", [1, 2, 3])
+def test_a_delta_that_begins_anywhere(n, d, dt, shift):
+    """The same kernel, and so the same bits, as at an aligned address."""
+    x, delta, w = rnd(n, d, seed=13).to(DEV), rnd(n, d, seed=14).to(dt).to(DEV), rnd(d, seed=15).to(DEV)
+    moved = torch.zeros(n * d + 4, dtype=dt, device=DEV)[shift:shift + n * d].view(n, d)
+    moved.copy_(delta)
+    got = []
+    for t in (delta, moved):
+        xs, out = x.clone(), torch.empty(n, d, device=DEV)
+        ops().add_rms_norm(xs, t, w, out, 1e-5, delta_scale=0.5)
+        got.append((xs, out))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("n", [1, 130])
+@pytest.mark.parametrize("H,G,dk", [(8, 2, 64), (32, 8, 128)])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_projection_weights_that_begin_anywhere(n, H, G, dk, dt, which):
+    """Bias, query norm or key norm one entry behind an aligned address: the same bits as with all of them aligned."""
+    wq, wk, bs = H * dk, G * dk, 8
+    rows = rnd(n, wq + 2 * wk, seed=16).to(DEV)
+    weights = [rnd(k, seed=17 + i).to(DEV) for i, k in enumerate((wq + 2 * wk, wq, wk))]
+    moved = list(weights)
+    moved[which] = torch.cat([torch.zeros(1, device=DEV), weights[which]])[1:]
+    slots = torch.arange(n, dtype=torch.int32, device=DEV)
+    got = []
+    for bias, qn, kn in (weights, moved):
+        q = torch.empty(n, wq, dtype=dt, device=DEV)
+        kc, vc = (torch.zeros(n // bs + 1, G, bs, dk, dtype=dt, device=DEV) for _ in range(2))
+        ops().qkv_rownorm_store(rows, bias, qn, kn, slots, q, kc, vc, H, G, dk, dk, bs, 1e-5)
+        got.append((q, kc, vc))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
