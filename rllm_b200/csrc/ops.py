@@ -1740,6 +1740,7 @@ def gemv_stream(a, w, out, epilogue=EPI_STORE, up_row_offset=0, grid=None, stage
 def linear_stack(x, w, out):
     """out[i] = x[i] . w[i]^T for the planes of x [G, m, k], w [G, n, k] and out [G, m, n] (each contiguous): products of one
     shape on inputs of their own.  Few rows: one launch that streams all the matrices (gemv_stream); else one product each."""
+    _need_cuda(x, w, out)
     _need_contig(x=x, w=w, out=out)
     (G, m, k), n = x.shape, w.shape[1]
     assert w.shape == (G, n, k) and out.shape == (G, m, n) and out.dtype == torch.float32

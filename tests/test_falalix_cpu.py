@@ -177,3 +177,12 @@ def test_a_pool_that_is_replaced_is_given_back(need):
     old = [weakref.ref(t) for t in grp.planes(1)]
     grp.pool = grp.pool_k = grp.pool_v = None
     assert all(ref() is None for ref in old)
+
+
+@pytest.mark.parametrize("m", [3, 16, 40])
+def test_stacked_products_refuse_tensors_of_the_host(m):
+    """In front of any launch, as the single products do."""
+    from rllm_b200.csrc import ops
+    x, w = torch.zeros(2, m, 2048, dtype=torch.bfloat16), torch.zeros(2, 4096, 2048, dtype=torch.bfloat16)
+    with pytest.raises(ops.KernelError, match="CUDA device only"):
+        ops.linear_stack(x, w, torch.zeros(2, m, 4096))
