@@ -695,7 +695,10 @@ template <int HD>
 __global__ void __launch_bounds__(HD) paged_flash_combine_kernel(const FlashParams p, int n_splits) {
     extern __shared__ float wgt[];               // [n_splits] m, then the weight, of each split; [n_splits] l
     pdl_launch_dependents();
-    // the step's index arrays were uploaded before its first kernel: this chain of reads is over when the partials are there
+    // Tiles and cu_q are written by copies on this stream alone, the tiles in the middle of a step by its first attention layer
+    // (AttentionPlan).  A copy waits for the kernels queued before it and those behind it wait for the copy, so that they are
+    // there when the attention kernel starts, and with it this one; a kernel that wrote them could still be running.  This chain
+    // of reads is over when the partials are there.
     const int tile = blockIdx.x, R = blockIdx.z;
     const int req = p.tile_req[tile], tok0 = p.tile_tok0[tile];
     const int nt = min(p.TT, p.cu_q[req + 1] - tok0);

@@ -118,7 +118,8 @@ norm_rows_vec_kernel(const float* in, long long ld_in, const float* __restrict__
 
 // Rows of at most 4 NV columns a thread: the row stays in registers, the weights are fetched ahead of the dependency wait, and
 // the old x with the row, so that behind the sum there is nothing left to wait for (8 rows of 4,096 with both outputs 2.42 ->
-// 2.24 us, 512 rows 7.0 -> 3.9; the loop above is left for rows of more than 8,192 columns).
+// 2.24 us, 512 rows 7.0 -> 3.9).  The loop above is left for rows of more than 8,192 columns, and from 128 rows on, where a block
+// has 256 threads and a thread at most 16 columns here, for rows of more than 4,096.
 template <typename TL, int NV>
 __global__ void __launch_bounds__(1024)
 norm_rows_reg_kernel(const float* in, long long ld_in, const float* __restrict__ w, float* x, int add, TL* low,

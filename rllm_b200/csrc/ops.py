@@ -1503,7 +1503,9 @@ def _tc_ok(a, w, _meta=False) -> bool:
 def gemm_tc(a, w, out, epilogue=EPI_STORE, up_row_offset=0, glu=None, tile=256):
     """out (+)= a . w^T on the tcgen05 tensor cores (TMA-fed, accumulators in tensor memory).
     epilogue as for skinny_gemm; glu = (limit, alpha, shift): the gated epilogue's constants (None:
-    SwiGLU); tile: rows of w per tile, 256, or 128 or 64 with the gated epilogue.  See gemm_tc.cu."""
+    SwiGLU); tile: rows of w per tile, 256, or 128 or 64 with the gated epilogue.
+    w is read ahead of the dependency wait, as in the few-row kernels: a weight, not what a kernel of this package has just been
+    launched to write.  See gemm_tc.cu."""
     _need_cuda(a, w, out)
     if not _tc_ok(a, w):
         raise KernelError("gemm_tc needs bfloat16 operands, k a multiple of 8 and 16-byte aligned rows")
@@ -2026,7 +2028,9 @@ def paged_attention_f32(q, k_cache, v_cache, out, ctx, block_table, H, K, hd, bl
 class AttentionPlan:
     """Tiles of one step for one attention geometry (query heads per key/value head, window):
     which requests take the decode shape (16-row tiles, split keys) and which the prefill shape
-    (64-row tiles).  Built once per step on the host and shared by every layer of that geometry."""
+    (64-row tiles).  Built once per step on the host, when the first layer of that geometry runs, and shared by all of them.
+    The tiles come to the device by a copy on the step's stream and have to: the kernel that merges split keys reads them
+    ahead of its dependency wait, which no kernel that wrote them would be finished for."""
 
     def __init__(self, ctx, H, K, window, device, chunk=0):
         g = H // K
