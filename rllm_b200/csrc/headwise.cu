@@ -68,14 +68,6 @@ norm_rows_kernel(const void* in, int in_dt, long long ld_in, const float* __rest
     }
 }
 
-// v * (rs * w), or joined to old in one rounding (fmaf).  Written out because the two kernels below have to agree: left to the
-// compiler, the one with a load between product and sum had one rounding and the one without had two.
-__device__ __forceinline__ float4 scaled_or_joined(float4 v, float rs, float4 w, bool join, float4 old) {
-    if (join)
-        return make_float4(fmaf(v.x, rs * w.x, old.x), fmaf(v.y, rs * w.y, old.y), fmaf(v.z, rs * w.z, old.z), fmaf(v.w, rs * w.w, old.w));
-    return make_float4(v.x * (rs * w.x), v.y * (rs * w.y), v.z * (rs * w.z), v.w * (rs * w.w));
-}
-
 // The same for float32 input whose rows, weight and outputs allow 16-byte accesses (d and the row strides
 // multiples of 4): four columns a thread and pass.  The sums are taken in another order than in the kernel
 // above; which of the two runs depends on the sizes and addresses only, never on the batch.
@@ -98,9 +90,15 @@ norm_rows_vec_kernel(const float* in, long long ld_in, const float* __restrict__
     for (int i = threadIdx.x * 4; i < d; i += blockDim.x * 4) {
         float4 v = *reinterpret_cast<const float4*>(row + i);
         const float4 ww = w ? *reinterpret_cast<const float4*>(w + i) : make_float4(1.f, 1.f, 1.f, 1.f);
-        float4* xp = x ? reinterpret_cast<float4*>(x + t * d + i) : nullptr;
-        v = scaled_or_joined(v, rs, ww, xp && add, xp && add ? *xp : v);
-        if (xp) *xp = v;
+        v.x *= rs * ww.x; v.y *= rs * ww.y; v.z *= rs * ww.z; v.w *= rs * ww.w;
+        if (x) {
+            float4* xp = reinterpret_cast<float4*>(x + t * d + i);
+            if (add) {
+                const float4 o = *xp;
+                v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+            }
+            *xp = v;
+        }
         if (low) {
             TL* lp = low + t * ld_low + i;
             if (sizeof(TL) == 4) {
@@ -114,6 +112,15 @@ norm_rows_vec_kernel(const float* in, long long ld_in, const float* __restrict__
             }
         }
     }
+}
+
+// v * (rs * w), or joined to old in one rounding.  Written out because the two kernels have to agree: the loop kernel above gets a
+// multiply-add from the compiler (written out there too, other forms of the loop were 4 to 16 % slower; the tests hold both to
+// the same bits), the one below, without a load between product and sum, got two roundings.
+__device__ __forceinline__ float4 scaled_or_joined(float4 v, float rs, float4 w, bool join, float4 old) {
+    if (join)
+        return make_float4(fmaf(v.x, rs * w.x, old.x), fmaf(v.y, rs * w.y, old.y), fmaf(v.z, rs * w.z, old.z), fmaf(v.w, rs * w.w, old.w));
+    return make_float4(v.x * (rs * w.x), v.y * (rs * w.y), v.z * (rs * w.z), v.w * (rs * w.w));
 }
 
 // Rows of at most 4 NV columns a thread: the row stays in registers, the weights are fetched ahead of the dependency wait, and
