@@ -287,20 +287,68 @@ RLLM_API int rllm_rope_unitnorm_store(const void* rows, int in_dt, long long ld,
 }
 
 // ------------------------------------------------------------------ latent attention: cache row and query parts
-// One block per token.  kv[t] = [latent (rank) | shared key part (r)] with rows ld_kv apart (float32);
-// the latent is RMS-normed with a weight, the key part rotated (pairs (i, i + r/2), or (2i, 2i + 1) when
-// `pairs`); both go to the
-// token's cache row [rank + r] (one key/value head).  q[t] = H heads of [plain (dq) | rotated (r)]
-// with rows ld_q apart; the rotated part of head h goes to q_att[t, h, rank : rank + r] (the first
-// rank entries of each head are written by the product that takes the plain part into latent space).
+// kv[t] = [latent (rank) | shared key part (r)] with rows ld_kv apart (float32); the latent is RMS-normed with a weight, the key
+// part rotated (pairs (i, i + r/2), or (2i, 2i + 1) when `pairs`); both go to the token's cache row [rank + r] (one key/value
+// head).  q[t] = H heads of [plain (dq) | rotated (r)] with rows ld_q apart; the rotated part of head h goes to
+// q_att[t, h, rank : rank + r] (the first rank entries of each head are written by the product that takes the plain part into
+// latent space).
+template <typename TI, typename TO>
+__device__ __forceinline__ void turn_pair(const TI* src, TO* dst, float2 a, float cs_mult, int j, int half, int pairs) {
+    const float c = a.x * cs_mult, s = a.y * cs_mult;
+    const int iu = pairs ? 2 * j : j, iv = pairs ? 2 * j + 1 : j + half;
+    const float u = to_f<TI>(src[iu]), w = to_f<TI>(src[iv]);
+    dst[iu] = from_f<TO>(u * c - w * s);
+    dst[iv] = from_f<TO>(w * c + u * s);
+}
+
+// One block per token: for as many tokens as fill the GPU that way.  Bound by its bytes; 32 registers, eight blocks an SM.
 template <typename TQ, typename TO>
 __global__ void __launch_bounds__(256)
 latent_rope_store_kernel(const TQ* q, long long ld_q, const float* kv, long long ld_kv,
                          const float* __restrict__ kv_norm_w, const float2* cs_table, float cs_mult,
                          const int* __restrict__ slots, TO* q_att, TO* cache, int H, int dq, int r, int rank, int bs,
                          float eps, int write_kv, int n_slots, int* err, int pairs) {
-    // Blocks y > 0: 256 (head, pair)s of the queries at a time.  Block y = 0: the latent, its norm and the shared key part.  (One block
-    // a token went through its 1,024 pairs four at a time, a round trip each, and through the latent behind them: 6.3 us.)
+    __shared__ float red[33];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int t = blockIdx.x, tid = threadIdx.x;
+    const int half = r >> 1, W = rank + r;
+    const float2* cs = cs_table + (size_t)t * half;
+    // queries: every (head, pair)
+    for (int i = tid; i < H * half; i += blockDim.x) {
+        const int h = i / half, j = i - h * half;
+        turn_pair<TQ, TO>(q + (size_t)t * ld_q + (size_t)h * (dq + r) + dq, q_att + ((size_t)t * H + h) * W + rank, cs[j], cs_mult, j,
+                          half, pairs);
+    }
+    const float* row = kv + (size_t)t * ld_kv;
+    float ss = 0.f;
+    for (int i = tid; i < rank; i += blockDim.x) ss += row[i] * row[i];
+    ss = block_sum(ss, red);
+    if (!write_kv) return;
+    int slot = slots[t];
+    if (slot >= n_slots) {
+        if (tid == 0 && err) atomicExch(err, RLLM_ERR_SLOT);
+        slot = -1;
+    }
+    if (slot < 0) return;
+    const float rs = 1.0f / sqrtf(ss / (float)rank + eps);
+    TO* dst = cache + (size_t)slot * W;                 // one head: page * bs + offset is the row
+    for (int i = tid; i < rank; i += blockDim.x) dst[i] = from_f<TO>(row[i] * rs * kv_norm_w[i]);
+    for (int j = tid; j < half; j += blockDim.x)
+        turn_pair<float, TO>(row + rank, dst + rank, cs[j], cs_mult, j, half, pairs);
+}
+
+// Several blocks per token, the same bits.  Blocks y > 0: the queries, 256 (head, pair)s at a time.  Block y = 0: the latent, its norm
+// and the shared key part.  A few tokens are a chain of memory round trips, which this takes side by side (the kernel above goes
+// through 1,024 pairs four at a time, a round trip each, and through the latent behind them): 8 tokens of 32 heads 3.6 us above,
+// 1.7 here, 512 tokens 6.3 and 3.7, 1,024 tokens 7.5 and 6.2.  It takes 40 registers and reads the angles twice; 2,048 tokens 11.1
+// above and 11.4 here.
+template <typename TQ, typename TO>
+__global__ void __launch_bounds__(256)
+latent_rope_store_split_kernel(const TQ* q, long long ld_q, const float* kv, long long ld_kv,
+                               const float* __restrict__ kv_norm_w, const float2* cs_table, float cs_mult,
+                               const int* __restrict__ slots, TO* q_att, TO* cache, int H, int dq, int r, int rank, int bs,
+                               float eps, int write_kv, int n_slots, int* err, int pairs) {
     __shared__ float red[33];
     constexpr int NR = 4;                               // columns of the latent a thread holds (rank up to 1,024)
     pdl_launch_dependents();
@@ -312,14 +360,8 @@ latent_rope_store_kernel(const TQ* q, long long ld_q, const float* kv, long long
         const unsigned all = (unsigned)H * half;
         for (unsigned i = (blockIdx.y - 1) * 256 + tid; i < all; i += (gridDim.y - 1) * 256) {
             const int h = i / half, j = i - h * half;
-            const TQ* src = q + (size_t)t * ld_q + (size_t)h * (dq + r) + dq;
-            const float2 a = cs[j];
-            const float c = a.x * cs_mult, s = a.y * cs_mult;
-            const int iu = pairs ? 2 * j : j, iv = pairs ? 2 * j + 1 : j + half;
-            const float u = to_f<TQ>(src[iu]), w = to_f<TQ>(src[iv]);
-            TO* dst = q_att + ((size_t)t * H + h) * W + rank;
-            dst[iu] = from_f<TO>(u * c - w * s);
-            dst[iv] = from_f<TO>(w * c + u * s);
+            turn_pair<TQ, TO>(q + (size_t)t * ld_q + (size_t)h * (dq + r) + dq, q_att + ((size_t)t * H + h) * W + rank, cs[j], cs_mult,
+                              j, half, pairs);
         }
         return;
     }
@@ -340,15 +382,8 @@ latent_rope_store_kernel(const TQ* q, long long ld_q, const float* kv, long long
 #pragma unroll
     for (int k = 0; k < NR; ++k) ss += v[k] * v[k];
     for (int i = tid + 256 * NR; i < rank; i += 256) ss += row[i] * row[i];
-    TO* dst = cache + (size_t)slot * W;                 // one head: page * bs + offset is the row
-    for (int j = tid; j < half; j += 256) {
-        const float2 a = cs[j];
-        const float c = a.x * cs_mult, s = a.y * cs_mult;
-        const int iu = pairs ? 2 * j : j, iv = pairs ? 2 * j + 1 : j + half;
-        const float u = row[rank + iu], w = row[rank + iv];
-        dst[rank + iu] = from_f<TO>(u * c - w * s);
-        dst[rank + iv] = from_f<TO>(w * c + u * s);
-    }
+    TO* dst = cache + (size_t)slot * W;
+    for (int j = tid; j < half; j += 256) turn_pair<float, TO>(row + rank, dst + rank, cs[j], cs_mult, j, half, pairs);
     ss = block_sum(ss, red);
     const float rs = 1.0f / sqrtf(ss / (float)rank + eps);
 #pragma unroll
@@ -367,12 +402,15 @@ RLLM_API int rllm_latent_rope_store(const void* q, int q_dt, long long ld_q, con
         ld_q < (long long)H * (dq + r) || ld_kv < rank + r)
         return (int)cudaErrorInvalidValue;
     const int ns = (int)(n_slots > 0x7fffffffLL ? 0x7fffffffLL : n_slots);
-    const long long blocks = ((long long)H * (r / 2) + 255) / 256;        // of queries; more than a grid has go round
-    const dim3 grid(n, 1 + (unsigned)(blocks < 65534 ? blocks : 65534));
+    // Blocks for a token's queries: what they fill, up to eight blocks an SM in all.  Where that is none, or where they would fill
+    // one and could have no second (1,024 tokens of 8 heads of 16 pairs: 3.4 us, in two blocks a token 3.75), one block a token.
+    const long long fill = ((long long)H * (r / 2) + 255) / 256, most = 8LL * rllm_sm_count() / n;
+    const bool split = most > (fill == 1 ? 1 : 0);
+    const dim3 grid(n, split ? 1 + (unsigned)(fill < most ? fill : most) : 1);
 #define LAUNCH(TQ, TO)                                                                                           \
-    return rllm_launch(latent_rope_store_kernel<TQ, TO>, grid, dim3(256), 0, stream, (const TQ*)q, ld_q, kv,      \
-                       ld_kv, kv_norm_w, (const float2*)cs_table, cs_mult, slots, (TO*)q_att, (TO*)cache, H, dq, r, \
-                       rank, bs, eps, write_kv, ns, err, pairs)
+    return rllm_launch(split ? latent_rope_store_split_kernel<TQ, TO> : latent_rope_store_kernel<TQ, TO>, grid,  \
+                       dim3(256), 0, stream, (const TQ*)q, ld_q, kv, ld_kv, kv_norm_w, (const float2*)cs_table,  \
+                       cs_mult, slots, (TO*)q_att, (TO*)cache, H, dq, r, rank, bs, eps, write_kv, ns, err, pairs)
     if (q_dt == RLLM_F32 && out_dt == RLLM_F32) { LAUNCH(float, float); }
     if (q_dt == RLLM_F32 && out_dt == RLLM_BF16) { LAUNCH(float, bf16); }
     if (q_dt == RLLM_BF16 && out_dt == RLLM_BF16) { LAUNCH(bf16, bf16); }

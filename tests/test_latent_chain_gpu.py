@@ -162,3 +162,26 @@ def test_output_rows_that_begin_anywhere(shift, H, rank):
     o.check_device_errors()
     assert torch.equal(base[shift:shift + size], aligned[:size])
     assert bool((base[:shift] == 7.0).all()) and bool((base[shift + size:] == 7.0).all())
+
+
+@pytest.mark.parametrize("H,rank,r", [(3, 250, 64), (16, 512, 64), (2, 1100, 32)])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_many_tokens_are_stored_as_few_are(H, rank, r, dt):
+    """One block a token, some, and as many as its queries fill: the same bits."""
+    o, n, dq, bs, W = ops(), 1300, 8, 32, rank + r
+    g = torch.Generator(device=DEV).manual_seed(rank)
+    q = torch.randn(n, H * (dq + r), generator=g, device=DEV).to(dt)
+    kv, w = torch.randn(n, W, generator=g, device=DEV), torch.randn(rank, generator=g, device=DEV)
+    cs = torch.randn(n, r // 2, 2, generator=g, device=DEV)
+    slots = torch.randperm(n, generator=g, device=DEV).to(torch.int32)
+    slots[5] = slots[1111] = -1
+    got = []
+    for step in (n, 700, 100):
+        q_att = torch.full((n, H * W), 7.0, dtype=dt, device=DEV)
+        cache = torch.full((-(-n // bs), 1, bs, W), 7.0, dtype=dt, device=DEV)
+        for a in range(0, n, step):
+            b = min(n, a + step)
+            o.latent_rope_store(q[a:b], kv[a:b], w, cs[a:b], 1.25, slots[a:b], q_att[a:b], cache, H, dq, r, rank, bs, 1e-6)
+        got.append((q_att, cache))
+    o.check_device_errors()
+    assert all(torch.equal(x, y) for other in got[1:] for x, y in zip(got[0], other))
