@@ -90,7 +90,8 @@ struct SvNorm {
 
 // Products of one shape on inputs of their own, run as one (store epilogue): W is their matrices one behind the other, X and C
 // their planes likewise.  A share may reach from one matrix into the next, not further; its chunks end where a matrix ends.
-// (One launch in place of several: their starts and ends, 2 to 4 us each, happen once.)
+// (One launch in place of several: their starts and ends, 2 to 4 us each, happen once.)  An instantiation of its own: with the cut in
+// every launch, a single product of 12 rows by 2,048 x 6,144 out of L2 took 7.53 us in place of 7.16.
 struct SvStack {
     int gran;                 // granules of one matrix (0: a single product)
     int m;                    // rows of X and of C per plane
@@ -112,7 +113,7 @@ __device__ __forceinline__ void sv_share(int n_gran, int c, int G, int& first, i
 // every atom) and every warp works on all slots, so that the warps are busy whatever the number of
 // rows; at the end of a chunk the four partial sums of a slot are added in warp order through
 // shared memory by the warp of that number, which writes the slot's rows.
-template <int NT, int EPI, typename TC, int ATOMS, int STAGES>
+template <int NT, int EPI, typename TC, int ATOMS, int STAGES, bool STACK>
 __global__ void __launch_bounds__(SV_THREADS)
 gemv_stream_kernel(const __grid_constant__ SvMaps maps, TC* __restrict__ C, int ldc, int m, int n, int K,
                    int up_row_offset, int* err, const SvNorm nm, const SvStack sk) {
@@ -139,14 +140,14 @@ gemv_stream_kernel(const __grid_constant__ SvMaps maps, TC* __restrict__ C, int 
     sv_share(n_gran, blockIdx.x, gridDim.x, g_first, g_last);
     const int nkb = (K + BK - 1) / BK;
     // chunks [g_first, g_cut) and [g_cut, g_last): the cut lies where the share passes from one stacked matrix into the next
-    const int plane0 = sk.gran ? g_first / sk.gran : 0;
-    const int g_cut = sk.gran ? min(g_last, (plane0 + 1) * sk.gran) : g_last;
+    const int plane0 = STACK ? g_first / sk.gran : 0;
+    const int g_cut = STACK ? min(g_last, (plane0 + 1) * sk.gran) : g_last;
     const int n_before = (g_cut - g_first + GRAN_PER_CHUNK - 1) / GRAN_PER_CHUNK;
-    const int n_chunks = n_before + (g_last - g_cut + GRAN_PER_CHUNK - 1) / GRAN_PER_CHUNK;
+    const int n_chunks = STACK ? n_before + (g_last - g_cut + GRAN_PER_CHUNK - 1) / GRAN_PER_CHUNK : n_before;
     auto chunk_first = [&](int chunk) {
-        return chunk < n_before ? g_first + chunk * GRAN_PER_CHUNK : g_cut + (chunk - n_before) * GRAN_PER_CHUNK;
+        return !STACK || chunk < n_before ? g_first + chunk * GRAN_PER_CHUNK : g_cut + (chunk - n_before) * GRAN_PER_CHUNK;
     };
-    auto chunk_size = [&](int chunk, int g0) { return min(GRAN_PER_CHUNK, (chunk < n_before ? g_cut : g_last) - g0); };
+    auto chunk_size = [&](int chunk, int g0) { return min(GRAN_PER_CHUNK, (STACK && chunk < n_before ? g_cut : g_last) - g0); };
     const int total = n_chunks * nkb;                     // stages this CTA streams
 
     // Every thread signals at once that the next kernel of the stream may be scheduled: all CTAs of
@@ -191,7 +192,7 @@ gemv_stream_kernel(const __grid_constant__ SvMaps maps, TC* __restrict__ C, int 
         };
         auto issue_x = [&](int it) {
             const int s = it % STAGES, kb = it % nkb;
-            const int x0 = sk.gran ? (plane0 + (it / nkb >= n_before)) * sk.m : 0;
+            const int x0 = STACK ? (plane0 + (it / nkb >= n_before)) * sk.m : 0;
             tma_load_3d(smem + (size_t)s * STAGE_BYTES + SV_W_BYTES, &maps.x, 0, x0, kb * ATOMS, &full_bar[s]);
         };
         if (lane != 0) return;
@@ -386,9 +387,9 @@ gemv_stream_kernel(const __grid_constant__ SvMaps maps, TC* __restrict__ C, int 
         }
         if (!waited) { pdl_wait(); waited = true; }      // C belongs to the kernels before until here
         // rows of this lane in slot `warp`: row g (sums 0, 1) and row g + 8 (sums 2, 3); batch columns 8j + 2t, + 1
-        const int row_end = min(n, (g0 + ng) * SV_GRAN);
+        const int row_end = min(n, (STACK ? g0 + ng : g_last) * SV_GRAN);
         TC* Cp = C;                                       // row r of stacked matrix p goes to column r - p * rows of plane p
-        if (EPI == SV_EPI_STORE && sk.gran) {
+        if (STACK) {
             const long long plane = plane0 + (chunk >= n_before);
             Cp += plane * sk.plane - plane * sk.gran * SV_GRAN;
         }
@@ -473,13 +474,16 @@ struct SvProblem {
     SvStack sk;
 };
 
-template <int NT, int EPI, typename TC, int ATOMS, int STAGES>
+template <int NT, int EPI, typename TC, int ATOMS, int STAGES, bool STACK = false>
 static int launch_sv_stages(const SvMaps& maps, void* C, int ldc, int m, int n, int K, int up, int grid, int* err,
                             const SvNorm& nm, const SvStack& sk, cudaStream_t stream) {
+    if constexpr (EPI == SV_EPI_STORE && sizeof(TC) == 4 && !STACK) {
+        if (sk.gran) return launch_sv_stages<NT, EPI, TC, ATOMS, STAGES, true>(maps, C, ldc, m, n, K, up, grid, err, nm, sk, stream);
+    }
     constexpr int SLOTS = 128 / ATOMS / 16;
     constexpr size_t smem = (size_t)STAGES * (SV_W_BYTES + ATOMS * NT * SV_GRAN_BYTES) +
                             2 * (SV_WARPS * SLOTS * NT * 32 * 4) * sizeof(float) + 1024;
-    auto kern = gemv_stream_kernel<NT, EPI, TC, ATOMS, STAGES>;
+    auto kern = gemv_stream_kernel<NT, EPI, TC, ATOMS, STAGES, STACK>;
     static bool attr_set = false;
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
